@@ -401,9 +401,10 @@ extern "C" iclblasStatus_t iclblasCreate(iclblasHandle_t* handle)
         int sms = 0;
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaMalloc(&c->ws.counters, sizeof(unsigned) * iclb::kCounterWords);
+        const size_t cbytes = sizeof(unsigned) * iclb::kCounterWords + sizeof(unsigned long long) * iclb::kPubWords;
+        if (e == cudaSuccess) e = cudaMalloc(&c->ws.counters, cbytes);
         if (e == cudaSuccess) e = cudaMalloc(&c->ws.dev_status, sizeof(int));
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->ws.counters, 0, sizeof(unsigned) * iclb::kCounterWords, c->own_stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->ws.counters, 0, cbytes, c->own_stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(c->ws.dev_status, 0, sizeof(int), c->own_stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->own_stream);
         if (e != cudaSuccess) {

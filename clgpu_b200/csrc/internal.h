@@ -33,13 +33,14 @@ struct Workspace {
     size_t scratch_bytes = 0;
     void* solver = nullptr;    // solver workspace (TRSM diagonal inverses), kept
     size_t solver_bytes = 0;   // apart so the GEMMs inside a solve can grow `scratch`
-    unsigned* counters = nullptr;   // kCounterWords words, zeroed at creation
+    unsigned* counters = nullptr;   // kCounterWords words and kPubWords 64-bit words, zeroed at creation
     int* dev_status = nullptr;      // one int, DeviceStatus bits
-    unsigned epoch = 0;             // host-side epoch for flag-based kernels
-    unsigned long long* pub = nullptr;   // TRSV: published solution entries (value, epoch), zeroed when grown
+    unsigned long long* pub = nullptr;   // TRSV: published solution entries (value, epoch), for solves longer
+                                         // than kPubWords values; zeroed when grown
     size_t pub_elems = 0;
 };
 constexpr int kCounterWords = 1 << 16;
+constexpr int kPubWords = 1 << 16;   // after the counters: TRSV's published solution entries
 
 // ---------------------------------------------------------------- adjoints
 cudaError_t strsm_backward(iclblasHandle_t h, int side, int uplo, int trans, int diag, int m, int n, float alpha,

@@ -3,22 +3,18 @@
 //
 // Replaces Strsv_simd16x16_* (one work-group of 256 serialising every
 // 16-column block with barriers) and the serial Strsv_naive / Ctrsv_naive
-// (libs/blas/funcs/Strsv/*, Ctrsv/*).  One launch covers the whole solve:
-//   - the n rows are cut into blocks of NB = 64; each CTA draws a ticket s
-//     from an atomic counter and owns block s of the solve order (forward for
-//     a lower op(A), backward for an upper one).  Tickets are handed out in
-//     start order, so a CTA only ever waits for CTAs that are already running:
-//     no deadlock however many CTAs fit on the GPU at once;
-//   - CTA s streams the tiles op(A)[blk s, blk j] for j < s (register
-//     prefetch of the next tile while it works on the current one), and for
-//     each waits until block j's solution is published (flag j == this call's
-//     epoch), then subtracts the tile times x_j;
-//   - it then solves its 64x64 diagonal block by substitution in shared
-//     memory, writes x_s, fences, and publishes flag s.
-// Every wait is bounded: after kSpinLimit polls the CTA records
-// kDevWaitTimeout in the device status word and every other CTA, which also
-// polls that word, returns; the host reports EXECUTION_FAILED.  Reads of
-// other CTAs' results go through L2 (ld.cg) so no stale L1 line is used.
+// (libs/blas/funcs/Strsv/*, Ctrsv/*).  One launch covers the whole solve: the
+// n rows are cut into blocks, one CTA per block; the CTAs draw tickets from
+// an atomic counter and own blocks in solve order (forward for a lower
+// op(A), backward for an upper one), so a CTA only ever waits for CTAs that
+// are already running.  Two kernels share that structure:
+//   - strsv_tma_kernel: long real solves that TMA can address, 128-row blocks;
+//   - trsv_block_kernel: everything else (complex data, short solves, any
+//     base address and leading dimension), 64-row blocks fetched element by
+//     element.
+// Every wait is bounded: a CTA that gives up records kDevWaitTimeout in the
+// device status word and returns, and so do the CTAs that wait for it; the
+// host reports EXECUTION_FAILED.
 #include <atomic>
 #include <cstddef>
 #include <type_traits>
@@ -29,20 +25,12 @@
 namespace iclb {
 namespace {
 
-constexpr int NB = 64;
 constexpr int kThreads = 256;
-constexpr long kSpinLimit = 1L << 22;
 
 __device__ __forceinline__ float zero_v(float) { return 0.f; }
 __device__ __forceinline__ cfloat zero_v(cfloat) { return cfloat{0.f, 0.f}; }
 __device__ __forceinline__ float conj_v(float v) { return v; }
 __device__ __forceinline__ cfloat conj_v(cfloat v) { return cfloat{v.re, -v.im}; }
-__device__ __forceinline__ float ldcg(const float* p) { return __ldcg(p); }
-__device__ __forceinline__ cfloat ldcg(const cfloat* p)
-{
-    float2 v = __ldcg((const float2*)p);
-    return cfloat{v.x, v.y};
-}
 __device__ __forceinline__ float ldg(const float* p) { return __ldg(p); }
 __device__ __forceinline__ cfloat ldg(const cfloat* p)
 {
@@ -59,6 +47,8 @@ __device__ __forceinline__ void msub(cfloat& acc, cfloat a, cfloat x)
 }
 __device__ __forceinline__ float addv(float a, float b) { return a + b; }
 __device__ __forceinline__ cfloat addv(cfloat a, cfloat b) { return cfloat{a.re + b.re, a.im + b.im}; }
+__device__ __forceinline__ float subv(float a, float b) { return a - b; }
+__device__ __forceinline__ cfloat subv(cfloat a, cfloat b) { return cfloat{a.re - b.re, a.im - b.im}; }
 __device__ __forceinline__ float divv(float a, float d) { return a / d; }
 // complex quotient through |d|^2 (the reference's cdiv, core/src/ocl/complex.h.cl:36)
 __device__ __forceinline__ cfloat divv(cfloat a, cfloat d)
@@ -72,157 +62,11 @@ __device__ __forceinline__ cfloat shfl(cfloat v, int src)
     return cfloat{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
 }
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ int ld_volatile(const int* p) { return *(const volatile int*)p; }
-
-// Thread t of the CTA holds tile elements (r, c) for r = t % NB and
-// c = t / NB + 4q, q = 0..15.  op N reads A down columns (consecutive r in a
-// warp), op T/C reads along rows of A (consecutive c in a warp: the warp
-// covers 32 consecutive r of one 4-column group, each thread loading one
-// element; A's rows are then strided, but the tile is small and latency, not
-// bandwidth, bounds these steps).
-template <class T>
-struct Tile {
-    T v[16];
-};
-
-template <class T>
-__device__ __forceinline__ void load_tile(Tile<T>& t, const T* __restrict__ A, long lda, int op, int r0, int nr,
-                                          int c0, int nc)
-{
-    const int r = threadIdx.x % NB, cb = threadIdx.x / NB;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int c = cb + 4 * q;
-        T val = zero_v(T());
-        if (r < nr && c < nc) {
-            // element (r, c) of op(A) restricted to the tile
-            if (op == 0) val = ldg(A + (long)(c0 + c) * lda + (r0 + r));
-            else {
-                val = ldg(A + (long)(r0 + r) * lda + (c0 + c));
-                if (op == 2) val = conj_v(val);
-            }
-        }
-        t.v[q] = val;
-    }
-}
-
-template <class T>
-__global__ void __launch_bounds__(kThreads) trsv_kernel(int n, int lower_op, int op, int unit, const T* __restrict__ A,
-                                                        long lda, T* x, long incx, unsigned* ticket, unsigned* flags,
-                                                        unsigned epoch, int* status)
-{
-    __shared__ T tile[NB][NB + 1];
-    __shared__ T xs[NB];
-    __shared__ T part[4][NB];
-    __shared__ unsigned s_sh;
-    __shared__ int abort_sh;
-
-    const int nb = (n + NB - 1) / NB;
-    if (threadIdx.x == 0) s_sh = atomicAdd(ticket, 1u);
-    __syncthreads();
-    const int s = (int)s_sh;
-    if (s == nb - 1 && threadIdx.x == 0) *ticket = 0u;  // every ticket of this launch is taken
-
-    // block index in row space for solve-order position p
-    auto blk = [&](int p) { return lower_op ? p : nb - 1 - p; };
-    const int rb = blk(s);
-    const int r0 = rb * NB, nr = min(NB, n - r0);
-    const int r = threadIdx.x % NB, cb = threadIdx.x / NB;
-
-    T acc = zero_v(T());  // partial sum of op(A)[r, cols of cb group] * x
-    Tile<T> cur;
-    {
-        const int jb = s > 0 ? blk(0) : rb;
-        load_tile(cur, A, lda, op, r0, nr, jb * NB, min(NB, n - jb * NB));
-    }
-    for (int p = 0; p <= s; ++p) {
-        const int jb = blk(p);
-        const int c0 = jb * NB, nc = min(NB, n - c0);
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 16; ++q) tile[r][cb + 4 * q] = cur.v[q];
-        if (p < s) {
-            const int nj = blk(p + 1);
-            load_tile(cur, A, lda, op, r0, nr, nj * NB, min(NB, n - nj * NB));
-        }
-        if (p == s) break;  // diagonal tile is in shared memory
-        // wait for block p of the solve order
-        if (threadIdx.x == 0) {
-            int ab = 0;
-            long it = 0;
-            while (ld_acquire(flags + p) != epoch) {
-                if (ld_volatile(status) != kDevOk) { ab = 1; break; }
-                if (++it > kSpinLimit) {
-                    atomicOr(status, (int)kDevWaitTimeout);
-                    ab = 1;
-                    break;
-                }
-                __nanosleep(64);
-            }
-            abort_sh = ab;
-        }
-        __syncthreads();
-        if (abort_sh) return;
-        if (threadIdx.x < nc) xs[threadIdx.x] = ldcg(x + (long)(c0 + threadIdx.x) * incx);
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int c = cb + 4 * q;
-            if (c < nc) msub(acc, tile[r][c], xs[c]);
-        }
-    }
-    // combine the 4 column-group partials with b, then solve the diagonal block
-    part[cb][r] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        // each lane owns rows lane and lane + 32
-        T b0 = zero_v(T()), b1 = zero_v(T());
-        if (lane < nr) b0 = addv(addv(x[(long)(r0 + lane) * incx], addv(part[0][lane], part[1][lane])),
-                                addv(part[2][lane], part[3][lane]));
-        if (lane + 32 < nr)
-            b1 = addv(addv(x[(long)(r0 + lane + 32) * incx], addv(part[0][lane + 32], part[1][lane + 32])),
-                      addv(part[2][lane + 32], part[3][lane + 32]));
-        if (lower_op) {
-            for (int k = 0; k < nr; ++k) {
-                const int owner = k & 31;
-                T bk = (k < 32) ? shfl(b0, owner) : shfl(b1, owner);
-                if (!unit) bk = divv(bk, tile[k][k]);
-                if (lane == owner) { if (k < 32) b0 = bk; else b1 = bk; }
-                if (lane > k && lane < nr) msub(b0, tile[lane][k], bk);
-                if (lane + 32 > k && lane + 32 < nr) msub(b1, tile[lane + 32][k], bk);
-            }
-        } else {
-            for (int k = nr - 1; k >= 0; --k) {
-                const int owner = k & 31;
-                T bk = (k < 32) ? shfl(b0, owner) : shfl(b1, owner);
-                if (!unit) bk = divv(bk, tile[k][k]);
-                if (lane == owner) { if (k < 32) b0 = bk; else b1 = bk; }
-                if (lane < k) msub(b0, tile[lane][k], bk);
-                if (lane + 32 < k) msub(b1, tile[lane + 32][k], bk);
-            }
-        }
-        if (lane < nr) x[(long)(r0 + lane) * incx] = b0;
-        if (lane + 32 < nr) x[(long)(r0 + lane + 32) * incx] = b1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) st_release(flags + s, epoch);
-}
 
 // ---------------------------------------------------------------- STRSV, TMA path
 // Float TRSV when A is 16-byte aligned with lda a multiple of 4 and >= n
-// (the usual case).  Same ticket-ordered one-launch structure as above, with
+// (the usual case).  The ticket-ordered one-launch structure, with
 // blocks of RB = 128 rows, one CTA of 256 threads per block (one CTA per SM),
 // and changes that shorten the chain of dependent block solves:
 //   - tiles arrive by TMA (boxes of 128 rows x 64 columns of op(A), half a
@@ -375,10 +219,12 @@ __device__ __forceinline__ bool poll_word(const unsigned long long* src, unsigne
     unsigned long long w = ld_relaxed_u64(src);
     if ((unsigned)(w >> 32) != epoch) {
         const unsigned long long t0 = tma::global_ns();
-        for (;;) {
+        // the status word is read on one poll in 64: its load would double
+        // the time between two looks at the entry
+        for (unsigned it = 1;; ++it) {
             w = ld_relaxed_u64(src);
             if ((unsigned)(w >> 32) == epoch) break;
-            if (ld_volatile(status) != kDevOk || tma::global_ns() - t0 > kTrsvWaitNs) return false;
+            if ((it & 63) == 0 && (ld_volatile(status) != kDevOk || tma::global_ns() - t0 > kTrsvWaitNs)) return false;
         }
     }
     v = __uint_as_float((unsigned)w);
@@ -884,13 +730,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const float xf = pick(o, own);
     if (ok) {
         // the hand-offs first, then the published words; the output x last
-        if (ndst > 0) {
-            float v[4];
+        float v[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v[k] = R0 + k < nr ? o[k] : 0.f;
-            st_async_f32x4(dx0, v[0], v[1], v[2], v[3], db0);
-            if (ndst > 1) st_async_f32x4(dx1, v[0], v[1], v[2], v[3], db1);
-        }
+        for (int k = 0; k < 4; ++k) v[k] = R0 + k < nr ? o[k] : 0.f;
+        // the next CTA of the cluster, which waits for them, first
+        if (ndst > 0 && cg == 4) st_async_f32x4(dx0, v[0], v[1], v[2], v[3], db0);
+        __syncwarp();
+        if (ndst > 0 && cg != 4) st_async_f32x4(dx0, v[0], v[1], v[2], v[3], db0);
+        if (ndst > 1) st_async_f32x4(dx1, v[0], v[1], v[2], v[3], db1);
         if (cg < 4 && row < nr) st_relaxed_u64(pub + r0 + row, ((unsigned long long)epoch << 32) | __float_as_uint(xf));
         if (cg < 4 && row < nr) x[(long)(r0 + row) * incx] = xf;
     } else {
@@ -907,6 +754,485 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (s == nb - 1) *(volatile unsigned*)epoch_word = epoch;
     }
     if constexpr (CL > 1) cluster_sync_all();
+}
+
+// ---------------------------------------------------------------- any layout, float and complex
+// 64-row blocks, 256 threads.  What bounds it is the chain of dependent block
+// steps, so everything that does not depend on the previous block is done
+// before that block arrives:
+//   - the diagonal block is inverted in FP64 (16 x 16 blocks by substitution,
+//     two doubling steps) and kept in FP32 registers, 2 rows x 8 columns a
+//     thread, and so is the tile next to it;
+//   - the other tiles are fetched by cp.async, element by element (4 or 8
+//     bytes: any base address and leading dimension), into a 3-stage ring and
+//     multiplied in the same thread layout: a thread's partial sums of all
+//     tiles stay in its registers, and the 8 threads that share rows add them
+//     once, together with the product of the last tile;
+//   - the chain step is then two register products, x = inv(D) (y - T x_prev),
+//     with one barrier between them, and solved entries travel as in
+//     strsv_tma_kernel: by st.async inside a cluster, as (value, epoch) words
+//     between clusters.  A thread's two rows make one remote store, and those
+//     to the next CTA of the cluster, which waits for them, go first.
+// A block whose inverse or right-hand side holds an infinity or a NaN is
+// solved by substitution instead, so that those reach exactly the entries
+// that substitution gives them to.
+// Measured (us; before: one substitution warp per block and a flag per
+// block): complex n = 3001 512, 88; n = 4096 88; n = 512 25; real with an odd
+// leading dimension n = 4096 67, n = 16384 354.  A step of the chain takes
+// 0.85 us (real) or 1.15 (complex).  Measured and dropped: W = inv(D) T formed
+// beforehand for a one-product step (8 us more before the chain starts, the
+// step no shorter: the hand-off, not the products, sets it).
+constexpr int NB = 64;
+constexpr int kBStages = 3;
+
+struct alignas(16) dcomplex {
+    double re, im;
+};
+__device__ __forceinline__ double wide(float v) { return (double)v; }
+__device__ __forceinline__ dcomplex wide(cfloat v) { return dcomplex{(double)v.re, (double)v.im}; }
+__device__ __forceinline__ float narrow(double v) { return (float)v; }
+__device__ __forceinline__ cfloat narrow(dcomplex v) { return cfloat{(float)v.re, (float)v.im}; }
+__device__ __forceinline__ void dset(double& v, double r) { v = r; }
+__device__ __forceinline__ void dset(dcomplex& v, double r) { v = dcomplex{r, 0.0}; }
+__device__ __forceinline__ double dneg(double v) { return -v; }
+__device__ __forceinline__ dcomplex dneg(dcomplex v) { return dcomplex{-v.re, -v.im}; }
+__device__ __forceinline__ void dmac(double& acc, double a, double b) { acc = fma(a, b, acc); }
+__device__ __forceinline__ void dmac(dcomplex& acc, dcomplex a, dcomplex b)
+{
+    acc.re = fma(a.re, b.re, acc.re);
+    acc.im = fma(a.re, b.im, acc.im);
+    acc.re = fma(-a.im, b.im, acc.re);
+    acc.im = fma(a.im, b.re, acc.im);
+}
+__device__ __forceinline__ double dinv(double v) { return 1.0 / v; }
+__device__ __forceinline__ dcomplex dinv(dcomplex v)
+{
+    const double q = 1.0 / fma(v.re, v.re, v.im * v.im);
+    return dcomplex{v.re * q, -v.im * q};
+}
+__device__ __forceinline__ double dmul(double a, double b) { return a * b; }
+__device__ __forceinline__ dcomplex dmul(dcomplex a, dcomplex b)
+{
+    return dcomplex{fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re)};
+}
+__device__ __forceinline__ bool finite_v(float v) { return isfinite(v); }
+__device__ __forceinline__ bool finite_v(cfloat v) { return isfinite(v.re) && isfinite(v.im); }
+__device__ __forceinline__ void madd_v(float& acc, float a, float x) { acc = fmaf(a, x, acc); }
+__device__ __forceinline__ void madd_v(cfloat& acc, cfloat a, cfloat x)
+{
+    acc.re = fmaf(a.re, x.re, acc.re);
+    acc.im = fmaf(a.re, x.im, acc.im);
+    acc.re = fmaf(-a.im, x.im, acc.re);
+    acc.im = fmaf(a.im, x.re, acc.im);
+}
+__device__ __forceinline__ float xor_add(float v, int o) { return v + __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ cfloat xor_add(cfloat v, int o) { return cfloat{xor_add(v.re, o), xor_add(v.im, o)}; }
+
+template <class T>
+using wide_t = decltype(wide(T()));
+
+// A thread's 8 columns of a 64-column tile are cg + 8j (j = 0 .. 7): its
+// entries of a block of x are stored next to each other, 16 bytes between the
+// 8 groups, so the 16-byte reads of 8 threads fall in different banks.
+template <class T>
+constexpr int kBGroup = 8 + 16 / (int)sizeof(T);
+template <class T>
+__device__ __forceinline__ int bidx(int c)
+{
+    return (c & 7) * kBGroup<T> + (c >> 3);
+}
+template <class T>
+constexpr int kBEntries = 8 * kBGroup<T>;
+// elements between the columns (op N) or rows (op T/C) of a staged tile: the
+// reads of a warp (8 column groups x 4 rows) fall in different banks
+constexpr int kBPitch = 72;
+template <class T>
+__device__ __forceinline__ int bpitch(int op)
+{
+    return op != 0 ? kBPitch : (sizeof(T) == 8 ? 66 : 68);
+}
+
+template <class T>
+struct alignas(16) BlockSmem {
+    T stage[kBStages][NB * kBPitch];   // tiles, [column][row] (op N) or [row][column]
+    T xin[kMaxCluster][kBEntries<T>];  // solved blocks of earlier CTAs of this cluster (st.async)
+    T xs[2][kBEntries<T>];             // a solved block from the published words
+    T y2[kBEntries<T>];                // b - the products of the earlier blocks
+    wide_t<T> Y[NB][NB + 1];  // FP64 inverse of the diagonal block (the other triangle: doubling temporaries)
+    T D[NB][NB + 1];          // the diagonal block of op(A)
+    uint64_t xbar[kMaxCluster];
+    unsigned s, epoch, cl;
+};
+static_assert(sizeof(BlockSmem<cfloat>) <= 232448 && 2 * (sizeof(BlockSmem<float>) + 1024) <= 233472,
+              "block kernel shared memory: one complex or two real CTAs per SM");
+
+__device__ __forceinline__ void cp_async_elem(float* dst, const float* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(tma::smem_u32(dst)), "l"(src), "r"(in ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_elem(cfloat* dst, const cfloat* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(tma::smem_u32(dst)), "l"(src), "r"(in ? 8 : 0)
+                 : "memory");
+}
+// two neighbouring entries into another CTA's shared memory, counted on its barrier
+__device__ __forceinline__ void st_async_pair(uint32_t addr, float a, float b, uint32_t bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(a), "f"(b), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_pair(uint32_t addr, cfloat a, cfloat b, uint32_t bar)
+{
+    st_async_f32x4(addr, a.re, a.im, b.re, b.im, bar);
+}
+
+// `cl`: CTAs per cluster (1: no cluster launch attribute)
+template <class T>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
+    trsv_block_kernel(int cl, int n, int lower_op, int op, int unit, const T* __restrict__ A, long lda, T* x,
+                      long incx, unsigned long long* pub, unsigned* ticket, unsigned* epoch_word, int* status)
+{
+    using W = wide_t<T>;
+    constexpr int kW = sizeof(T) / 4;  // published words per entry
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BlockSmem<T>& S = *reinterpret_cast<BlockSmem<T>*>(smem_raw);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int nb = (n + NB - 1) / NB;
+    const unsigned rank = cl > 1 ? cluster_rank() : 0u;
+    if (t == 0) {
+        const unsigned e = *(volatile unsigned*)epoch_word + 1u;
+        S.epoch = e == 0u ? 1u : e;
+        if (cl == 1) S.s = atomicAdd(ticket, 1u);
+        for (int r = 0; r < cl; ++r) tma::mbar_init(&S.xbar[r], 1);
+        tma::mbar_init_fence();
+        // one arrival (this one, declaring the bytes) plus a block per earlier rank
+        for (unsigned r = 0; r < rank; ++r) tma::mbar_expect_tx(&S.xbar[r], NB * sizeof(T));
+    }
+    if (cl > 1) {
+        // every CTA of the cluster has set up its barriers before any shared
+        // memory of another CTA is written
+        __syncthreads();
+        cluster_sync_all();
+        if (rank == 0 && t == 0) {
+            const unsigned c = atomicAdd(ticket, 1u);
+            for (unsigned r = 0; r < (unsigned)cl; ++r) st_cluster_u32(map_to(&S.cl, r), c);
+            if (c == gridDim.x / cl - 1) *ticket = 0u;  // every ticket of this launch is taken
+        }
+        cluster_sync_all();
+        if (t == 0) S.s = S.cl * cl + rank;
+    }
+    __syncthreads();
+    const int s = (int)S.s;
+    const unsigned epoch = S.epoch;
+    const int cfirst = cl > 1 ? (int)S.cl * cl : nb;  // first block (solve order) delivered by this cluster
+    if (cl == 1 && s == nb - 1 && t == 0) *ticket = 0u;
+    if (s >= nb) {  // a cluster's spare CTA past the last block
+        cluster_sync_all();
+        return;
+    }
+    auto blk = [&](int p) { return lower_op ? p : nb - 1 - p; };
+    const int kb = blk(s), r0 = kb * NB, nr = min(NB, n - r0);
+    // element (r, c) of op(A), before conjugation
+    auto at = [&](int r, int c) -> const T* { return op == 0 ? A + (long)c * lda + r : A + (long)r * lda + c; };
+    // thread layout of inv(D) and of every tile: rows R0 and R0 + 8 (next to
+    // each other in a stored block of x), columns cg + 8j
+    const int cg = lane & 7, R0 = (warp >> 1) * 16 + (warp & 1) * 4 + (lane >> 3);
+    // copies of a 64 x 64 tile: op N rows lane and lane + 32 of columns
+    // warp*8 .. +7, op T/C columns lane and lane + 32 of rows warp*8 .. +7
+    // (consecutive lanes read consecutive addresses)
+    const int ntile = max(0, s - 1), P = bpitch<T>(op);
+    auto fetch_to = [&](int i, int st) {
+        if (i >= 0) {
+            const int c0 = blk(i) * NB, nc = min(NB, n - c0);
+            T* dst = &S.stage[st][warp * 8 * P + lane];
+            const T* src = op == 0 ? at(r0 + lane, c0 + warp * 8) : at(r0 + warp * 8, c0 + lane);
+            const int nf = op == 0 ? nr : nc, ng = op == 0 ? nc : nr;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int f = 32 * (q & 1), g = q >> 1;
+                const bool in = lane + f < nf && warp * 8 + g < ng;
+                cp_async_elem(dst + g * P + f, in ? src + (long)g * lda + f : A, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto fetch = [&](int i) { fetch_to(i < ntile ? i : -1, i % kBStages); };
+    // this thread's share of a staged tile
+    auto read_tile = [&](int st, T(&m)[2][8]) {
+        const T* src = &S.stage[st][op == 0 ? cg * P + R0 : R0 * P + cg];
+        const int rs = op == 0 ? 8 : 8 * P, cs = op == 0 ? 8 * P : 8;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                m[k][j] = src[k * rs + j * cs];
+                if (op == 2) m[k][j] = conj_v(m[k][j]);
+            }
+    };
+    // the tile next to D first, in the last stage, which the ring reaches last
+    fetch_to(s - 1, kBStages - 1);
+    for (int i = 0; i < kBStages - 1; ++i) fetch(i);
+
+    // ---- diagonal block: D, then its FP64 inverse
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const int f = lane + 32 * (q & 1), g = warp * 8 + (q >> 1);
+        const int r = op == 0 ? f : g, c = op == 0 ? g : f;
+        T v = zero_v(T());
+        if (r < nr && c < nr) {
+            v = ldg(at(r0 + r, r0 + c));
+            if (op == 2) v = conj_v(v);
+        }
+        S.D[r][c] = v;
+    }
+    if (t < NB) S.y2[bidx<T>(t)] = t < nr ? x[(long)(r0 + t) * incx] : zero_v(T());  // b
+    __syncthreads();
+    if (t < NB) {
+        // thread t owns column j of the 16 x 16 diagonal block at o; the
+        // column stays in registers
+        const int o = t & ~15, j = t & 15;
+        W y[16];
+        auto solve_row = [&](int i, int k0, int k1) {
+            W acc;
+            dset(acc, i == j ? 1.0 : 0.0);
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (k >= k0 && k < k1) dmac(acc, dneg(wide(S.D[o + i][o + k])), y[k]);
+            return (unit || o + i >= nr) ? acc : dmul(acc, dinv(wide(S.D[o + i][o + i])));
+        };
+        if (lower_op) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                y[i] = solve_row(i, 0, i);
+                if (i < j) dset(y[i], 0.0);
+            }
+        } else {
+#pragma unroll
+            for (int i = 15; i >= 0; --i) {
+                y[i] = solve_row(i, i + 1, 16);
+                if (i > j) dset(y[i], 0.0);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) S.Y[o + i][o + j] = y[i];
+    }
+    __syncthreads();
+    // the product C Y11 (lower; C Y22 upper) waits in the block's mirror
+    // image, which the inverse does not use
+    // doubling (h = 16, then 32): the off-diagonal h x h block of each
+    // 2h x 2h diagonal block is -Y22 C Y11 (lower) or -Y11 C Y22 (upper);
+    // 32 / h products at a time, 2 x TC outputs per thread
+    auto doubling = [&](auto hc) {
+        constexpr int h = decltype(hc)::value;
+        constexpr int TPG = kThreads / (32 / h), TC = h / 16;
+        const int pr = t / TPG, u = t % TPG, o = pr * 2 * h;
+        const int tr = (u / 16) * 2, tcl = u % 16;
+        W acc[2][TC];
+        auto prod = [&](auto ea, auto eb) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) dset(acc[i][j], 0.0);
+#pragma unroll 4
+            for (int k = 0; k < h; ++k) {
+                W a[2], bb[TC];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) a[i] = ea(tr + i, k);
+#pragma unroll
+                for (int j = 0; j < TC; ++j) bb[j] = eb(k, tcl + 16 * j);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < TC; ++j) dmac(acc[i][j], a[i], bb[j]);
+            }
+        };
+        // rows and columns of the off-diagonal block C and of the two inverses
+        const int rl = lower_op ? o + h : o, cl0 = lower_op ? o : o + h;
+        prod([&](int r, int k) { return wide(S.D[rl + r][cl0 + k]); },
+             [&](int k, int c) { return S.Y[cl0 + k][cl0 + c]; });
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < TC; ++j) S.Y[cl0 + tr + i][rl + tcl + 16 * j] = acc[i][j];
+        __syncthreads();
+        prod([&](int r, int k) { return S.Y[rl + r][rl + k]; },
+             [&](int k, int c) { return S.Y[cl0 + k][rl + c]; });
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < TC; ++j) S.Y[rl + tr + i][cl0 + tcl + 16 * j] = dneg(acc[i][j]);
+        __syncthreads();
+        if (h < 32) {  // the next step reads this block with its zeros
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; ++j) dset(S.Y[cl0 + tr + i][rl + tcl + 16 * j], 0.0);
+            __syncthreads();
+        }
+    };
+    doubling(std::integral_constant<int, 16>{});
+    doubling(std::integral_constant<int, 32>{});
+
+    T iv[2][8], tc[2][8];
+    // element (r, c) of the inverse
+    auto inv_at = [&](int r, int c) {
+        return r < nr && c < nr && (lower_op ? c <= r : c >= r) ? narrow(S.Y[r][c]) : zero_v(T());
+    };
+    bool fin = true;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            iv[k][j] = inv_at(R0 + 8 * k, cg + 8 * j);
+            fin = fin && finite_v(iv[k][j]);
+        }
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 1) : "memory");
+    __syncthreads();  // the tile next to D has arrived
+    read_tile(kBStages - 1, tc);
+    const bool inv_ok = __syncthreads_and(fin);
+    // a[k] += row R0 + 8k of this thread's columns of M times its entries of v
+    auto load_x = [&](const T* v, T(&q)[8]) {
+        alignas(16) T w[8];
+#pragma unroll
+        for (int i = 0; i < 2 * kW; ++i)
+            reinterpret_cast<float4*>(w)[i] = *reinterpret_cast<const float4*>(&v[cg * kBGroup<T> + i * 4 / kW]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[j] = w[j];
+    };
+    auto mul = [&](const T(&m)[2][8], const T* v, T(&a)[2]) {
+        T q[8];
+        load_x(v, q);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            T b1 = zero_v(T());
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                madd_v(a[k], m[k][j], q[j]);
+                madd_v(b1, m[k][j + 1], q[j + 1]);
+            }
+            a[k] = addv(a[k], b1);
+        }
+    };
+    // the sums over the 8 threads that share rows, in each of them
+    auto share = [&](T(&a)[2]) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) a[k] = xor_add(a[k], o);
+    };
+
+    bool bad = false;
+    // the solved entries of the block with solve index p: delivered into this
+    // CTA's shared memory by an earlier CTA of the cluster (every thread
+    // waits on the transaction barrier), else polled from the published words
+    // into `buf` (the caller's barrier makes them visible)
+    auto poll_block = [&](int p, T* buf) {
+        const int c0 = blk(p) * NB, nc = min(NB, n - c0);
+        if (t < NB * kW) {
+            float v = 0.f;
+            if (t / kW < nc && !poll_word(pub + (long)c0 * kW + t, epoch, status, v)) bad = true;
+            reinterpret_cast<float*>(&buf[bidx<T>(t / kW)])[t % kW] = v;
+        }
+    };
+    auto wait_in = [&](int p) {
+        if (!xbar_wait_bounded(&S.xbar[p - cfirst], kTrsvWaitNs)) bad = true;
+        return (const T*)S.xin[p - cfirst];
+    };
+
+    // ---- the earlier blocks but the last, in solve order
+    T acc[2] = {zero_v(T()), zero_v(T())};
+    for (int i = 0; i < ntile; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 2) : "memory");
+        // two buffers: a thread that runs ahead writes the other one
+        if (i < cfirst) poll_block(i, S.xs[i & 1]);
+        // tile i has arrived, and every thread is done with tile i - 1
+        if (__syncthreads_or(bad)) { bad = true; break; }
+        fetch(i + kBStages - 1);
+        const T* xv = i >= cfirst ? wait_in(i) : S.xs[i & 1];
+        T m[2][8];
+        read_tile(i % kBStages, m);
+        mul(m, xv, acc);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+
+    // ---- this block's step of the chain
+    // hand-off: lane cg sends this thread's two rows to rank + 1 + cg
+    uint32_t dx = 0, db = 0;
+    if (cl > 1 && rank + 1 + cg < (unsigned)cl && cfirst + (int)rank + 1 + cg < nb) {
+        dx = map_to(&S.xin[rank][bidx<T>(R0)], rank + 1 + cg);
+        db = map_to(&S.xbar[rank], rank + 1 + cg);
+    }
+    // the solved entries of block s-1, once they are known (every thread calls it)
+    auto last_x = [&]() -> const T* {
+        if (s - 1 >= cfirst) return wait_in(s - 1);
+        poll_block(s - 1, S.xs[(s - 1) & 1]);
+        bad = __syncthreads_or(bad);
+        return S.xs[(s - 1) & 1];
+    };
+    // the b entry of the row this lane (cg < 2) writes to y2
+    const T brow = cg < 2 ? S.y2[bidx<T>(R0 + 8 * cg)] : zero_v(T());
+    if (!bad && s >= 1) mul(tc, last_x(), acc);
+    share(acc);
+    T o[2] = {zero_v(T()), zero_v(T())};
+    T yr = zero_v(T());
+    if (cg < 2) {
+        yr = subv(brow, cg == 0 ? acc[0] : acc[1]);
+        S.y2[bidx<T>(R0 + 8 * cg)] = yr;
+    }
+    // a wait failed, or a non-finite right-hand side
+    const int vote = __syncthreads_or((bad ? 1 : 0) | (finite_v(yr) && inv_ok ? 0 : 2));
+    if (vote == 0) {
+        mul(iv, S.y2, o);
+        share(o);
+    } else {
+        bad = __syncthreads_or(bad);
+        if (!bad) {
+            // substitution by one warp: each lane owns rows lane and lane + 32
+            if (warp == 0) {
+                T b0 = S.y2[bidx<T>(lane)], b1 = S.y2[bidx<T>(lane + 32)];
+                for (int kk = 0; kk < nr; ++kk) {
+                    const int k = lower_op ? kk : nr - 1 - kk;
+                    T bk = (k < 32) ? shfl(b0, k & 31) : shfl(b1, k & 31);
+                    if (!unit) bk = divv(bk, S.D[k][k]);
+                    if (lane == (k & 31)) { if (k < 32) b0 = bk; else b1 = bk; }
+                    const bool u0 = lower_op ? lane > k : lane < k, u1 = lower_op ? lane + 32 > k : lane + 32 < k;
+                    if (u0 && lane < nr) msub(b0, S.D[lane][k], bk);
+                    if (u1 && lane + 32 < nr) msub(b1, S.D[lane + 32][k], bk);
+                }
+                S.y2[bidx<T>(lane)] = b0;
+                S.y2[bidx<T>(lane + 32)] = b1;
+            }
+            __syncthreads();
+            o[0] = S.y2[bidx<T>(R0)];
+            o[1] = S.y2[bidx<T>(R0 + 8)];
+        }
+    }
+    if (!bad) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (R0 + 8 * k >= nr) o[k] = zero_v(T());
+        // the hand-offs first, then the published words; the output x last
+        if (db != 0 && cg == 0) st_async_pair(dx, o[0], o[1], db);
+        __syncwarp();
+        if (db != 0 && cg != 0) st_async_pair(dx, o[0], o[1], db);
+        const int k = cg / kW, row = R0 + 8 * k;
+        if (cg < 2 * kW && row < nr) {
+            const T v = k == 0 ? o[0] : o[1];
+            const float f = reinterpret_cast<const float*>(&v)[cg % kW];
+            st_relaxed_u64(pub + (long)(r0 + row) * kW + cg % kW, ((unsigned long long)epoch << 32) | __float_as_uint(f));
+            reinterpret_cast<float*>(&x[(long)(r0 + row) * incx])[cg % kW] = f;
+        }
+    } else {
+        atomicOr(status, (int)kDevWaitTimeout);
+    }
+    // after a failed wait, let bytes that other CTAs of the cluster may still
+    // send land before leaving (each wait bounded)
+    if (__syncthreads_or(bad) && t == 0)
+        for (unsigned r = 0; r < rank; ++r) xbar_wait_bounded(&S.xbar[r], kTrsvWaitNs);
+    if (t == 0 && s == nb - 1) *(volatile unsigned*)epoch_word = epoch;
+    if (cl > 1) cluster_sync_all();
 }
 
 // the number of clusters of CL CTAs of the STRSV kernel the current device
@@ -940,9 +1266,33 @@ int strsv_cluster_capacity(int device, int smem)
     return v - 1;
 }
 
+// Published-entry words for a solve of `words` values.  Calls that fit use
+// the handle's fixed area, which lives as long as the handle (a captured
+// launch may keep its address); only longer solves use the grown buffer.
+cudaError_t trsv_pub(iclblasHandle_t h, size_t words, unsigned long long** pub)
+{
+    if (words <= (size_t)kPubWords) {
+        *pub = reinterpret_cast<unsigned long long*>(h->ws.counters + kCounterWords);
+        return cudaSuccess;
+    }
+    if (words > h->ws.pub_elems) {
+        if (h->ws.pub) cudaFree(h->ws.pub);
+        h->ws.pub = nullptr;
+        h->ws.pub_elems = 0;
+        cudaError_t e = cudaMalloc(&h->ws.pub, words * sizeof(unsigned long long));
+        if (e != cudaSuccess) return e;
+        e = cudaMemsetAsync(h->ws.pub, 0, words * sizeof(unsigned long long), h->stream);
+        if (e != cudaSuccess) return e;
+        h->ws.pub_elems = words;
+    }
+    *pub = h->ws.pub;
+    return cudaSuccess;
+}
+
 template <int CL>
 cudaError_t strsv_launch(iclblasHandle_t h, int smem, int nb, const CUtensorMap& map, int n, int lower_op, int op,
-                         int unit, float* x, int incx, unsigned* ticket, unsigned* epoch_word)
+                         int unit, float* x, int incx, unsigned long long* pub, unsigned* ticket,
+                         unsigned* epoch_word)
 {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -957,7 +1307,7 @@ cudaError_t strsv_launch(iclblasHandle_t h, int smem, int nb, const CUtensorMap&
     cfg.attrs = attr;
     cfg.numAttrs = CL > 1 ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, strsv_tma_kernel<CL>, map, n, lower_op, op, unit, x, (long)incx,
-                                       h->ws.pub, ticket, epoch_word, h->ws.dev_status);
+                                       pub, ticket, epoch_word, h->ws.dev_status);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -970,16 +1320,9 @@ cudaError_t strsv_tma(iclblasHandle_t h, int uplo, int trans, int diag, int n, c
     // op N: boxes of 128 rows x 64 columns of A; op T: 64 rows x 128 columns
     if (lda < n || !tma::map_f32_colmajor(&map, A, n, n, lda, op == 0 ? RB : HB, op == 0 ? HB : RB))
         return cudaSuccess;
-    if ((size_t)n > h->ws.pub_elems) {
-        if (h->ws.pub) cudaFree(h->ws.pub);
-        h->ws.pub = nullptr;
-        h->ws.pub_elems = 0;
-        cudaError_t e = cudaMalloc(&h->ws.pub, (size_t)n * sizeof(unsigned long long));
-        if (e != cudaSuccess) return e;
-        e = cudaMemsetAsync(h->ws.pub, 0, (size_t)n * sizeof(unsigned long long), h->stream);
-        if (e != cudaSuccess) return e;
-        h->ws.pub_elems = n;
-    }
+    unsigned long long* pub = nullptr;
+    cudaError_t e = trsv_pub(h, (size_t)n, &pub);
+    if (e != cudaSuccess) return e;
     const int smem = (int)sizeof(FastSmem) + 1024;
     // the attribute belongs to the current device's copy of each kernel
     static std::atomic<unsigned long long> smem_set{0};
@@ -990,8 +1333,8 @@ cudaError_t strsv_tma(iclblasHandle_t h, int uplo, int trans, int diag, int n, c
                                  (const void*)strsv_tma_kernel<5>, (const void*)strsv_tma_kernel<6>,
                                  (const void*)strsv_tma_kernel<7>, (const void*)strsv_tma_kernel<8>};
         for (const void* k : kernels) {
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (e != cudaSuccess) return e;
+            if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+                return e;
         }
         smem_set.fetch_or(bit);
     }
@@ -1021,51 +1364,118 @@ cudaError_t strsv_tma(iclblasHandle_t h, int uplo, int trans, int diag, int n, c
             if (caps[c] > 0 && caps[c] * c >= nb) cl = c;
         if (!cl && caps[8] > 0) cl = 8;
         switch (cl) {
-        case 8: return strsv_launch<8>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 7: return strsv_launch<7>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 6: return strsv_launch<6>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 5: return strsv_launch<5>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 4: return strsv_launch<4>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 3: return strsv_launch<3>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
-        case 2: return strsv_launch<2>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
+        case 8: return strsv_launch<8>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 7: return strsv_launch<7>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 6: return strsv_launch<6>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 5: return strsv_launch<5>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 4: return strsv_launch<4>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 3: return strsv_launch<3>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+        case 2: return strsv_launch<2>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
         default: break;
         }
     }
-    return strsv_launch<1>(h, smem, nb, map, n, lower_op, op, unit, x, incx, ticket, epoch_word);
+    return strsv_launch<1>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+}
+
+// the number of clusters of `cl` CTAs of the block kernel the current device
+// holds at once (0: none), asked once per device and cluster size
+template <class T>
+int trsv_block_capacity(int device, int cl)
+{
+    static std::atomic<int> cap[64][kMaxCluster + 1];  // capacity + 1; 0: not asked yet
+    std::atomic<int>& c = cap[device & 63][cl];
+    int v = c.load();
+    if (v == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cl;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)cl);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = sizeof(BlockSmem<T>);
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, trsv_block_kernel<T>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        v = clusters + 1;
+        c.store(v);
+    }
+    return v - 1;
 }
 
 template <class T>
-cudaError_t trsv_impl(iclblasHandle_t h, int uplo, int trans, int diag, int n, const T* A, int lda, T* x, int incx)
+cudaError_t trsv_block(iclblasHandle_t h, int uplo, int trans, int diag, int n, const T* A, int lda, T* x, int incx)
 {
     const int nb = (n + NB - 1) / NB;
-    constexpr int kFlagBase = kCounterWords / 2;
     if (nb > kCounterWords / 2 - 1) return cudaErrorInvalidValue;
-    const int op = trans;  // 0 N, 1 T, 2 C (C == T for real data)
+    const int op = trans == ICLBLAS_OP_N ? 0 : (trans == ICLBLAS_OP_C && sizeof(T) == sizeof(cfloat)) ? 2 : 1;
     const bool lower = uplo == ICLBLAS_FILL_MODE_LOWER;
     const int lower_op = (op == 0) ? lower : !lower;
-    unsigned epoch = ++h->ws.epoch;
-    if (epoch == 0) epoch = ++h->ws.epoch;
-    unsigned* ticket = h->ws.counters;  // zero between launches
-    unsigned* flags = h->ws.counters + kFlagBase;
-    trsv_kernel<T><<<nb, kThreads, 0, h->stream>>>(n, lower_op, op, diag == ICLBLAS_DIAG_UNIT, A, lda, x, incx,
-                                                   ticket, flags, epoch, h->ws.dev_status);
-    return cudaGetLastError();
+    constexpr int kW = sizeof(T) / 4;
+    unsigned long long* pub = nullptr;
+    cudaError_t e = trsv_pub(h, (size_t)n * kW, &pub);
+    if (e != cudaSuccess) return e;
+    // the attribute belongs to the current device's copy of the kernel
+    static std::atomic<unsigned long long> smem_set{0};
+    const unsigned long long bit = 1ull << (h->device & 63);
+    if (!(smem_set.load() & bit)) {
+        e = cudaFuncSetAttribute(trsv_block_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(BlockSmem<T>));
+        if (e != cudaSuccess) return e;
+        smem_set.fetch_or(bit);
+    }
+    // the cluster size as for strsv_tma_kernel: the largest for which every
+    // cluster of the launch is resident at once, else 8, else none
+    int cl = 1;
+    if (nb > 1) {
+        for (int c = kMaxCluster; c >= 2 && cl == 1; --c) {
+            const int cap = trsv_block_capacity<T>(h->device, c);
+            if (cap > 0 && cap * c >= nb) cl = c;
+        }
+        if (cl == 1 && trsv_block_capacity<T>(h->device, kMaxCluster) > 0) cl = kMaxCluster;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cl;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)((nb + cl - 1) / cl * cl));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sizeof(BlockSmem<T>);
+    cfg.stream = h->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = cl > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, trsv_block_kernel<T>, cl, n, lower_op, op, (int)(diag == ICLBLAS_DIAG_UNIT), A,
+                           (long)lda, x, (long)incx, pub, h->ws.counters, h->ws.counters + kCounterWords - 1,
+                           h->ws.dev_status);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t strsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const float* A, int lda, float* x, int incx)
 {
-    bool used = false;
-    cudaError_t e = strsv_tma(h, uplo, trans, diag, n, A, lda, x, incx, used);
-    if (e != cudaSuccess || used) return e;
-    return trsv_impl<float>(h, uplo, trans == ICLBLAS_OP_C ? ICLBLAS_OP_T : trans, diag, n, A, lda, x, incx);
+    // short solves are bound by the time to the first block's inverse, which
+    // 64-row blocks have sooner (n = 512: 19 us against 30 with 128-row
+    // blocks, n = 1024 25 and 34, n = 2048 41 and 42, n = 3072 55 and 52)
+    if (n > 2048) {
+        bool used = false;
+        cudaError_t e = strsv_tma(h, uplo, trans, diag, n, A, lda, x, incx, used);
+        if (e != cudaSuccess || used) return e;
+    }
+    return trsv_block<float>(h, uplo, trans, diag, n, A, lda, x, incx);
 }
 
 cudaError_t ctrsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const cfloat* A, int lda, cfloat* x,
                   int incx)
 {
-    return trsv_impl<cfloat>(h, uplo, trans, diag, n, A, lda, x, incx);
+    return trsv_block<cfloat>(h, uplo, trans, diag, n, A, lda, x, incx);
 }
 
 }  // namespace iclb
