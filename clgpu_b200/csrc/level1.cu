@@ -12,6 +12,7 @@
 // test_nrm2.hpp:23-57, test_asum.hpp:23-33); iamax returns the reference's
 // 0-based first maximal index (tests/blas_reference/blas_reference.cpp:46-64)
 // exactly, for every n (no float-encoded indices).
+#include <algorithm>
 #include <climits>
 #include <mutex>
 
@@ -36,14 +37,36 @@ __host__ int l1_grid(iclblasHandle_t h, long units, int per_sm = 8)
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+// Launch shape of a reduction over n elements in `units` per-thread units.
+// Short vectors take one CTA of 1024 threads, which holds the whole sum: the
+// partials, fences and ticket between CTAs cost about 2.5 us, as much as
+// the rest of the call (n = 4099: 5.7 us with five CTAs).
+struct RedShape {
+    int grid, threads;
+};
+constexpr long kOneBlockElems = 16384;
+__host__ RedShape red_shape(iclblasHandle_t h, long n, long units, int per_sm)
+{
+    if (n <= kOneBlockElems) return {1, (int)std::min(1024L, (units + 31) / 32 * 32)};
+    return {l1_grid(h, units, per_sm), kThreads};
+}
+
 // ---------------------------------------------------------------- axpy/scal
 // y = fma(alpha, x, y): one rounding of alpha*x + y (the reference kernel
-// computes this_y += alpha*this_x, Saxpy_noinc.cl).
-__global__ void __launch_bounds__(kThreads) saxpy_vec(long n4, float alpha, const float4* __restrict__ x,
+// computes this_y += alpha*this_x, Saxpy_noinc.cl).  The n % 4 last elements
+// go to the first threads of the same launch: a launch of their own costs a
+// short vector about 3 us, as much as the whole of its other work.
+__global__ void __launch_bounds__(kThreads) saxpy_vec(long n, float alpha, const float4* __restrict__ x,
                                                       float4* __restrict__ y)
 {
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
+    const long stride = (long)gridDim.x * blockDim.x, n4 = n >> 2;
+    const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid < (n & 3)) {
+        const float* xt = (const float*)(x + n4);
+        float* yt = (float*)(y + n4);
+        yt[tid] = fmaf(alpha, xt[tid], yt[tid]);
+    }
+    for (long i = tid; i < n4; i += stride) {
         float4 a = ld_stream4(x + i), b = ld_stream4(y + i);
         b.x = fmaf(alpha, a.x, b.x);
         b.y = fmaf(alpha, a.y, b.y);
@@ -61,10 +84,12 @@ __global__ void __launch_bounds__(kThreads) saxpy_strided(long n, float alpha, c
         y[i * incy] = fmaf(alpha, x[i * incx], y[i * incy]);
 }
 
-__global__ void __launch_bounds__(kThreads) sscal_vec(long n4, float alpha, float4* __restrict__ x)
+__global__ void __launch_bounds__(kThreads) sscal_vec(long n, float alpha, float4* __restrict__ x)
 {
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
+    const long stride = (long)gridDim.x * blockDim.x, n4 = n >> 2;
+    const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid < (n & 3)) ((float*)(x + n4))[tid] *= alpha;
+    for (long i = tid; i < n4; i += stride) {
         float4 a = ld_stream4(x + i);
         a.x *= alpha; a.y *= alpha; a.z *= alpha; a.w *= alpha;
         __stcs(x + i, a);
@@ -146,8 +171,8 @@ __device__ __forceinline__ double rterm(float a, float b)
 }
 
 // Sum over i of term(x[i], y[i]).  VEC: unit stride, 16-byte aligned.
-template <Red OP, bool VEC>
-__global__ void __launch_bounds__(kThreads) sreduce_kernel(long n, const float* __restrict__ x, long incx,
+template <Red OP, bool VEC, int NT = kThreads>
+__global__ void __launch_bounds__(NT) sreduce_kernel(long n, const float* __restrict__ x, long incx,
                                                            const float* __restrict__ y, long incy,
                                                            double* __restrict__ partials, unsigned* counter,
                                                            float* __restrict__ result)
@@ -196,6 +221,10 @@ __global__ void __launch_bounds__(kThreads) sreduce_kernel(long n, const float* 
         }
     }
     double bs = block_sum(acc, sh);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *result = OP == Red::Nrm2 ? (float)sqrt(bs) : (float)bs;
+        return;
+    }
     if (threadIdx.x == 0) partials[blockIdx.x] = bs;
     if (!last_block(counter)) return;
     double s = 0.0;
@@ -217,8 +246,8 @@ __device__ __forceinline__ double cterm(float re, float im)
     return (double)re * (double)re + (double)im * (double)im;
 }
 
-template <Red OP, bool VEC>
-__global__ void __launch_bounds__(kThreads) creduce_kernel(long n, const cfloat* __restrict__ x, long incx,
+template <Red OP, bool VEC, int NT = kThreads>
+__global__ void __launch_bounds__(NT) creduce_kernel(long n, const cfloat* __restrict__ x, long incx,
                                                            double* __restrict__ partials, unsigned* counter,
                                                            float* __restrict__ result)
 {
@@ -253,6 +282,10 @@ __global__ void __launch_bounds__(kThreads) creduce_kernel(long n, const cfloat*
         }
     }
     double bs = block_sum(acc, sh);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *result = OP == Red::Nrm2 ? (float)sqrt(bs) : (float)bs;
+        return;
+    }
     if (threadIdx.x == 0) partials[blockIdx.x] = bs;
     if (!last_block(counter)) return;
     double s = 0.0;
@@ -265,8 +298,8 @@ __global__ void __launch_bounds__(kThreads) creduce_kernel(long n, const cfloat*
 }
 
 // cdotu / cdotc: sum conj?(x)*y in complex double (test_dot.hpp:22-51).
-template <bool CONJ, bool VEC>
-__global__ void __launch_bounds__(kThreads) cdot_kernel(long n, const cfloat* __restrict__ x, long incx,
+template <bool CONJ, bool VEC, int NT = kThreads>
+__global__ void __launch_bounds__(NT) cdot_kernel(long n, const cfloat* __restrict__ x, long incx,
                                                         const cfloat* __restrict__ y, long incy,
                                                         double* __restrict__ partials, unsigned* counter,
                                                         cfloat* __restrict__ result)
@@ -307,6 +340,10 @@ __global__ void __launch_bounds__(kThreads) cdot_kernel(long n, const cfloat* __
     }
     double bre = block_sum(re, sh);
     double bim = block_sum(im, sh);
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) *result = cfloat{(float)bre, (float)bim};
+        return;
+    }
     if (threadIdx.x == 0) {
         partials[2 * blockIdx.x] = bre;
         partials[2 * blockIdx.x + 1] = bim;
@@ -384,8 +421,8 @@ __device__ __forceinline__ float iakey(T v)
     return MIN ? -absval(v) : absval(v);
 }
 
-template <class T, bool VEC, bool MIN = false>
-__global__ void __launch_bounds__(kThreads) iamax_kernel(long n, const T* __restrict__ x, long incx,
+template <class T, bool VEC, bool MIN = false, int NT = kThreads>
+__global__ void __launch_bounds__(NT) iamax_kernel(long n, const T* __restrict__ x, long incx,
                                                          Cand* __restrict__ partials, unsigned* counter,
                                                          int* __restrict__ result)
 {
@@ -422,6 +459,15 @@ __global__ void __launch_bounds__(kThreads) iamax_kernel(long n, const T* __rest
         for (long i = tid; i < n; i += stride) cand_take(c, iakey<MIN>(x[i * incx]), (int)i);
     }
     Cand b = block_cand(c, sh);
+    auto finish = [&](Cand r) {
+        int idx = r.i;
+        if (isnan_v(x[0]) || idx == INT_MAX) idx = 0;
+        *result = idx;
+    };
+    if (gridDim.x == 1) {
+        if (threadIdx.x == 0) finish(b);
+        return;
+    }
     if (threadIdx.x == 0) partials[blockIdx.x] = b;
     if (!last_block(counter)) return;
     Cand r{-INFINITY, INT_MAX};
@@ -433,9 +479,7 @@ __global__ void __launch_bounds__(kThreads) iamax_kernel(long n, const T* __rest
     }
     r = block_cand(r, sh);
     if (threadIdx.x == 0) {
-        int idx = r.i;
-        if (isnan_v(x[0]) || idx == INT_MAX) idx = 0;
-        *result = idx;
+        finish(r);
         *counter = 0u;
     }
 }
@@ -446,10 +490,7 @@ __global__ void __launch_bounds__(kThreads) iamax_kernel(long n, const T* __rest
 cudaError_t saxpy(iclblasHandle_t h, int n, float alpha, const float* x, int incx, float* y, int incy)
 {
     if (incx == 1 && incy == 1 && aligned16(x) && aligned16(y)) {
-        long n4 = n >> 2;
-        if (n4 > 0) saxpy_vec<<<l1_grid(h, n4, 4), kThreads, 0, h->stream>>>(n4, alpha, (const float4*)x, (float4*)y);
-        long rem = n - n4 * 4;
-        if (rem > 0) saxpy_strided<<<1, 32, 0, h->stream>>>(rem, alpha, x + n4 * 4, 1, y + n4 * 4, 1);
+        saxpy_vec<<<l1_grid(h, n >> 2, 4), kThreads, 0, h->stream>>>(n, alpha, (const float4*)x, (float4*)y);
     } else {
         saxpy_strided<<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx, y, incy);
     }
@@ -459,10 +500,7 @@ cudaError_t saxpy(iclblasHandle_t h, int n, float alpha, const float* x, int inc
 cudaError_t sscal(iclblasHandle_t h, int n, float alpha, float* x, int incx)
 {
     if (incx == 1 && aligned16(x)) {
-        long n4 = n >> 2;
-        if (n4 > 0) sscal_vec<<<l1_grid(h, n4), kThreads, 0, h->stream>>>(n4, alpha, (float4*)x);
-        long rem = n - n4 * 4;
-        if (rem > 0) sscal_strided<<<1, 32, 0, h->stream>>>(rem, alpha, x + n4 * 4, 1);
+        sscal_vec<<<l1_grid(h, n >> 2), kThreads, 0, h->stream>>>(n, alpha, (float4*)x);
     } else {
         sscal_strided<<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx);
     }
@@ -491,12 +529,18 @@ cudaError_t sreduce(iclblasHandle_t h, Red op, int n, const float* x, int incx, 
                     float* result)
 {
     const bool vec = incx == 1 && aligned16(x) && (op != Red::Dot || (incy == 1 && aligned16(y)));
-    const int grid = l1_grid(h, vec ? ((long)n + 3) / 4 : n, op == Red::Asum ? 6 : 8);
-    double* partials = (double*)scratch(h, sizeof(double) * (size_t)grid);
-    if (!partials) return cudaErrorMemoryAllocation;
+    const RedShape g = red_shape(h, n, vec ? ((long)n + 3) / 4 : n, op == Red::Asum ? 6 : 8);
+    double* partials = nullptr;
+    if (g.grid > 1 && !(partials = (double*)scratch(h, sizeof(double) * (size_t)g.grid)))
+        return cudaErrorMemoryAllocation;
     unsigned* ctr = h->ws.counters;
-#define LAUNCH(OP, V) \
-    sreduce_kernel<OP, V><<<grid, kThreads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result)
+#define LAUNCH(OP, V)                                                                                            \
+    do {                                                                                                         \
+        if (g.grid > 1)                                                                                          \
+            sreduce_kernel<OP, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+        else                                                                                                     \
+            sreduce_kernel<OP, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+    } while (0)
     switch (op) {
     case Red::Dot: if (vec) LAUNCH(Red::Dot, true); else LAUNCH(Red::Dot, false); break;
     case Red::Asum: if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false); break;
@@ -583,37 +627,50 @@ cudaError_t noalloc_scratch_addr(int device, SdotNoAllocScratch** out)
 cudaError_t sdot_noalloc(iclblasHandle_t h, int n, const float* x, int incx, const float* y, int incy, float* result)
 {
     const bool vec = incx == 1 && aligned16(x) && incy == 1 && aligned16(y);
-    const int grid = l1_grid(h, vec ? ((long)n + 3) / 4 : n);
-    if (grid > kSdotNoAllocMaxBlocks) return cudaErrorNotSupported;
+    const RedShape g = red_shape(h, n, vec ? ((long)n + 3) / 4 : n, 8);
+    if (g.grid > kSdotNoAllocMaxBlocks) return cudaErrorNotSupported;
     SdotNoAllocScratch* sc = nullptr;
     cudaError_t e = noalloc_scratch_addr(h->device, &sc);
     if (e != cudaSuccess) return e;
+    if (g.grid == 1) {
+        if (vec)
+            sreduce_kernel<Red::Dot, true, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
+                                                                                 &sc->counter, result);
+        else
+            sreduce_kernel<Red::Dot, false, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
+                                                                                  &sc->counter, result);
+        return cudaGetLastError();
+    }
     // the array keeps the previous call's contents: the ticket must start at 0
     e = cudaMemsetAsync(&sc->counter, 0, sizeof(unsigned), h->stream);
     if (e != cudaSuccess) return e;
     if (vec)
-        sreduce_kernel<Red::Dot, true><<<grid, kThreads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                          &sc->counter, result);
+        sreduce_kernel<Red::Dot, true><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
+                                                                            &sc->counter, result);
     else
-        sreduce_kernel<Red::Dot, false><<<grid, kThreads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                           &sc->counter, result);
+        sreduce_kernel<Red::Dot, false><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
+                                                                             &sc->counter, result);
     return cudaGetLastError();
 }
 
 cudaError_t creduce_real(iclblasHandle_t h, Red op, int n, const cfloat* x, int incx, float* result)
 {
     const bool vec = incx == 1 && aligned16(x);
-    const int grid = l1_grid(h, vec ? ((long)n + 1) / 2 : n);
-    double* partials = (double*)scratch(h, sizeof(double) * (size_t)grid);
-    if (!partials) return cudaErrorMemoryAllocation;
+    const RedShape g = red_shape(h, n, vec ? ((long)n + 1) / 2 : n, 8);
+    double* partials = nullptr;
+    if (g.grid > 1 && !(partials = (double*)scratch(h, sizeof(double) * (size_t)g.grid)))
+        return cudaErrorMemoryAllocation;
     unsigned* ctr = h->ws.counters;
-    if (op == Red::Asum) {
-        if (vec) creduce_kernel<Red::Asum, true><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, ctr, result);
-        else creduce_kernel<Red::Asum, false><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, ctr, result);
-    } else {
-        if (vec) creduce_kernel<Red::Nrm2, true><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, ctr, result);
-        else creduce_kernel<Red::Nrm2, false><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, ctr, result);
-    }
+#define LAUNCH(OP, V)                                                                                        \
+    do {                                                                                                     \
+        if (g.grid > 1)                                                                                      \
+            creduce_kernel<OP, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);   \
+        else                                                                                                 \
+            creduce_kernel<OP, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);  \
+    } while (0)
+    if (op == Red::Asum) { if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false); }
+    else { if (vec) LAUNCH(Red::Nrm2, true); else LAUNCH(Red::Nrm2, false); }
+#undef LAUNCH
     return cudaGetLastError();
 }
 
@@ -621,11 +678,18 @@ cudaError_t cdot(iclblasHandle_t h, bool conj, int n, const cfloat* x, int incx,
                  cfloat* result)
 {
     const bool vec = incx == 1 && incy == 1 && aligned16(x) && aligned16(y);
-    const int grid = l1_grid(h, vec ? ((long)n + 1) / 2 : n);
-    double* partials = (double*)scratch(h, 2 * sizeof(double) * (size_t)grid);
-    if (!partials) return cudaErrorMemoryAllocation;
+    const RedShape g = red_shape(h, n, vec ? ((long)n + 1) / 2 : n, 8);
+    double* partials = nullptr;
+    if (g.grid > 1 && !(partials = (double*)scratch(h, 2 * sizeof(double) * (size_t)g.grid)))
+        return cudaErrorMemoryAllocation;
     unsigned* ctr = h->ws.counters;
-#define LAUNCH(C, V) cdot_kernel<C, V><<<grid, kThreads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result)
+#define LAUNCH(C, V)                                                                                           \
+    do {                                                                                                       \
+        if (g.grid > 1)                                                                                        \
+            cdot_kernel<C, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+        else                                                                                                   \
+            cdot_kernel<C, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+    } while (0)
     if (conj) { if (vec) LAUNCH(true, true); else LAUNCH(true, false); }
     else { if (vec) LAUNCH(false, true); else LAUNCH(false, false); }
 #undef LAUNCH
@@ -637,13 +701,20 @@ template <class T, bool MIN>
 cudaError_t iamax_impl(iclblasHandle_t h, int n, const T* x, int incx, int* result)
 {
     const bool vec = incx == 1 && aligned16(x);
-    const int grid = l1_grid(h, vec ? ((long)n + (16 / sizeof(T)) - 1) / (16 / sizeof(T)) : n, 6);
-    Cand* partials = (Cand*)scratch(h, sizeof(Cand) * (size_t)grid);
-    if (!partials) return cudaErrorMemoryAllocation;
-    if (vec)
-        iamax_kernel<T, true, MIN><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, h->ws.counters, result);
-    else
-        iamax_kernel<T, false, MIN><<<grid, kThreads, 0, h->stream>>>(n, x, incx, partials, h->ws.counters, result);
+    const RedShape g = red_shape(h, n, vec ? ((long)n + (16 / sizeof(T)) - 1) / (16 / sizeof(T)) : n, 6);
+    Cand* partials = nullptr;
+    if (g.grid > 1 && !(partials = (Cand*)scratch(h, sizeof(Cand) * (size_t)g.grid)))
+        return cudaErrorMemoryAllocation;
+    unsigned* ctr = h->ws.counters;
+#define LAUNCH(V)                                                                                                \
+    do {                                                                                                         \
+        if (g.grid > 1)                                                                                          \
+            iamax_kernel<T, V, MIN><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);     \
+        else                                                                                                     \
+            iamax_kernel<T, V, MIN, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);    \
+    } while (0)
+    if (vec) LAUNCH(true); else LAUNCH(false);
+#undef LAUNCH
     return cudaGetLastError();
 }
 }  // namespace

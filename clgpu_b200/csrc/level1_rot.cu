@@ -142,17 +142,29 @@ struct RotmOp {
 };
 
 // ---------------------------------------------------------------- kernels
-// 128-bit path: n4 float4 words of each vector; T is the element type the
-// op is defined on (four floats or two complex per word).  Op::kUnroll words
-// per thread per iteration, grid-strided.
+// 128-bit path over n elements; T is the element type the op is defined on
+// (four floats or two complex per float4 word).  Op::kUnroll words per thread
+// per iteration, grid-strided; the elements past the last whole word go to
+// the first threads (a launch of their own would cost a short call as much
+// as the rest of it).
 template <class T, class Op>
-__global__ void __launch_bounds__(kThreads) pair_vec_kernel(long n4, float4* x, float4* y, Op op)
+__global__ void __launch_bounds__(kThreads) pair_vec_kernel(long n, float4* x, float4* y, Op op)
 {
     if (!op.prepare()) return;
     constexpr int per = (int)(16 / sizeof(T));
     constexpr int U = Op::kUnroll;
-    const long stride = (long)gridDim.x * blockDim.x;
+    const long stride = (long)gridDim.x * blockDim.x, n4 = n / per;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n % per) {
+        T* xt = (T*)(x + n4) + i;
+        T* yt = (T*)(y + n4) + i;
+        T a = *xt;
+        T b{};
+        if (Op::kReadY) b = *yt;
+        op(a, b);
+        if (Op::kWriteX) *xt = a;
+        *yt = b;
+    }
     for (; i + (U - 1) * stride < n4; i += U * stride) {
         float4 a[U], b[U];
 #pragma unroll
@@ -197,22 +209,17 @@ __global__ void __launch_bounds__(kThreads) pair_strided_kernel(long n, T* x, lo
     }
 }
 
-// Unit strides with both bases 16-byte aligned: the vector path over whole
-// words plus a one-warp tail; otherwise the strided path.
+// Unit strides with both bases 16-byte aligned: the vector path; otherwise
+// the strided path.
 template <class T, class Op>
 cudaError_t run_pair(iclblasHandle_t h, long n, T* x, long incx, T* y, long incy, Op op)
 {
     if (incx == 1 && incy == 1 && aligned16(x) && aligned16(y)) {
         constexpr long per = 16 / sizeof(T);
         const long n4 = n / per;
-        if (n4 > 0) {
-            long g = (n4 + (long)kThreads * Op::kUnroll - 1) / ((long)kThreads * Op::kUnroll);
-            g = std::min<long>(g, 4L * h->sm_count);
-            pair_vec_kernel<T, Op><<<(int)g, kThreads, 0, h->stream>>>(n4, (float4*)x, (float4*)y, op);
-        }
-        const long rem = n - n4 * per;
-        if (rem > 0)
-            pair_strided_kernel<T, Op><<<1, 32, 0, h->stream>>>(rem, x + n4 * per, 1, y + n4 * per, 1, op);
+        long g = (n4 + (long)kThreads * Op::kUnroll - 1) / ((long)kThreads * Op::kUnroll);
+        g = std::max(1L, std::min<long>(g, 4L * h->sm_count));
+        pair_vec_kernel<T, Op><<<(int)g, kThreads, 0, h->stream>>>(n, (float4*)x, (float4*)y, op);
     } else {
         pair_strided_kernel<T, Op><<<grid_for(h, n), kThreads, 0, h->stream>>>(n, x, incx, y, incy, op);
     }
