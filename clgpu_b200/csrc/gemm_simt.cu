@@ -9,11 +9,27 @@
 // Because every thread keeps whole outputs and walks k in order, a result is
 // bit-identical to the serial oracle for the same inputs.
 //
-// Structure: register-tiled CTA tiles (BM x BN, BK = 8) staged through
-// double-buffered shared memory with register prefetch of the next k tile;
-// the global loads are arranged so consecutive threads read consecutive
-// addresses for each operand layout (op N vs T/C).
+// Structure: register-tiled CTA tiles (BM x BN) whose operands arrive by
+// cp.async, one element per copy, in a ring of shared-memory stages, always
+// k-major: the copies of an operand that is contiguous along k (A of op T/C,
+// B of op N) scatter into that layout, so neither the layout nor the
+// alignment of an operand changes the main loop, no register holds data in
+// flight, and K tiles are under way while earlier ones are multiplied.
+//
+// What bounds it: large products the FMA pipe (ncu at 4096^3: 72-76 % busy,
+// warps waiting for it) together with shared-memory reads (69 %: a 16-byte
+// read costs four passes however many lanes share the address, so 8 x 8
+// outputs a thread spend as many cycles reading as multiplying); small ones
+// the latency of one k step times k, since each output sums k in order.
+// Against register-staged tiles of the same shapes (us before, after):
+// 8192 x 8192 x 4096 NN 11981, 11112, TN 11978, 10524; 2000 x 1500 x 3001 TN
+// with odd leading dimensions 670, 463; 1000^3 98.4, 68.6; 512^3 34.9, 18.5;
+// 256^3 18.5, 8.3; 128 x 100 x 3000 171, 41.  Complex: 4096 x 4096 x 2048 NN
+// 6185, 6226, TN 6456, 6004; 1000 x 750 x 1500 TN 375, 301; 500^3 61.5, 41.0;
+// (re, im) pairs updated by fma.rn.f32x2 measured 10 % slower than scalar
+// FMAs there.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -26,7 +42,6 @@ __device__ __forceinline__ cfloat conj_if(cfloat v, bool c) { return c ? cfloat{
 __device__ __forceinline__ float zero_v(float) { return 0.f; }
 __device__ __forceinline__ cfloat zero_v(cfloat) { return cfloat{0.f, 0.f}; }
 
-__device__ __forceinline__ void mac(float& acc, float a, float b) { acc = fmaf(a, b, acc); }
 __device__ __forceinline__ void mac(cfloat& acc, cfloat a, cfloat b)
 {
     acc.re = fmaf(a.re, b.re, acc.re);
@@ -99,164 +114,210 @@ __device__ __forceinline__ void lds_vec(T* dst, const T* src)
     }
 }
 
-// Threads: (BM/TM) x (BN/TN).  Each thread owns TM x TN outputs split in two
-// halves along each dimension (rows ty*TM/2 + {0..TM/2-1} and
-// BM/2 + ty*TM/2 + ...) so its shared-memory reads are conflict-free vectors.
-template <class T, int BM, int BN, int BK, int TM, int TN>
+__device__ __forceinline__ void cp_async_elem(float* dst, const float* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(in ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_elem(cfloat* dst, const cfloat* src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(in ? 8 : 0)
+                 : "memory");
+}
+
+// Threads: (BM/TM) x (BN/TN).  Each thread owns TM x TN outputs in runs of VA
+// rows and VB columns (16 bytes, or all it has) spread evenly over the tile,
+// so its shared-memory reads are conflict-free vectors.
+// The warp covers 4 thread rows x 8 thread columns: a fragment read then
+// touches 4 or 8 distinct vectors, one shared-memory pass each.
+// ST: stages of the ring.  MB: CTAs per SM the registers are bounded for.
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST>
 struct Cfg {
     static constexpr int TX = BN / TN, TY = BM / TM, NT = TX * TY;
     static constexpr int A_PER = BM * BK / NT, B_PER = BN * BK / NT;
+    // rows apart: copies that scatter (8 consecutive k of 2 or 4 rows a
+    // warp) fall in different banks, and fragment reads stay 16-byte aligned
+    static constexpr int VA = TM < 16 / (int)sizeof(T) ? TM : 16 / (int)sizeof(T), NA = TM / VA;
+    static constexpr int VB = TN < 16 / (int)sizeof(T) ? TN : 16 / (int)sizeof(T), NB = TN / VB;
+    static constexpr int PAD = 16 / (int)sizeof(T);
+    static constexpr int A_EL = BK * (BM + PAD), B_EL = BK * (BN + PAD);
+    static constexpr int SMEM = ST * (A_EL + B_EL) * (int)sizeof(T);
     static_assert(A_PER * NT == BM * BK && B_PER * NT == BN * BK, "tile/thread mismatch");
+    static_assert(TX % 8 == 0 && TY % 4 == 0 && BK % 8 == 0 && NT % 32 == 0, "warp layout");
+    static_assert(NT % BM == 0 || BM % NT == 0, "copy layout");
+    static_assert(NT % BN == 0 || BN % NT == 0, "copy layout");
 };
 
-template <class T, int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN>::NT)
+// Copies of one operand's BX x BK tile into [kk][i] (pitch PX).  CONTIG_K:
+// element (i, kk) at p[i*ld + kk], else at p[kk*ld + i].
+template <class T, int BX, int BK, int NT, int PX>
+struct TileCopy {
+    static constexpr int PER = BX * BK / NT;
+    const T* base;   // first element this thread copies, at k = 0
+    long ld;
+    bool contig_k;
+    int i0, kk0;     // its row and k
+    int rows;        // rows of the operand from the tile's first
+    __device__ TileCopy(const T* p, long ld_, bool ck, int x0, int nx) : ld(ld_), contig_k(ck), rows(nx - x0)
+    {
+        const int t = threadIdx.x;
+        if (ck) { kk0 = t % 8; i0 = t / 8; } else { i0 = t % BX; kk0 = t / BX; }
+        base = p + (ck ? (long)(x0 + i0) * ld + kk0 : (long)kk0 * ld + x0 + i0);
+    }
+    __device__ void copy(T* dst, int k0, int k) const
+    {
+        if (contig_k) {
+            constexpr int KH = BK / 8, RS = NT / 8;   // k octets; rows per pass
+            const T* src = base + k0;
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int kk = 8 * (q % KH), i = (q / KH) * RS;
+                const bool in = i0 + i < rows && k0 + kk0 + kk < k;
+                cp_async_elem(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)i * ld + kk : base, in);
+            }
+        } else {
+            constexpr int KS = NT >= BX ? NT / BX : 1, IP = NT >= BX ? 1 : BX / NT;   // k per pass; row passes
+            const T* src = base + (long)k0 * ld;
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int kk = (q / IP) * KS, i = (q % IP) * NT;
+                const bool in = i0 + i < rows && k0 + kk0 + kk < k;
+                cp_async_elem(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)kk * ld + i : base, in);
+            }
+        }
+    }
+};
+
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB>
+__global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     gemm_simt_kernel(int ta, int tb, int m, int n, int k, T alpha, const T* __restrict__ A, long lda,
                      const T* __restrict__ B, long ldb, T beta, T* __restrict__ C, long ldc, int tri)
 {
-    using CF = Cfg<T, BM, BN, BK, TM, TN>;
-    constexpr int NT = CF::NT, TX = CF::TX;
-    // rows padded by 4 elements: the k-contiguous operand's stores (consecutive
-    // kk in a warp) fall in different banks, and fragment reads stay aligned
-    __shared__ __align__(16) T As[2][BK][BM + 4];
-    __shared__ __align__(16) T Bs[2][BK][BN + 4];
+    using CF = Cfg<T, BM, BN, BK, TM, TN, ST>;
+    constexpr int NT = CF::NT, TX = CF::TX, PA = BM + CF::PAD, PB = BN + CF::PAD;
+    extern __shared__ __align__(16) unsigned char simt_smem[];
+    T* As = reinterpret_cast<T*>(simt_smem);  // [stage][kk][i]
+    T* Bs = As + ST * CF::A_EL;
 
-    const int tid = threadIdx.x;
-    const int tx = tid % TX, ty = tid / TX;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int WX = TX / 8;  // warps along n
+    const int ty = (warp / WX) * 4 + lane / 8, tx = (warp % WX) * 8 + lane % 8;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed;
     // tiles wholly outside it have no work
     if ((tri == 1 && m0 + BM - 1 < n0) || (tri == 2 && m0 > n0 + BN - 1)) return;
-    const bool a_trans = ta != ICLBLAS_OP_N, a_conj = ta == ICLBLAS_OP_C;
-    const bool b_trans = tb != ICLBLAS_OP_N, b_conj = tb == ICLBLAS_OP_C;
+    const bool a_conj = ta == ICLBLAS_OP_C, b_conj = tb == ICLBLAS_OP_C;
+    const TileCopy<T, BM, BK, NT, PA> ca(A, lda, ta != ICLBLAS_OP_N, m0, m);
+    const TileCopy<T, BN, BK, NT, PB> cb(B, ldb, tb == ICLBLAS_OP_N, n0, n);
 
-    T ra[CF::A_PER], rb[CF::B_PER];
-
-    // Element e of the A tile (BM x BK): op N reads down columns of A
-    // (contiguous in i), op T/C along rows (contiguous in kk).
-    auto load_a = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < CF::A_PER; ++q) {
-            const int e = tid + q * NT;
-            int i, kk;
-            if (!a_trans) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-            const int gi = m0 + i, gk = k0 + kk;
-            T v = zero_v(T());
-            if (gi < m && gk < k) v = a_trans ? conj_if(A[(long)gi * lda + gk], a_conj) : A[(long)gk * lda + gi];
-            ra[q] = v;
-        }
-    };
-    auto store_a = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < CF::A_PER; ++q) {
-            const int e = tid + q * NT;
-            int i, kk;
-            if (!a_trans) { i = e % BM; kk = e / BM; } else { kk = e % BK; i = e / BK; }
-            As[buf][kk][i] = ra[q];
-        }
-    };
-    // Element e of the B tile (BK x BN): op N contiguous in kk, op T/C in j.
-    auto load_b = [&](int k0) {
-#pragma unroll
-        for (int q = 0; q < CF::B_PER; ++q) {
-            const int e = tid + q * NT;
-            int j, kk;
-            if (!b_trans) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-            const int gj = n0 + j, gk = k0 + kk;
-            T v = zero_v(T());
-            if (gj < n && gk < k) v = b_trans ? conj_if(B[(long)gk * ldb + gj], b_conj) : B[(long)gj * ldb + gk];
-            rb[q] = v;
-        }
-    };
-    auto store_b = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < CF::B_PER; ++q) {
-            const int e = tid + q * NT;
-            int j, kk;
-            if (!b_trans) { kk = e % BK; j = e / BK; } else { j = e % BN; kk = e / BN; }
-            Bs[buf][kk][j] = rb[q];
-        }
-    };
-
-    // float: accumulators in pairs along j (acc[i][2j], acc[i][2j+1])
-    constexpr bool kPair = std::is_same<T, float>::value && TN % 2 == 0;
+    // float: accumulators in pairs along the longer dimension of the thread's
+    // outputs (fewer values of the other operand to duplicate)
+    constexpr bool kPair = std::is_same<T, float>::value, kPairI = kPair && TM > TN;
     using AccT = std::conditional_t<kPair, unsigned long long, T>;
-    constexpr int TNA = kPair ? TN / 2 : TN;
-    AccT acc[TM][TNA];
+    constexpr int TMA = kPairI ? TM / 2 : TM, TNA = kPair && !kPairI ? TN / 2 : TN;
+    AccT acc[TMA][TNA];
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TMA; ++i)
 #pragma unroll
         for (int j = 0; j < TNA; ++j) {
             if constexpr (kPair) acc[i][j] = 0ull;  // (+0.f, +0.f)
             else acc[i][j] = zero_v(T());
         }
     auto acc_at = [&](int i, int j) -> T {
-        if constexpr (kPair) return half2f(acc[i][j >> 1], j & 1);
+        if constexpr (kPairI) return half2f(acc[i >> 1][j], i & 1);
+        else if constexpr (kPair) return half2f(acc[i][j >> 1], j & 1);
         else return acc[i][j];
     };
 
     const int ktiles = (k + BK - 1) / BK;
-    if (ktiles > 0) {
-        load_a(0);
-        load_b(0);
-        store_a(0);
-        store_b(0);
-    }
-    __syncthreads();
-    for (int t = 0; t < ktiles; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < ktiles) {
-            load_a((t + 1) * BK);
-            load_b((t + 1) * BK);
+    auto fetch = [&](int t) {
+        if (t < ktiles) {
+            ca.copy(As + (t % ST) * CF::A_EL, t * BK, k);
+            cb.copy(Bs + (t % ST) * CF::B_EL, t * BK, k);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int t = 0; t < ST - 1; ++t) fetch(t);
+    for (int t = 0; t < ktiles; ++t) {
+        // tile t has arrived, and every thread is done with tile t - 1,
+        // whose stage the next copies overwrite
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();
+        fetch(t + ST - 1);
+        const T* at = As + (t % ST) * CF::A_EL + ty * CF::VA;
+        const T* bt = Bs + (t % ST) * CF::B_EL + tx * CF::VB;
+        // fragments of k kk + 1 are read while those of kk are multiplied
+        T a[2][TM], b[2][TN];
+        auto read = [&](int kk) {
+            T* fa = a[kk & 1];
+            T* fb = b[kk & 1];
+#pragma unroll
+            for (int q = 0; q < CF::NA; ++q) lds_vec<T, CF::VA>(fa + q * CF::VA, at + kk * PA + q * (BM / CF::NA));
+#pragma unroll
+            for (int q = 0; q < CF::NB; ++q) lds_vec<T, CF::VB>(fb + q * CF::VB, bt + kk * PB + q * (BN / CF::NB));
+        };
+        read(0);
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
-            T a[TM], b[TN];
-            lds_vec<T, TM / 2>(a, &As[buf][kk][ty * (TM / 2)]);
-            lds_vec<T, TM / 2>(a + TM / 2, &As[buf][kk][BM / 2 + ty * (TM / 2)]);
-            lds_vec<T, TN / 2>(b, &Bs[buf][kk][tx * (TN / 2)]);
-            lds_vec<T, TN / 2>(b + TN / 2, &Bs[buf][kk][BN / 2 + tx * (TN / 2)]);
-            if constexpr (kPair) {
-                unsigned long long bp[TN / 2];
+            if (kk + 1 < BK) read(kk + 1);
+            T* fa = a[kk & 1];
+            T* fb = b[kk & 1];
+            if constexpr (!std::is_same<T, float>::value) {
 #pragma unroll
-                for (int j = 0; j < TN / 2; ++j) bp[j] = pack2(b[2 * j], b[2 * j + 1]);
+                for (int i = 0; i < TM; ++i) fa[i] = conj_if(fa[i], a_conj);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) fb[j] = conj_if(fb[j], b_conj);
+            }
+            if constexpr (kPairI) {
+                unsigned long long ap[TMA];
+#pragma unroll
+                for (int i = 0; i < TMA; ++i) ap[i] = pack2(fa[2 * i], fa[2 * i + 1]);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const unsigned long long bp = pack2(fb[j], fb[j]);
+#pragma unroll
+                    for (int i = 0; i < TMA; ++i) mac2(acc[i][j], ap[i], bp);
+                }
+            } else if constexpr (kPair) {
+                unsigned long long bp[TNA];
+#pragma unroll
+                for (int j = 0; j < TNA; ++j) bp[j] = pack2(fb[2 * j], fb[2 * j + 1]);
 #pragma unroll
                 for (int i = 0; i < TM; ++i) {
-                    const unsigned long long ap = pack2(a[i], a[i]);
+                    const unsigned long long ap = pack2(fa[i], fa[i]);
 #pragma unroll
-                    for (int j = 0; j < TN / 2; ++j) mac2(acc[i][j], ap, bp[j]);
+                    for (int j = 0; j < TNA; ++j) mac2(acc[i][j], ap, bp[j]);
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) mac(acc[i][j], a[i], b[j]);
+                    for (int j = 0; j < TN; ++j) mac(acc[i][j], fa[i], fb[j]);
             }
         }
-        if (t + 1 < ktiles) {
-            store_a(buf ^ 1);
-            store_b(buf ^ 1);
-        }
-        __syncthreads();
     }
 
     // the row's C values are all loaded before any is stored, so the loads
     // overlap (C is read only when beta != 0)
     const bool read_c = !is_zero(beta);
+    auto col = [&](int j) { return n0 + (j / CF::VB) * (BN / CF::NB) + tx * CF::VB + j % CF::VB; };
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int gi = m0 + (i < TM / 2 ? ty * (TM / 2) + i : BM / 2 + ty * (TM / 2) + (i - TM / 2));
+        const int gi = m0 + (i / CF::VA) * (BM / CF::NA) + ty * CF::VA + i % CF::VA;
         if (gi >= m) continue;
         T cv[TN];
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int gj = n0 + (j < TN / 2 ? tx * (TN / 2) + j : BN / 2 + tx * (TN / 2) + (j - TN / 2));
+            const int gj = col(j);
             const bool in = tri == 0 || (tri == 1 ? gi >= gj : gi <= gj);
             cv[j] = (read_c && gj < n && in) ? C[(long)gj * ldc + gi] : zero_v(T());
         }
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int gj = n0 + (j < TN / 2 ? tx * (TN / 2) + j : BN / 2 + tx * (TN / 2) + (j - TN / 2));
+            const int gj = col(j);
             if (gj >= n) continue;
             if (tri != 0 && (tri == 1 ? gi < gj : gi > gj)) continue;
             C[(long)gj * ldc + gi] = epilogue(alpha, acc_at(i, j), beta, &cv[j]);
@@ -264,45 +325,93 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN>::NT)
     }
 }
 
-template <class T, int BM, int BN, int BK, int TM, int TN>
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB>
 cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alpha, const T* A, int lda, const T* B,
                    int ldb, T beta, T* C, int ldc, int tri)
 {
-    using CF = Cfg<T, BM, BN, BK, TM, TN>;
+    using CF = Cfg<T, BM, BN, BK, TM, TN, ST>;
+    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB>;
+    if (CF::SMEM > 48 * 1024) {
+        // the attribute belongs to the current device's copy of the kernel
+        static std::atomic<unsigned long long> smem_set{0};
+        const unsigned long long bit = 1ull << (h->device & 63);
+        if (!(smem_set.load() & bit)) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM);
+            if (e != cudaSuccess) return e;
+            smem_set.fetch_or(bit);
+        }
+    }
     dim3 grid(ceil_div(m, BM), ceil_div(n, BN));
-    gemm_simt_kernel<T, BM, BN, BK, TM, TN><<<grid, CF::NT, 0, h->stream>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb,
-                                                                            beta, C, ldc, tri);
+    kern<<<grid, CF::NT, CF::SMEM, h->stream>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
     return cudaGetLastError();
 }
 
 }  // namespace
 
+namespace {
+// Estimated SM cycles per k step of a product whose busiest SM works on
+// `ctas` tiles: a lone CTA is bound by its latency, several by throughput.
+// Both constants per tile are measured (B200, k of 1000 to 3000).
+struct TileCost {
+    int bm, bn;
+    int alone, each;
+};
+constexpr TileCost kRealTiles[] = {{128, 128, 209, 184}, {128, 64, 120, 97}, {64, 64, 105, 62}, {32, 32, 41, 24},
+                                   {16, 16, 26, 13}};
+constexpr TileCost kCplxTiles[] = {{64, 64, 260, 205}, {32, 32, 92, 58}, {16, 16, 58, 21}};
+
+// the tile of the least estimated time
+template <int N>
+int pick_tile(const TileCost (&c)[N], int sms, int m, int n, bool tri)
+{
+    int best = 0;
+    double best_t = 0;
+    for (int q = 0; q < N; ++q) {
+        const long tm = ceil_div(m, c[q].bm), tn = ceil_div(n, c[q].bn);
+        const long tiles = tri ? (tm * tn + std::max(tm, tn)) / 2 : tm * tn;
+        const double t = std::max((double)c[q].alone, (double)ceil_div(tiles, sms) * c[q].each);
+        if (q == 0 || t < best_t) {
+            best = q;
+            best_t = t;
+        }
+    }
+    return best;
+}
+}  // namespace
+
 cudaError_t sgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, float alpha, const float* A, int lda,
                        const float* B, int ldb, float beta, float* C, int ldc, int tri)
 {
-    // the largest tile that still gives every SM a CTA: 128 x 128 (256
-    // threads, 8 x 8 outputs each), 64 x 64 (256 threads, 4 x 4), or for small
-    // products 32 x 32 (64 threads, 4 x 4; config 1's 512^3 has 16 tiles of
-    // 128 x 128 and 64 of 64 x 64)
-    auto tiles = [&](int t) {
-        long c = (long)ceil_div(m, t) * ceil_div(n, t);
-        if (tri != 0) c = (c + std::min(ceil_div(m, t), ceil_div(n, t))) / 2;
-        return c;
-    };
-    if (tiles(128) >= h->sm_count)
-        return launch<float, 128, 128, 16, 8, 8>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
-    if (tiles(64) >= h->sm_count)
-        return launch<float, 64, 64, 8, 4, 4>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
-    return launch<float, 32, 32, 8, 4, 4>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
+#define LAUNCH(...) launch<float, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri)
+    switch (pick_tile(kRealTiles, h->sm_count, m, n, tri != 0)) {
+    case 0:
+        // 16 x 8 outputs a thread read less shared memory per product, 8 x 8
+        // hide latency with twice the warps: 4096^3 51.3 against 49.1
+        // TFLOP/s, 3000 x 3000 x 1000 (4 tiles an SM) 39.7 against 41.8
+        if ((long)ceil_div(m, 128) * ceil_div(n, 128) >= 6L * h->sm_count) return LAUNCH(128, 128, 16, 16, 8, 3, 2);
+        return LAUNCH(128, 128, 16, 8, 8, 3, 2);
+    case 1: return LAUNCH(128, 64, 16, 8, 8, 4, 3);
+    case 2: return LAUNCH(64, 64, 16, 8, 8, 4, 6);
+    case 3: return LAUNCH(32, 32, 16, 4, 4, 4, 4);
+    default: return LAUNCH(16, 16, 32, 2, 2, 4, 4);
+    }
+#undef LAUNCH
 }
 
 cudaError_t cgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, cfloat alpha, const cfloat* A, int lda,
                        const cfloat* B, int ldb, cfloat beta, cfloat* C, int ldc)
 {
-    const long big_tiles = (long)ceil_div(m, 64) * ceil_div(n, 64);
-    if (big_tiles >= h->sm_count)
-        return launch<cfloat, 64, 64, 8, 4, 4>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0);
-    return launch<cfloat, 32, 32, 8, 2, 2>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0);
+#define LAUNCH(...) launch<cfloat, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0)
+    switch (pick_tile(kCplxTiles, h->sm_count, m, n, false)) {
+    case 0:
+        // 4096 x 4096 x 2048 (28 tiles an SM): 8 x 8 outputs a thread 6226 us,
+        // 8 x 4 6653; 2048^3 (7): 8 x 4 1684 us, 8 x 8 slower than 1716
+        if ((long)ceil_div(m, 64) * ceil_div(n, 64) >= 16L * h->sm_count) return LAUNCH(64, 64, 8, 8, 8, 4, 2);
+        return LAUNCH(64, 64, 8, 8, 4, 4, 3);
+    case 1: return LAUNCH(32, 32, 16, 4, 2, 3, 4);
+    default: return LAUNCH(16, 16, 16, 2, 2, 3, 4);
+    }
+#undef LAUNCH
 }
 
 }  // namespace iclb
