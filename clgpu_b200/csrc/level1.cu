@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(NT) sreduce_kernel(long n, const float* __rest
         }
     }
     double bs = block_sum(acc, sh);
-    if (gridDim.x == 1) {
+    if constexpr (NT == 1024) {  // the only block
         if (threadIdx.x == 0) *result = OP == Red::Nrm2 ? (float)sqrt(bs) : (float)bs;
         return;
     }
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(NT) creduce_kernel(long n, const cfloat* __res
         }
     }
     double bs = block_sum(acc, sh);
-    if (gridDim.x == 1) {
+    if constexpr (NT == 1024) {  // the only block
         if (threadIdx.x == 0) *result = OP == Red::Nrm2 ? (float)sqrt(bs) : (float)bs;
         return;
     }
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(NT) cdot_kernel(long n, const cfloat* __restri
     }
     double bre = block_sum(re, sh);
     double bim = block_sum(im, sh);
-    if (gridDim.x == 1) {
+    if constexpr (NT == 1024) {  // the only block
         if (threadIdx.x == 0) *result = cfloat{(float)bre, (float)bim};
         return;
     }
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(NT) iamax_kernel(long n, const T* __restrict__
         if (isnan_v(x[0]) || idx == INT_MAX) idx = 0;
         *result = idx;
     };
-    if (gridDim.x == 1) {
+    if constexpr (NT == 1024) {  // the only block
         if (threadIdx.x == 0) finish(b);
         return;
     }
