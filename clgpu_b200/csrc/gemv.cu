@@ -53,6 +53,20 @@ __device__ __forceinline__ cfloat axpby(cfloat alpha, cfloat s, cfloat beta, con
     return r;
 }
 
+__device__ __forceinline__ float ldg_of(const float* p) { return __ldg(p); }
+__device__ __forceinline__ cfloat ldg_of(const cfloat* p)
+{
+    const float2 v = __ldg((const float2*)p);
+    return cfloat{v.x, v.y};
+}
+// another block's partial sum, past this SM's L1
+__device__ __forceinline__ float ldcg_of(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ cfloat ldcg_of(const cfloat* p)
+{
+    const float2 v = __ldcg((const float2*)p);
+    return cfloat{v.x, v.y};
+}
+
 template <class T>
 __device__ __forceinline__ T warp_sum_t(T v);
 template <>
@@ -64,14 +78,15 @@ __device__ __forceinline__ cfloat warp_sum_t<cfloat>(cfloat v)
 }
 
 // ------------------------------------------------------------------ op N
-// Block (rt, s): rows [rt*R*128, +R*128), columns [s*cps, min(n, (s+1)*cps)).
-// VEC: lda*sizeof(T) and A are 16-byte aligned, so each thread's R rows of a
-// column are one 128-bit load.
-template <class T, bool VEC>
-__global__ void __launch_bounds__(kNThreads) gemv_n_kernel(int m, int n, T alpha, const T* __restrict__ A, long lda,
-                                                           const T* __restrict__ x, long incx, T beta,
-                                                           T* __restrict__ y, long incy, int cps,
-                                                           T* __restrict__ partial, unsigned* counters)
+// Large aligned matrices: block (rt, s) owns rows [rt*R*128, +R*128) and
+// columns [s*cps, min(n, (s+1)*cps)); a thread's R rows of a column are one
+// 128-bit load.  (The kernel below with G = 1 measured 4 % slower here:
+// complex 8192 x 8192 87 us against 83.)
+template <class T>
+__global__ void __launch_bounds__(kNThreads) gemv_n_stream_kernel(int m, int n, T alpha, const T* __restrict__ A, long lda,
+                                                                  const T* __restrict__ x, long incx, T beta,
+                                                                  T* __restrict__ y, long incy, int cps,
+                                                                  T* __restrict__ partial, unsigned* counters)
 {
     constexpr int R = 16 / sizeof(T);
     constexpr int XC = 256;  // x values staged per chunk
@@ -93,7 +108,7 @@ __global__ void __launch_bounds__(kNThreads) gemv_n_kernel(int m, int n, T alpha
         __syncthreads();
         if (row0 < m) {
             const T* Ac = A + (long)cb * lda + row0;
-            if (VEC && row0 + R <= m) {
+            if (row0 + R <= m) {
                 int c = 0;
                 for (; c + 8 <= cn; c += 8) {
                     float4 v[8];
@@ -144,6 +159,153 @@ __global__ void __launch_bounds__(kNThreads) gemv_n_kernel(int m, int n, T alpha
         for (int k = 0; k < splits; ++k) sum = add(sum, ((volatile T*)partial)[(long)k * m + row]);
         T* yp = y + row * incy;
         *yp = axpby(alpha, sum, beta, yp);
+    }
+    if (threadIdx.x == 0) counters[blockIdx.x] = 0u;
+}
+
+// Block (rt, s): rows [rt*R*128, +R*128), columns [s*cps, min(n, (s+1)*cps)),
+// in G groups of 128 threads that take turns of 8 columns.
+// VEC: lda*sizeof(T) and A are 16-byte aligned, so each thread's R rows of a
+// column are one 128-bit load.  Otherwise its rows are 128 apart: every load
+// of a warp is one run of 32 elements, and a block still reads whole runs of
+// 128 * R elements of a column (runs of 128 alone measured 3 times slower on
+// 9001 x 9000).
+// G = 1 when the matrix fills the GPU with bandwidth-bound blocks.  Smaller
+// ones are bound by the time of a few dependent steps: a batch of 8 columns
+// per load latency, then the last block's sum over the slices.  G = 4 does
+// four batches at once, adds the groups in shared memory and splits that
+// last sum over the groups as well.
+// Measured (us, before and after, operands in L2): real 256 x 256 10.7, 4.2;
+// 423 x 9911, lda 425, 41, 9.1; 4096 x 4096 19.0, 12.3; 5000 x 5001 42, 15.8;
+// 9001 x 9000 (G = 1) 78, 61; complex 3001 x 1777, lda 3003, 18.2, 9.1.
+template <class T, bool VEC, int G>
+__global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T alpha, const T* __restrict__ A, long lda,
+                                                               const T* __restrict__ x, long incx, T beta,
+                                                               T* __restrict__ y, long incy, int cps,
+                                                               T* __restrict__ partial, unsigned* counters)
+{
+    constexpr int R = 16 / sizeof(T);
+    constexpr int RS = VEC ? 1 : kNThreads;  // rows of a thread: row0 + r * RS
+    constexpr int XC = 256;  // x values staged per chunk
+    __shared__ T xs[XC];
+    __shared__ T red[G > 1 ? G - 1 : 1][G > 1 ? R * kNThreads : 1];
+    const int tid = threadIdx.x % kNThreads, g = G > 1 ? threadIdx.x / kNThreads : 0;
+    const int splits = gridDim.y;
+    const int s = blockIdx.y;
+    const long row0 = VEC ? ((long)blockIdx.x * kNThreads + tid) * R : (long)blockIdx.x * kNThreads * R + tid;
+    const int c0 = s * cps;
+    const int c1 = min(n, c0 + cps);
+
+    T acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = zero_of(T());
+    // acc of group 0 += those of the other groups, in order
+    auto add_groups = [&]() {
+        if constexpr (G > 1) {
+            if (g > 0)
+#pragma unroll
+                for (int r = 0; r < R; ++r) red[g - 1][r * kNThreads + tid] = acc[r];
+            __syncthreads();
+            if (g == 0)
+#pragma unroll
+                for (int q = 0; q < G - 1; ++q)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) acc[r] = add(acc[r], red[q][r * kNThreads + tid]);
+        }
+    };
+
+    for (int cb = c0; cb < c1; cb += XC) {
+        const int cn = min(XC, c1 - cb);
+        __syncthreads();
+        for (int i = threadIdx.x; i < cn; i += kNThreads * G) xs[i] = x[(long)(cb + i) * incx];
+        __syncthreads();
+        if (row0 < m) {
+            const T* Ac = A + (long)cb * lda + row0;
+            if (VEC && row0 + R <= m) {
+                int c = 8 * g;
+                for (; c + 8 <= cn; c += 8 * G) {
+                    float4 v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = ld_stream4((const float4*)(Ac + (long)(c + u) * lda));
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const T* e = (const T*)&v[u];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) madd<false>(acc[r], e[r], xs[c + u]);
+                    }
+                }
+                for (const int ce = min(c + 8, cn); c < ce; ++c) {
+                    float4 v = ld_stream4((const float4*)(Ac + (long)c * lda));
+                    const T* e = (const T*)&v;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) madd<false>(acc[r], e[r], xs[c]);
+                }
+            } else {
+                int c = 8 * g;
+                // (VEC: the few rows past the last whole vector)
+                for (; !VEC && c + 8 <= cn; c += 8 * G) {
+                    T v[8][R];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            v[u][r] = row0 + r * RS < m ? ldg_of(Ac + (long)(c + u) * lda + r * RS) : zero_of(T());
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+#pragma unroll
+                        for (int r = 0; r < R; ++r) madd<false>(acc[r], v[u][r], xs[c + u]);
+                }
+                for (; c < cn; c += VEC ? 8 * G : cn) {
+                    for (int u = c; u < min(c + 8, cn); ++u) {
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            if (row0 + r * RS < m) madd<false>(acc[r], Ac[(long)u * lda + r * RS], xs[u]);
+                    }
+                }
+            }
+        }
+    }
+    add_groups();
+
+    if (splits == 1) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (g == 0 && row0 + r * RS < m) {
+                T* yp = y + (row0 + r * RS) * incy;
+                *yp = axpby(alpha, acc[r], beta, yp);
+            }
+        return;
+    }
+    // publish this slice's partial sums; the last slice of the row tile adds
+    // them, each group a run of consecutive slices
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (g == 0 && row0 + r * RS < m) partial[(long)s * m + row0 + r * RS] = acc[r];
+    if (!last_block_of(counters + blockIdx.x, splits)) return;
+    const int per = (splits + G - 1) / G, k1 = min(splits, (g + 1) * per);
+    constexpr int KU = 32 / R;  // slices in flight
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = zero_of(T());
+    for (int k = g * per; k < k1; k += KU) {
+        T t[KU][R];
+#pragma unroll
+        for (int u = 0; u < KU; ++u)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                t[u][r] = (k + u < k1 && row0 + r * RS < m) ? ldcg_of(partial + (long)(k + u) * m + row0 + r * RS)
+                                                            : zero_of(T());
+#pragma unroll
+        for (int u = 0; u < KU; ++u)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r] = add(acc[r], t[u][r]);
+    }
+    add_groups();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const long row = row0 + r * RS;
+        if (g != 0 || row >= m) continue;
+        T* yp = y + row * incy;
+        *yp = axpby(alpha, acc[r], beta, yp);
     }
     if (threadIdx.x == 0) counters[blockIdx.x] = 0u;
 }
@@ -200,7 +362,25 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_kernel(int m, int n, T alpha
         for (int k = 0; k < R; ++k)
             if (r + k < r1) madd<CONJ>(acc, Ac[r + k], x[r + k]);
     } else {
-        for (int r = r0 + lane; r < r1; r += 32) madd<CONJ>(acc, Ac[r], x[(long)r * incx]);
+        // real data: 8 loads of each operand in flight, the last ones
+        // predicated (9001 x 9000 147 us with one at a time, 74 so; 1000 x 1000
+        // 9.0, 3.4); complex data measured slower that way
+        if constexpr (sizeof(T) == sizeof(float)) {
+            for (int r = r0 + lane; r < r1; r += 8 * 32) {
+                T v[8], xv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const bool in = r + u * 32 < r1;
+                    v[u] = in ? ldg_of(Ac + r + u * 32) : zero_of(T());
+                    xv[u] = in ? ldg_of(x + (long)(r + u * 32) * incx) : zero_of(T());
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (r + u * 32 < r1) madd<CONJ>(acc, v[u], xv[u]);
+            }
+        } else {
+            for (int r = r0 + lane; r < r1; r += 32) madd<CONJ>(acc, Ac[r], x[(long)r * incx]);
+        }
     }
     acc = warp_sum_t(acc);
     if (S == 1) {
@@ -237,13 +417,21 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
         const bool vec = aligned16(A) && ((long)lda * sizeof(T)) % 16 == 0;
         const int rows_per_block = kNThreads * R;
         const int rt = ceil_div(m, rows_per_block);
-        int splits = 1;
-        if (rt < target && rt <= kCounterWords) {
+        // bandwidth-bound: enough blocks of 64 columns and more to fill the
+        // GPU (one group a block); else four groups a block and as many
+        // slices as the SMs hold blocks, at least one batch of columns a
+        // group (16384 x 16384 with four groups: 297 us against 159)
+        const bool small = (long)rt * max(1, n / 64) < target;
+        int splits = 1, unit = 8;
+        if (small) {
+            unit = 32;
+            splits = max(1, min(ceil_div(2 * h->sm_count, rt), ceil_div(n, unit)));
+        } else if (rt < target && rt <= kCounterWords) {
             splits = ceil_div(target, rt);
             splits = min(splits, max(1, n / 64));
         }
         int cps = ceil_div(n, splits);
-        cps = (cps + 7) & ~7;
+        cps = (cps + unit - 1) / unit * unit;
         splits = ceil_div(n, cps);
         T* partial = nullptr;
         if (splits > 1) {
@@ -251,19 +439,24 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
             if (!partial) return cudaErrorMemoryAllocation;
         }
         dim3 grid(rt, splits);
-        if (vec)
-            gemv_n_kernel<T, true><<<grid, kNThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, cps,
-                                                                      partial, h->ws.counters);
+#define LAUNCH(V, G)                                                                                       \
+    gemv_n_kernel<T, V, G><<<grid, kNThreads * G, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, \
+                                                                  cps, partial, h->ws.counters)
+        if (small) { if (vec) LAUNCH(true, 4); else LAUNCH(false, 4); }
+        else if (!vec) LAUNCH(false, 1);
         else
-            gemv_n_kernel<T, false><<<grid, kNThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy,
-                                                                       cps, partial, h->ws.counters);
+            gemv_n_stream_kernel<T><<<grid, kNThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, cps,
+                                                                       partial, h->ws.counters);
+#undef LAUNCH
         return cudaGetLastError();
     }
     // op T / C: columns of A are dot products with x
     const bool vec = aligned16(A) && ((long)lda * sizeof(T)) % 16 == 0 && incx == 1 && aligned16(x);
     const int warps_target = target * (kTThreads / 32);
     int S = 1;
-    if (n < warps_target && n <= kCounterWords) S = min(ceil_div(warps_target, n), max(1, m / 1024));
+    // (a real scalar load brings a quarter as much: shorter slices)
+    if (n < warps_target && n <= kCounterWords)
+        S = min(ceil_div(warps_target, n), max(1, m / (vec || sizeof(T) != sizeof(float) ? 1024 : 512)));
     int rps = ceil_div(m, S);
     rps = (rps + 32 * R - 1) / (32 * R) * (32 * R);
     S = ceil_div(m, rps);
