@@ -1109,64 +1109,129 @@ __device__ __forceinline__ void put(const SplitOut& o, long idx, float x)
     if (o.nlev > 2) ((__nv_bfloat16*)o.plane[2])[idx] = l;
 }
 
-// Real operands: 32 rows x 64 K per block (256 threads).  Reads are coalesced
-// along the source's contiguous dimension (through shared memory); each
-// thread then writes two consecutive K values: one bfloat162 per plane, or a
-// float2 for TF32 (128- or 256-byte rows per warp).  Row r goes to
-// plane + r * o.kpad, K values [0, kw) (zeros for k >= K; kw even).
-// `tri` masks L to a triangle (1: keep k <= r, 2: keep k >= r; `unit` puts 1
-// on the diagonal); tiles wholly outside the kept triangle are left
+// Real operands: 64 rows x 64 K per block (256 threads).  Bound by HBM (4
+// bytes in, 4 to 6 out per element), so what matters is bytes in flight: a
+// thread issues its 16 loads (four 16-byte ones when `vin`: S and its stride
+// 16-byte aligned) before it uses any, along the source's contiguous
+// dimension and through shared memory, and then writes 8 consecutive K of a
+// row at a time, 16 bytes per BF16 plane (`vout`: every plane row 16-byte
+// aligned and kw a multiple of 8; else pairs).  8192^2 into three planes:
+// 102 us (6.6 TB/s); with 4-byte loads one at a time and pair stores 193.
+// Row r goes to plane + r * o.kpad, K values [0, kw) (zeros for k >= K; kw
+// even).  `tri` masks L to a triangle (1: keep k <= r, 2: keep k >= r; `unit`
+// puts 1 on the diagonal); tiles wholly outside the kept triangle are left
 // unwritten.  blockIdx.z selects one of several equal operands: source
 // + z * szs, destination row offset + z * dzs.
 __global__ void __launch_bounds__(256) split_real_kernel(int R, int K, const float* __restrict__ S, long rs, long ks,
-                                                         SplitOut o, long kw, int tri, int unit, long szs, long dzs)
+                                                         SplitOut o, long kw, int tri, int unit, long szs, long dzs,
+                                                         int vin, int vout)
 {
-    __shared__ float tile[32][65];
-    const int k0 = blockIdx.x * 64, r0 = blockIdx.y * 32, t = threadIdx.x;
-    if ((tri == 1 && k0 > r0 + 31) || (tri == 2 && k0 + 63 < r0)) return;
+    __shared__ float tile[64][65];
+    const int k0 = blockIdx.x * 64, r0 = blockIdx.y * 64, t = threadIdx.x;
+    if ((tri == 1 && k0 > r0 + 63) || (tri == 2 && k0 + 63 < r0)) return;
     S += (long)blockIdx.z * szs;
     const long dz = (long)blockIdx.z * dzs;
-    if (rs == 1) {  // contiguous along r
-        for (int idx = t; idx < 32 * 64; idx += 256) {
-            const int rr = idx % 32, kk = idx / 32;
-            const int r = r0 + rr, k = k0 + kk;
-            tile[rr][kk] = (r < R && k < K) ? S[(long)r + (long)k * ks] : 0.f;
+    // f runs along the contiguous dimension of the source, g across it
+    const bool rc = rs == 1;
+    const int f0 = rc ? r0 : k0, nf = rc ? R : K, g0 = rc ? k0 : r0, ng = rc ? K : R;
+    const long gs = rc ? ks : rs;
+    float v[16];
+    if (vin && f0 + 64 <= nf) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int f = (t % 16) * 4, g = t / 16 + 16 * u;
+            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g0 + g < ng) w = __ldg(reinterpret_cast<const float4*>(S + (long)(g0 + g) * gs + f0 + f));
+            v[4 * u] = w.x;
+            v[4 * u + 1] = w.y;
+            v[4 * u + 2] = w.z;
+            v[4 * u + 3] = w.w;
         }
-    } else {        // contiguous along k (ks == 1)
-        for (int idx = t; idx < 32 * 64; idx += 256) {
-            const int kk = idx % 64, rr = idx / 64;
-            const int r = r0 + rr, k = k0 + kk;
-            tile[rr][kk] = (r < R && k < K) ? S[(long)r * rs + k] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int f = (t % 16) * 4 + u % 4, g = t / 16 + 16 * (u / 4);
+            tile[rc ? f : g][rc ? g : f] = v[u];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int f = t % 64, g = t / 64 + 4 * u;
+            v[u] = (f0 + f < nf && g0 + g < ng) ? __ldg(S + (long)(g0 + g) * gs + f0 + f) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int f = t % 64, g = t / 64 + 4 * u;
+            tile[rc ? f : g][rc ? g : f] = v[u];
         }
     }
     __syncthreads();
-    for (int idx = t; idx < 32 * 32; idx += 256) {
-        const int kp = idx % 32, rr = idx / 32;
-        const int r = r0 + rr, k = k0 + 2 * kp;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int rr = t / 8 + 32 * u, kk = (t % 8) * 8;
+        const int r = r0 + rr, k = k0 + kk;
         if (r >= R || k >= kw) continue;
-        float a = tile[rr][2 * kp], b = tile[rr][2 * kp + 1];
-        if (tri) {
-            const bool ka = tri == 1 ? k <= r : k >= r, kb = tri == 1 ? k + 1 <= r : k + 1 >= r;
-            a = ka ? ((unit && k == r) ? 1.f : a) : 0.f;
-            b = kb ? ((unit && k + 1 == r) ? 1.f : b) : 0.f;
+        float x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            x[e] = tile[rr][kk + e];
+            if (tri) {
+                const bool keep = tri == 1 ? k + e <= r : k + e >= r;
+                x[e] = keep ? ((unit && k + e == r) ? 1.f : x[e]) : 0.f;
+            }
         }
         const long off = ((long)r + dz) * o.kpad + k;  // even: 4- and 8-byte aligned pairs
         if (o.tf32) {
-            *reinterpret_cast<float2*>((float*)o.plane[0] + off) = make_float2(to_tf32(a), to_tf32(b));
+            float* d = (float*)o.plane[0] + off;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = to_tf32(x[e]);
+            if (vout) {
+                reinterpret_cast<float4*>(d)[0] = make_float4(x[0], x[1], x[2], x[3]);
+                reinterpret_cast<float4*>(d)[1] = make_float4(x[4], x[5], x[6], x[7]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; e += 2)
+                    if (k + e < kw) *reinterpret_cast<float2*>(d + e) = make_float2(x[e], x[e + 1]);
+            }
         } else {
-            __nv_bfloat16 ha, ma, la, hb, mb, lb;
-            split3(a, ha, ma, la);
-            split3(b, hb, mb, lb);
-            *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)o.plane[0] + off) = __halves2bfloat162(ha, hb);
-            if (o.nlev > 1)
-                *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)o.plane[1] + off) = __halves2bfloat162(ma, mb);
-            if (o.nlev > 2)
-                *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)o.plane[2] + off) = __halves2bfloat162(la, lb);
+            uint32_t w[3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                __nv_bfloat16 ha, ma, la, hb, mb, lb;
+                split3(x[2 * e], ha, ma, la);
+                split3(x[2 * e + 1], hb, mb, lb);
+                w[0][e] = (uint32_t)__bfloat16_as_ushort(ha) | ((uint32_t)__bfloat16_as_ushort(hb) << 16);
+                w[1][e] = (uint32_t)__bfloat16_as_ushort(ma) | ((uint32_t)__bfloat16_as_ushort(mb) << 16);
+                w[2][e] = (uint32_t)__bfloat16_as_ushort(la) | ((uint32_t)__bfloat16_as_ushort(lb) << 16);
+            }
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                if (l >= o.nlev) break;
+                __nv_bfloat16* d = (__nv_bfloat16*)o.plane[l] + off;
+                if (vout) {
+                    *reinterpret_cast<uint4*>(d) = make_uint4(w[l][0], w[l][1], w[l][2], w[l][3]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (k + 2 * e < kw) reinterpret_cast<uint32_t*>(d)[e] = w[l][e];
+                }
+            }
         }
     }
 }
 
-// IEEE half operands (HGEMM): the same 32 x 64 tiling, values copied into
+// Launches split_real_kernel: nz operands of R rows, K values [0, kw) each.
+cudaError_t launch_split_real(cudaStream_t st, const float* S, int R, int K, long rs, long ks, const SplitOut& o,
+                              long kw, int tri, int unit, int nz, long szs, long dzs)
+{
+    const int vin = ((uintptr_t)S & 15) == 0 && ((rs == 1 ? ks : rs) & 3) == 0 && (szs & 3) == 0;
+    bool vout = (kw & 7) == 0 && (o.kpad & 7) == 0;
+    for (int l = 0; l < (o.tf32 ? 1 : o.nlev); ++l) vout = vout && ((uintptr_t)o.plane[l] & 15) == 0;
+    dim3 grid((unsigned)ceil_div(kw, 64L), (unsigned)ceil_div(R, 64), (unsigned)nz);
+    split_real_kernel<<<grid, 256, 0, st>>>(R, K, S, rs, ks, o, kw, tri, unit, szs, dzs, vin, (int)vout);
+    return cudaGetLastError();
+}
+
+// IEEE half operands (HGEMM): 32 x 64 tiles, values copied into
 // the K-major padded plane unchanged (zeros past K).
 __global__ void __launch_bounds__(256) pack_half_kernel(int R, int K, const __half* __restrict__ S, long rs, long ks,
                                                         __half* __restrict__ plane, long kpad)
@@ -1394,9 +1459,7 @@ cudaError_t run_split(iclblasHandle_t h, const T* S, int R, int K, long rs, long
                       const SplitOut& o, long out_rows)
 {
     if (std::is_same<T, float>::value) {
-        dim3 grid((unsigned)ceil_div(o.kpad, 64L), (unsigned)ceil_div(R, 32));
-        split_real_kernel<<<grid, 256, 0, h->stream>>>(R, K, (const float*)S, rs, ks, o, o.kpad, 0, 0, 0, 0);
-        return cudaGetLastError();
+        return launch_split_real(h->stream, (const float*)S, R, K, rs, ks, o, o.kpad, 0, 0, 1, 0, 0);
     }
     dim3 grid(ceil_div(K, 32), ceil_div(R, 32));
     split_kernel<T><<<grid, dim3(32, 8), 0, h->stream>>>(R, K, S, rs, ks, conj, mode, o);
@@ -1709,9 +1772,7 @@ cudaError_t split_planes_tc(iclblasHandle_t h, const float* S, int R, int K, lon
     o.tf32 = dst.tf32;
     o.kpad = dst.pitch;
     for (int l = 0; l < dst.nlev; ++l) o.plane[l] = (char*)dst.plane[l] + (row0 * dst.pitch + k0) * esize;
-    dim3 grid((unsigned)ceil_div(kw, 64L), (unsigned)ceil_div(R, 32), (unsigned)nz);
-    split_real_kernel<<<grid, 256, 0, h->stream>>>(R, K, S, rs, ks, o, kw, tri, unit, szs, dzs);
-    return cudaGetLastError();
+    return launch_split_real(h->stream, S, R, K, rs, ks, o, kw, tri, unit, nz, szs, dzs);
 }
 
 template cudaError_t gemm_tc<float>(iclblasHandle_t, int, int, int, int, int, float, const float*, int, const float*,

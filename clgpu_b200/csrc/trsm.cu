@@ -275,7 +275,9 @@ constexpr size_t kInvDiag64Smem = sizeof(double) * (2 * 64 * 65 + 32 * 33 + 64);
 // STEP 0 forms T = C * P^-1 (lower) or T = C * Q^-1 (upper) with C read from
 // A through op; STEP 1 forms the off-diagonal block -Q^-1 T (lower) or
 // -P^-1 T (upper) into the inverse.  FP64, TS x TS tiles, 256 threads, each
-// thread (TS/16) x (TS/16) outputs; blockIdx.z enumerates the 2s blocks.
+// thread (TS/16) x (TS/16) outputs; blockIdx.z enumerates the 2s blocks.  K
+// runs only over the slices where the triangular factor (P^-1 or Q^-1: Y in
+// STEP 0, X in STEP 1) is not zero.
 template <class T, int TS, int STEP>
 __global__ void __launch_bounds__(256) trsm_inv_double_kernel(int n, int op, int m_lower, int s, int big,
                                                               const T* __restrict__ A, long lda,
@@ -346,12 +348,18 @@ __global__ void __launch_bounds__(256) trsm_inv_double_kernel(int n, int op, int
             Ys[idx % KC][idx / KC] = ry[u];
         }
     };
-    load(0);
-    for (int k0 = 0; k0 < s; k0 += KC) {
+    // Y columns j0 .. j0+TS-1 (STEP 0) or X rows i0 .. i0+TS-1 (STEP 1) of a
+    // lower factor are zero above (STEP 0) or right of (STEP 1) the diagonal,
+    // those of an upper one below or left of it
+    const bool from_diag = (STEP == 0) == (m_lower != 0);
+    const int d0 = STEP == 0 ? j0 : i0;
+    const int kb = from_diag ? d0 : 0, ke = from_diag ? s : min(s, d0 + TS);
+    load(kb);
+    for (int k0 = kb; k0 < ke; k0 += KC) {
         __syncthreads();
         store();
         __syncthreads();
-        if (k0 + KC < s) load(k0 + KC);
+        if (k0 + KC < ke) load(k0 + KC);
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
             W xv[PT], yv[PT];
