@@ -25,8 +25,8 @@
 //                 per instruction, 4 per stage) and tcgen05.commit;
 //      warps 2-9  epilogue: two warps per 32-lane TMEM quarter, 128 columns
 //                 each (two halves of four warps).
-//    Each pipeline stage is one (K block, product) pair.  The BF16 modes run
-//    the products of every K block small-first -- 3xBF16: mid*hi, hi*mid,
+//    A pipeline stage is one K block: all split levels of it in the BF16
+//    modes, one level in TF32 and HGEMM.  The BF16 modes run the products of every K block small-first -- 3xBF16: mid*hi, hi*mid,
 //    hi*hi; 6xBF16: lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi -- into a
 //    fresh accumulator per chunk of one K block.  The tensor core's FP32
 //    accumulation loses a fraction of an ulp of the running value at every
@@ -106,6 +106,7 @@ struct Params {
     int M, N;          // output rows / columns of the (real) GEMM
     int kblocks;       // K_pad / elements-per-row-block
     int nprod;         // products per K block (1, 3 or 6)
+    int nlev;          // split levels of an operand (TF32, HGEMM: 1)
     int chunk;         // K blocks per TMEM chunk (drained into registers)
     int pa[6], pb[6];  // split level of A and B for each product
     int complex_out;   // columns come in (re, im) pairs
@@ -690,6 +691,14 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint8_t* tiles = smem;
     using TC = Tile<BN_>;
     constexpr int BN = TC::BN, STAGES = TC::STAGES, STAGE_BYTES = TC::STAGE_BYTES, EPI_COLS = TC::EPI_COLS;
+    // BF16 modes: a stage holds every level of one K block of both operands,
+    // read by all of the block's products.  (A stage per product loaded each
+    // level up to three times: 32 KiB per 256 clocks of MMAs, twice what an
+    // SM gets from L2.  3xBF16 and 6xBF16, us before and after: 8192^3 2690,
+    // 2181 and 5850, 4297; 2048^3 74, 60 and 118, 95; 512 x 4096 x 512 29,
+    // 25 and 40, 31.)
+    constexpr bool KB = !TF32 && OUT != OUT_F16;
+    const int nlev = KB ? p.nlev : 1, nstages = STAGES / nlev, stage_bytes = nlev * STAGE_BYTES;
     uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
     uint64_t* empty = full + STAGES;
     uint64_t* tfull = empty + STAGES;
@@ -702,7 +711,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
     const int ntiles = tile_count(p.tri, tiles_m, tiles_n, BM, BN);
-    const int steps = p.kblocks * p.nprod;
+    const int steps = KB ? p.kblocks : p.kblocks * p.nprod;  // stages of a tile
+    const int step_prods = KB ? p.nprod : 1;                 // products of a stage
     constexpr bool MN_OK = OUT == OUT_F16;  // MN-major operands: HGEMM only
 
     if (threadIdx.x == 0) {
@@ -739,20 +749,23 @@ __global__ void __launch_bounds__(THREADS, 1)
                 int tm, tn;
                 tile_at(p.tri, t, tiles_m, tiles_n, BM, BN, tm, tn);
                 for (int st = 0; st < steps && ok; ++st) {
-                    const int kb = st / p.nprod, pr = st % p.nprod;
+                    const int kb = KB ? st : st / p.nprod, pr = KB ? 0 : st % p.nprod;
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-                    uint8_t* sa = tiles + s * STAGE_BYTES;
-                    uint8_t* sb = sa + A_TILE;
-                    mbar_expect_tx(&full[s], STAGE_BYTES);
+                    uint8_t* sa = tiles + s * stage_bytes;
+                    uint8_t* sb = sa + nlev * A_TILE;
+                    mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
                     const int kx = kb * (TF32 ? 32 : 64);
-                    load_operand(sa, ma[p.pa[pr]], MN_OK && p.a_mn, BM, kx, tm * BM, &full[s]);
-                    load_operand(sb, mb[p.pb[pr]], MN_OK && p.b_mn, BN, kx, tn * BN, &full[s]);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                    for (int l = 0; l < nlev; ++l) {
+                        load_operand(sa + l * A_TILE, ma[KB ? l : p.pa[pr]], MN_OK && p.a_mn, BM, kx, tm * BM, &full[s]);
+                        load_operand(sb + l * TC::B_TILE, mb[KB ? l : p.pb[pr]], MN_OK && p.b_mn, BN, kx, tn * BN,
+                                     &full[s]);
+                    }
+                    if (++s == nstages) { s = 0; ph ^= 1; }
                 }
             }
             if (!ok) {
                 // wait (bounded) for the copies this thread issued, then leave
-                for (int i = 0; i < STAGES; ++i) mbar_drain(&full[(s + i) % STAGES], ph);
+                for (int i = 0; i < nstages; ++i) mbar_drain(&full[(s + i) % nstages], ph);
             }
         }
     } else if (warp == 1) {
@@ -766,7 +779,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             int acc = 0;
             uint32_t acc_ph = 0;
             bool ok = true;
-            const int chunk_steps = p.chunk * p.nprod;
+            const int chunk_steps = KB ? p.chunk : p.chunk * p.nprod;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 for (int c0 = 0; c0 < steps && ok; c0 += chunk_steps) {
                     if (!mbar_wait(&tempty[acc], acc_ph ^ 1, abort_flag)) { ok = false; break; }
@@ -776,15 +789,20 @@ __global__ void __launch_bounds__(THREADS, 1)
                     for (int st = c0; st < c1; ++st) {
                         if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t sa = smem_u32(tiles + s * STAGE_BYTES);
-                        const uint32_t sb = sa + A_TILE;
-                        const uint64_t da = a_mn ? smem_desc_mn_sw128(sa) : smem_desc_sw128(sa);
-                        const uint64_t db = b_mn ? smem_desc_mn_sw128(sb) : smem_desc_sw128(sb);
+                        const uint32_t sa = smem_u32(tiles + s * stage_bytes);
+                        const uint32_t sb = sa + nlev * A_TILE;
+                        for (int pr = 0; pr < step_prods; ++pr) {
+                            const uint32_t pa = sa + (KB ? p.pa[pr] * A_TILE : 0);
+                            const uint32_t pb = sb + (KB ? p.pb[pr] * TC::B_TILE : 0);
+                            const uint64_t da = a_mn ? smem_desc_mn_sw128(pa) : smem_desc_sw128(pa);
+                            const uint64_t db = b_mn ? smem_desc_mn_sw128(pb) : smem_desc_sw128(pb);
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)  // 4 x 32 bytes of K per stage
-                            umma<TF32>(d, da + a_step * kk, db + b_step * kk, idesc, (st > c0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; ++kk)  // 4 x 32 bytes of K per tile row
+                                umma<TF32>(d, da + a_step * kk, db + b_step * kk, idesc,
+                                           (st > c0 || pr > 0 || kk > 0) ? 1u : 0u);
+                        }
                         umma_commit(&empty[s]);
-                        if (++s == STAGES) { s = 0; ph ^= 1; }
+                        if (++s == nstages) { s = 0; ph ^= 1; }
                     }
                     // chunk done (or aborted): the epilogue may read this accumulator
                     umma_commit(&tfull[acc]);
@@ -919,6 +937,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* tiles = smem;
+    // BF16 modes: a stage holds every level of one K block (as above)
+    constexpr bool KB = !TF32 && OUT != OUT_F16;
+    const int nlev = KB ? p.nlev : 1, nstages = STAGES / nlev, stage_bytes = nlev * STAGE_BYTES;
     uint64_t* full = (uint64_t*)(smem + RING_BYTES);
     uint64_t* empty = full + STAGES;
     uint64_t* tfull = empty + STAGES;
@@ -934,7 +955,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int pair = blockIdx.x / 2, npairs = gridDim.x / 2;
     const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + BN - 1) / BN;
     const int ntiles = tile_count(p.tri, tiles_m, tiles_n, 2 * BM, BN);
-    const int steps = p.kblocks * p.nprod;
+    const int steps = KB ? p.kblocks : p.kblocks * p.nprod;  // stages of a tile
+    const int step_prods = KB ? p.nprod : 1;                 // products of a stage
     constexpr bool MN_OK = OUT == OUT_F16;  // MN-major operands: HGEMM only
 
     if (threadIdx.x == 0) {
@@ -971,32 +993,36 @@ __global__ void __launch_bounds__(THREADS, 1)
                 int tm, tn;
                 tile_at(p.tri, t, tiles_m, tiles_n, 2 * BM, BN, tm, tn);
                 for (int st = 0; st < steps && ok; ++st) {
-                    const int kb = st / p.nprod, pr = st % p.nprod;
+                    const int kb = KB ? st : st / p.nprod, pr = KB ? 0 : st % p.nprod;
                     if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-                    uint8_t* sa = tiles + s * STAGE_BYTES;
-                    uint8_t* sb = sa + A_TILE;
-                    if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                    uint8_t* sa = tiles + s * stage_bytes;
+                    uint8_t* sb = sa + nlev * A_TILE;
+                    if (leader) mbar_expect_tx(&full[s], 2u * (uint32_t)stage_bytes);
                     const uint32_t bar = map_rank(&full[s], 0);
                     const int kx = kb * (TF32 ? 32 : 64);
                     const int ra = tm * 2 * BM + (int)rank * BM, rb = tn * BN + (int)rank * 128;
-                    if (MN_OK && p.a_mn) {
-                        for (int i = 0; i < BM / 64; ++i)
-                            tma_load_2d_pair(sa + i * MN_CHUNK_BYTES, ma[p.pa[pr]], ra + i * 64, kx, bar);
-                    } else {
-                        tma_load_2d_pair(sa, ma[p.pa[pr]], kx, ra, bar);
+                    for (int l = 0; l < nlev; ++l) {
+                        const CUtensorMap* la = ma[KB ? l : p.pa[pr]];
+                        const CUtensorMap* lb = mb[KB ? l : p.pb[pr]];
+                        if (MN_OK && p.a_mn) {
+                            for (int i = 0; i < BM / 64; ++i)
+                                tma_load_2d_pair(sa + i * MN_CHUNK_BYTES, la, ra + i * 64, kx, bar);
+                        } else {
+                            tma_load_2d_pair(sa + l * A_TILE, la, kx, ra, bar);
+                        }
+                        if (MN_OK && p.b_mn) {
+                            for (int i = 0; i < 128 / 64; ++i)
+                                tma_load_2d_pair(sb + i * MN_CHUNK_BYTES, lb, rb + i * 64, kx, bar);
+                        } else {
+                            tma_load_2d_pair(sb + l * B_HALF, lb, kx, rb, bar);
+                        }
                     }
-                    if (MN_OK && p.b_mn) {
-                        for (int i = 0; i < 128 / 64; ++i)
-                            tma_load_2d_pair(sb + i * MN_CHUNK_BYTES, mb[p.pb[pr]], rb + i * 64, kx, bar);
-                    } else {
-                        tma_load_2d_pair(sb, mb[p.pb[pr]], kx, rb, bar);
-                    }
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                    if (++s == nstages) { s = 0; ph ^= 1; }
                 }
             }
             if (!ok && leader) {
                 // wait (bounded) for the copies in flight to this CTA's barriers, then leave
-                for (int i = 0; i < STAGES; ++i) mbar_drain(&full[(s + i) % STAGES], ph);
+                for (int i = 0; i < nstages; ++i) mbar_drain(&full[(s + i) % nstages], ph);
             }
         }
     } else if (warp == 1) {
@@ -1013,7 +1039,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             int acc = 0;
             uint32_t acc_ph = 0;
             bool ok = true;
-            const int chunk_steps = p.chunk * p.nprod;
+            const int chunk_steps = KB ? p.chunk : p.chunk * p.nprod;
             for (int t = pair; t < ntiles && ok; t += npairs) {
                 for (int c0 = 0; c0 < steps && ok; c0 += chunk_steps) {
                     if (!mbar_wait(&tempty[acc], acc_ph ^ 1, abort_flag)) { ok = false; break; }
@@ -1023,16 +1049,20 @@ __global__ void __launch_bounds__(THREADS, 1)
                     for (int st = c0; st < c1; ++st) {
                         if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t sa = smem_u32(tiles + s * STAGE_BYTES);
-                        const uint32_t sb = sa + A_TILE;
-                        const uint64_t da = a_mn ? smem_desc_mn_sw128(sa) : smem_desc_sw128(sa);
-                        const uint64_t db = b_mn ? smem_desc_mn_sw128(sb) : smem_desc_sw128(sb);
+                        const uint32_t sa = smem_u32(tiles + s * stage_bytes);
+                        const uint32_t sb = sa + nlev * A_TILE;
+                        for (int pr = 0; pr < step_prods; ++pr) {
+                            const uint32_t pa = sa + (KB ? p.pa[pr] * A_TILE : 0);
+                            const uint32_t pb = sb + (KB ? p.pb[pr] * B_HALF : 0);
+                            const uint64_t da = a_mn ? smem_desc_mn_sw128(pa) : smem_desc_sw128(pa);
+                            const uint64_t db = b_mn ? smem_desc_mn_sw128(pb) : smem_desc_sw128(pb);
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            umma_pair<TF32>(d, da + a_step * kk, db + b_step * kk, idesc,
-                                            (st > c0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; ++kk)
+                                umma_pair<TF32>(d, da + a_step * kk, db + b_step * kk, idesc,
+                                                (st > c0 || pr > 0 || kk > 0) ? 1u : 0u);
+                        }
                         commit_both(&empty[s]);
-                        if (++s == STAGES) { s = 0; ph ^= 1; }
+                        if (++s == nstages) { s = 0; ph ^= 1; }
                     }
                     commit_both(&tfull[acc]);
                     if (!ok) {
@@ -1447,6 +1477,7 @@ void set_mode_params(Params& p, const ModeInfo& mi, long kext)
     const int kblk = ROW_BYTES / (mi.tf32 ? 4 : 2);
     p.kblocks = (int)((kext + kblk - 1) / kblk);
     p.nprod = mi.nprod;
+    p.nlev = mi.nlev;
     p.chunk = mi.tf32 ? p.kblocks : (mi.nprod == 3 ? 4 : 1);
     for (int i = 0; i < 6; ++i) {
         p.pa[i] = mi.pa[i];
@@ -1533,9 +1564,29 @@ cudaError_t launch_engine(iclblasHandle_t h, const ModeInfo& mi, const Operand* 
     const long rows_a = a[0].rows, rows_b = b[0].rows;
     const int m = (int)rows_a;
     const int pair_tiles = ceil_div(m, 2 * BM) * ceil_div((long)rows_b, 256);
-    const bool pairs = pair_tiles * 2 >= h->sm_count;
     const int tiles256 = ceil_div(m, BM) * ceil_div((long)rows_b, 256);
-    const int bn = pairs ? 128 : (tiles256 * 4 < h->sm_count * 3 ? 128 : 256);  // B box rows
+    const int tiles128 = ceil_div(m, BM) * ceil_div((long)rows_b, 128);
+    // CTA pairs when they fill the GPU, unless half of each tile's columns
+    // would be empty; 128-column tiles when 256-column ones would leave a
+    // quarter of the SMs idle
+    bool pairs = pair_tiles * 2 >= h->sm_count && rows_b > 128;
+    // (BF16 modes: three quarters; a pair reads each B row from L2 once for
+    // both its CTAs)
+    if (!mi.tf32 && !p.out_half && rows_b > 128 && pair_tiles * 8 >= h->sm_count * 3) pairs = true;
+    bool narrow = tiles256 * 4 < h->sm_count * 3 || rows_b <= 128;
+    if (p.out_half && p.kblocks < 16) {
+        // short K: the tile's epilogue, not its products, takes the time, and
+        // pairs lose to single tiles (100352 x 64 x 256: 25.5 us against 19.5;
+        // 25088 x 512 x 128: 15.4 against 12.8).  Microseconds of a tile
+        // (measured) times the rounds over the SMs, 128 or 256 columns
+        const double n128 = ceil_div(tiles128, h->sm_count) * (1.4 + 0.25 * p.kblocks);
+        const double n256 = ceil_div(tiles256, h->sm_count) * (2.3 + 0.35 * p.kblocks);
+        pairs = false;
+        narrow = n128 <= n256;
+    }
+    // a stage of 256 columns and three levels would fill the ring
+    if (!mi.tf32 && !p.out_half && mi.nlev > 2) narrow = true;
+    const int bn = pairs || narrow ? 128 : 256;  // B box rows
     CUtensorMap ma[3], mb[3], mc;
     for (int l = 0; l < 3; ++l) {
         const int ll = l < mi.nlev ? l : 0;
