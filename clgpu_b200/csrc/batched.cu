@@ -49,7 +49,7 @@ cudaError_t batch_tc_create_gemm(iclblasHandle_t h, iclblasBatchPlan* plan, cons
                                  int tb);
 cudaError_t batch_tc_inverses(iclblasHandle_t h, const iclblasBatchPlan* plan, const float* const* A);
 cudaError_t batch_tc_solve(iclblasHandle_t h, const iclblasBatchPlan* plan, int adjoint, float alpha,
-                           const float* const* A, float* const* B, int operator_ready);
+                           const float* const* A, float* const* B, int operator_ready, bool forked);
 cudaError_t batch_tc_dA(iclblasHandle_t h, const iclblasBatchPlan* plan, float scale, const float* const* P,
                         const float* const* Q, float* const* dA);
 cudaError_t batch_tc_gemm(iclblasHandle_t h, const iclblasBatchPlan* plan, float alpha, const float* const* A,
@@ -157,22 +157,33 @@ __global__ void __launch_bounds__(kInvThreads) batched_inv_kernel(const int2* __
     }
     for (int idx = t; idx < TB * TB; idx += kInvThreads) Y[idx % TB][idx / TB] = 0.0;
     __syncthreads();
-    // 1. 16 x 16 diagonal sub-blocks, one column per thread
+    // 1. 16 x 16 diagonal sub-blocks, one column per thread, kept in registers
+    // (each step then waits for one FMA chain, not for shared memory and a
+    // division)
     if (t < TB) {
-        const int b = (t / 16) * 16, j = t % 16;
+        const int b = t & ~15, j = t & 15;
+        double y[16], rd[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) rd[i] = 1.0 / D[b + i][b + i];
         if (lower_op) {
+#pragma unroll
             for (int i = 0; i < 16; ++i) {
-                double y = (i == j) ? 1.0 : 0.0;
-                for (int k = j; k < i; ++k) y = fma(-D[b + i][b + k], Y[b + k][b + j], y);
-                Y[b + i][b + j] = (i >= j) ? y / D[b + i][b + i] : 0.0;
+                double acc = (i == j) ? 1.0 : 0.0;
+#pragma unroll
+                for (int k = 0; k < i; ++k) acc = fma(-D[b + i][b + k], y[k], acc);
+                y[i] = (i >= j) ? acc * rd[i] : 0.0;
             }
         } else {
+#pragma unroll
             for (int i = 15; i >= 0; --i) {
-                double y = (i == j) ? 1.0 : 0.0;
-                for (int k = i + 1; k <= j; ++k) y = fma(-D[b + i][b + k], Y[b + k][b + j], y);
-                Y[b + i][b + j] = (i <= j) ? y / D[b + i][b + i] : 0.0;
+                double acc = (i == j) ? 1.0 : 0.0;
+#pragma unroll
+                for (int k = i + 1; k < 16; ++k) acc = fma(-D[b + i][b + k], y[k], acc);
+                y[i] = (i <= j) ? acc * rd[i] : 0.0;
             }
         }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) Y[b + i][b + j] = y[i];
     }
     __syncthreads();
     // 2. doubling: blocks of size h combine into 2h (h = 16: two pairs, one
@@ -1082,6 +1093,34 @@ cudaError_t batch_plan_create_gemm(iclblasHandle_t h, int transa, int transb, in
     return cudaSuccess;
 }
 
+namespace {
+// The inverses of a tensor-core plan: two passes bound by FP64 and latency.
+// They run on the handle's second stream beside the split of the operands,
+// which is bound by HBM (`forked`: the caller joins the streams), unless
+// that stream would have to be created during a stream capture.
+cudaError_t tc_form_inverses(iclblasHandle_t h, const iclblasBatchPlan* p, int lower_op, int op,
+                             const float* const* A, bool& forked)
+{
+    forked = false;
+    bool can = h->aux_stream && h->fork_ev && h->join_ev;
+    if (!can) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        can = cudaStreamIsCapturing(h->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+        cudaGetLastError();
+    }
+    cudaStream_t side = h->stream;
+    if (can) {
+        const cudaError_t e = fork_side(h, &side);
+        if (e != cudaSuccess) return e;
+        forked = true;
+    }
+    StreamScope on_side(h, side);
+    const cudaError_t e = launch_inv(h, p->inv_items, p->n_inv, p->main.dims, p->inv_off, lower_op, op,
+                                     p->diag == ICLBLAS_DIAG_UNIT, A, p->inv);
+    return e != cudaSuccess ? e : batch_tc_inverses(h, p, A);
+}
+}  // namespace
+
 cudaError_t batch_trsm(iclblasHandle_t h, const iclblasBatchPlan* p, float alpha, const float* const* A,
                        float* const* B)
 {
@@ -1089,14 +1128,19 @@ cudaError_t batch_trsm(iclblasHandle_t h, const iclblasBatchPlan* p, float alpha
     const bool right = p->side == ICLBLAS_SIDE_RIGHT;
     const int lower_op = lower_op_of(p->uplo, p->trans) ^ (right ? 1 : 0);
     const int op = (p->trans != ICLBLAS_OP_N) ^ (right ? 1 : 0);
+    if (p->tc) {
+        bool forked = false;
+        cudaError_t e = tc_form_inverses(h, p, lower_op, op, A, forked);
+        if (e == cudaSuccess) p->inv_formed = true;
+        if (e == cudaSuccess || forked) {
+            const cudaError_t r = e == cudaSuccess ? batch_tc_solve(h, p, 0, alpha, A, B, 0, forked) : join_side(h);
+            if (e == cudaSuccess) e = r;
+        }
+        return e;
+    }
     cudaError_t e = launch_inv(h, p->inv_items, p->n_inv, p->main.dims, p->inv_off, lower_op, op,
                                p->diag == ICLBLAS_DIAG_UNIT, A, p->inv);
     if (e != cudaSuccess) return e;
-    if (p->tc) {
-        if ((e = batch_tc_inverses(h, p, A)) != cudaSuccess) return e;
-        p->inv_formed = true;
-        return batch_tc_solve(h, p, 0, alpha, A, B, 0);
-    }
     p->inv_formed = true;
     return launch_trsm(h, p->main, p->counter, p->inv_off, p->inv, lower_op, op, 0, right, alpha, A, B);
 }
@@ -1126,12 +1170,14 @@ cudaError_t batch_trsm_backward(iclblasHandle_t h, const iclblasBatchPlan* p, fl
     const int f_op = op ^ (right ? 1 : 0);
     cudaError_t e = cudaSuccess;
     const bool reuse = p->reuse_inv && p->inv_formed;
+    bool forked = false;
     if (!reuse) {
-        e = launch_inv(h, p->inv_items, p->n_inv, p->main.dims, p->inv_off, f_lower, f_op, unit, A, p->inv);
-        if (e == cudaSuccess && p->tc) e = batch_tc_inverses(h, p, A);
+        e = p->tc ? tc_form_inverses(h, p, f_lower, f_op, A, forked)
+                  : launch_inv(h, p->inv_items, p->n_inv, p->main.dims, p->inv_off, f_lower, f_op, unit, A, p->inv);
+        if (e != cudaSuccess && forked) join_side(h);
     }
     if (e == cudaSuccess)
-        e = p->tc ? batch_tc_solve(h, p, 1, alpha, A, G, reuse ? 1 : 0)
+        e = p->tc ? batch_tc_solve(h, p, 1, alpha, A, G, reuse ? 1 : 0, forked)
                   : launch_trsm(h, p->main, p->counter, p->inv_off, p->inv, !f_lower, !f_op, 1, right, alpha, A, G);
     if (e != cudaSuccess || !dA) return e;
     const float s = alpha != 0.f ? -1.f / alpha : 0.f;

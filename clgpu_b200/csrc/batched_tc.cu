@@ -56,6 +56,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -643,11 +644,81 @@ struct InvLaunch {
     Opnd w, wt;
     int nlev;
 };
-constexpr int kInvLd = 65;
+// Elements between rows in shared memory: reading a tensor-core fragment of
+// the left factor (8 rows x 4 K) wants a pitch of 4 modulo 32 words, of the
+// right factor (4 K x 8 columns) 8 modulo 32 (4 modulo 16 for FP64).
+constexpr int kInvLdA = 68, kInvLdB = 72;
 template <class Acc>
 constexpr int inv_smem_bytes()
 {
-    return 3 * 64 * kInvLd * (int)sizeof(float) + 64 * kInvLd * (int)sizeof(Acc);
+    return (2 * kInvLdB + kInvLdA) * 64 * (int)sizeof(float) + 64 * kInvLdA * (int)sizeof(Acc);
+}
+
+// D += A B, 8 x 8 x 4 in FP64: lane l holds A(l / 4, l % 4), B(l % 4, l / 4)
+// and D(l / 4, 2 (l % 4) + {0, 1})
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// 64 x 64 x 64 product of the CTA, out(r, c, v) called for every element of
+// X Y: X (pitch lx) and Y (pitch ly) row-major, K in [kb(c0), ke(r0)) only
+// (multiples of 16) for a tile at rows r0 and columns c0.
+// FP64: m8n8k4 tensor-core products, a warp 32 x 16 outputs, so that an
+// FP32 operand is converted 6 times per 64 FMAs a lane (a 4 x 4 register
+// tile converts 32 times, which bounded the pass: FP32 -> FP64 conversions
+// run at a quarter of the FMA rate).  FP32: 4 x 4 outputs a thread.
+template <class Acc, class TY, class KB, class KE, class Out>
+__device__ __forceinline__ void inv_product(const float* X, int lx, const TY* Y, int ly, KB kb, KE ke, Out out)
+{
+    const int t = threadIdx.x;
+    if constexpr (std::is_same<Acc, double>::value) {
+        const int lane = t & 31, w = t >> 5, r0 = (w >> 2) * 32, c0 = (w & 3) * 16;
+        double d[4][2][2] = {};
+        const float* xp = X + (r0 + (lane >> 2)) * lx + (lane & 3);
+        const TY* yp = Y + (lane & 3) * ly + c0 + (lane >> 2);
+        const int k1 = ke(r0 + 32);
+#pragma unroll 4
+        for (int k = kb(c0); k < k1; k += 4) {
+            double a[4], b[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = (double)xp[8 * i * lx + k];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) b[j] = (double)yp[k * ly + 8 * j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma(d[i][j], a[i], b[j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    out(r0 + 8 * i + (lane >> 2), c0 + 8 * j + 2 * (lane & 3) + e, d[i][j][e]);
+    } else {
+        const int tr = (t >> 4) * 4, tc = (t & 15) * 4;
+        float acc[4][4] = {};
+        const int k1 = ke(tr & ~15) < 64 ? ke((tr & ~15) + 16) : 64;
+        for (int k = kb(tc & ~15); k < k1; ++k) {
+            const float4 bv = *reinterpret_cast<const float4*>(Y + k * ly + tc);
+            const float b[4] = {bv.x, bv.y, bv.z, bv.w};
+            float a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = X[(tr + i) * lx + k];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) out(tr + i, tc + j, acc[i][j]);
+    }
 }
 
 template <bool TF32, class Acc>
@@ -657,11 +728,14 @@ __global__ void __launch_bounds__(256) btc_inv_kernel(const __grid_constant__ In
     constexpr int ESIZE = TF32 ? 4 : 2;
     constexpr int EPC = 16 / ESIZE;  // elements per 16-byte chunk
     constexpr int CPR = TR / EPC;    // chunks per 128-element row
-    extern __shared__ double inv_smem[];
-    Acc(*T)[kInvLd] = (Acc(*)[kInvLd])inv_smem;
-    float(*P)[kInvLd] = (float(*)[kInvLd])((Acc*)inv_smem + 64 * kInvLd);
-    float(*Q)[kInvLd] = P + 64;
-    float(*Cm)[kInvLd] = Q + 64;  // C, then the off-diagonal block of the inverse
+    extern __shared__ __align__(16) double inv_smem[];
+    Acc* const T = (Acc*)inv_smem;  // C P^-1 (lower) or C Q^-1 (upper), pitch kInvLdA
+    float* const P = (float*)(T + 64 * kInvLdA);
+    float* const Q = P + 64 * kInvLdB;
+    float* const Cm = Q + 64 * kInvLdB;  // C, then the off-diagonal block of the inverse; pitch kInvLdA
+    // the first product reads R = P (lower) or Q (upper) as its right factor,
+    // the second L = Q (lower) or P (upper) as its left one
+    const int lp = p.lower ? kInvLdB : kInvLdA, lq = p.lower ? kInvLdA : kInvLdB;
     const int t = threadIdx.x;
     const int2 it = p.items[blockIdx.x];
     const int inst = it.x, b = it.y;
@@ -690,55 +764,24 @@ __global__ void __launch_bounds__(256) btc_inv_kernel(const __grid_constant__ In
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const int idx = t + u * 256, rr = idx % 64, cc = idx / 64;
-            P[rr][cc] = vp[u];
-            Q[rr][cc] = vq[u];
-            Cm[rr][cc] = vc[u];
+            P[rr * lp + cc] = vp[u];
+            Q[rr * lq + cc] = vq[u];
+            Cm[rr * kInvLdA + cc] = vc[u];
         }
     }
     __syncthreads();
-    const int tr = (t >> 4) * 4, tc = (t & 15) * 4;
-    {
-        // T = C P^-1 (lower) or C Q^-1 (upper)
-        float(*R)[kInvLd] = p.lower ? P : Q;
-        Acc acc[4][4] = {};
-        for (int k = 0; k < 64; ++k) {
-            Acc a[4], bb[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = Cm[tr + i][k];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bb[j] = R[k][tc + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) T[tr + i][tc + j] = acc[i][j];
-    }
+    // T = C R, R triangular like M: rows of R before (lower) or after (upper)
+    // a column tile are zero there
+    const bool lo = p.lower != 0;
+    inv_product<Acc>(
+        Cm, kInvLdA, lo ? P : Q, kInvLdB, [&](int c0) { return lo ? c0 & ~15 : 0; },
+        [&](int) { return 64; }, [&](int r, int c, Acc v) { T[r * kInvLdA + c] = v; });
     __syncthreads();
-    {
-        // off-diagonal block of the inverse: -Q^-1 T (lower) or -P^-1 T (upper), into Cm
-        float(*L)[kInvLd] = p.lower ? Q : P;
-        Acc acc[4][4] = {};
-        for (int k = 0; k < 64; ++k) {
-            Acc a[4], bb[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = L[tr + i][k];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bb[j] = T[k][tc + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
-        }
-        // Cm is read only by the first product, which every thread has finished
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) Cm[tr + i][tc + j] = (float)(-acc[i][j]);
-    }
+    // off-diagonal block of the inverse: -L T, into Cm (read only by the first
+    // product, which every thread has finished)
+    inv_product<Acc>(
+        lo ? Q : P, kInvLdA, (const Acc*)T, kInvLdA, [](int) { return 0; },
+        [&](int r1) { return lo ? min(64, r1) : 64; }, [&](int r, int c, Acc v) { Cm[r * kInvLdA + c] = (float)(-v); });
     __syncthreads();
     // planes: pass 0 inv (threads along a row's chunks), pass 1 inv^T
     // (consecutive threads take consecutive rows: reading down a column of
@@ -751,12 +794,21 @@ __global__ void __launch_bounds__(256) btc_inv_kernel(const __grid_constant__ In
             // element (r, c0 + e) of inv (pass 0) or inv^T (pass 1)
             const int gr = pass ? c0 : r, gc = pass ? r : c0;  // quadrant of inv holding it
             const int hr = gr >> 6, hc = gc >> 6;
-            const float(*S)[kInvLd] = hr == hc ? (hr ? Q : P) : Cm;
+            const float* S = hr == hc ? (hr ? Q : P) : Cm;
+            const int ls = hr == hc ? (hr ? lq : lp) : kInvLdA;
             const bool zero = hr != hc && (p.lower ? hr == 0 : hr == 1);
-            float x[EPC];
+            alignas(16) float x[EPC];
+            if (pass == 0) {
 #pragma unroll
-            for (int e = 0; e < EPC; ++e)
-                x[e] = zero ? 0.f : (pass ? S[(c0 + e) & 63][r & 63] : S[r & 63][(c0 + e) & 63]);
+                for (int e = 0; e < EPC; e += 4)
+                    *reinterpret_cast<float4*>(&x[e]) = *reinterpret_cast<const float4*>(S + (r & 63) * ls + (c0 & 63) + e);
+            } else {
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) x[e] = S[((c0 + e) & 63) * ls + (r & 63)];
+            }
+            if (zero)
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) x[e] = 0.f;
             char* tile = o.base + tile_index(o, inst, b, c0 / KT) * TILE_BYTES;
             const int off16 = swz(r, c0 % KT, ESIZE);
             if (TF32) {
@@ -1196,8 +1248,10 @@ cudaError_t batch_tc_inverses(iclblasHandle_t h, const iclblasBatchPlan* plan, c
 // its transpose, with the inverse planes already formed; operator_ready:
 // the operator tiles of the plan's last forward call are still valid
 // (same A), so the adjoint (BF16 modes) splits only its first block.
+// `forked`: the inverses form on the handle's second stream (fork_side), to
+// be joined before the first product.
 cudaError_t batch_tc_solve(iclblasHandle_t h, const iclblasBatchPlan* plan, int adjoint, float alpha,
-                           const float* const* A, float* const* B, int operator_ready)
+                           const float* const* A, float* const* B, int operator_ready, bool forked)
 {
     const BatchTc& t = *plan->tc;
     // operator tiles: L[r][k] = S[r][k], S = M = op(A) (forward, and the
@@ -1211,6 +1265,10 @@ cudaError_t batch_tc_solve(iclblasHandle_t h, const iclblasBatchPlan* plan, int 
     const SplitKind ky{const_cast<const float* const*>(B), t.info_y, t.right ? 0 : 1, xp};
     const TcRange sr = !adjoint ? t.split_f : ((operator_ready && t.a_mn_b) ? t.split_b_first : t.split_b);
     cudaError_t e = run_split(h, t, sr, ks, ky);
+    if (forked) {
+        const cudaError_t j = join_side(h);
+        if (e == cudaSuccess) e = j;
+    }
     if (e != cudaSuccess) return e;
     const std::vector<TcRange>& invs = adjoint ? t.inv_b : t.inv_f;
     const std::vector<TcRange>& upds = adjoint ? t.upd_b : t.upd_f;
