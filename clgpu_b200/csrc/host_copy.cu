@@ -4,15 +4,19 @@
 // (core/src/ocl/ocl_buffer.cpp:27-42) and reads the outputs back before
 // returning (core/src/ocl/ocl_kernel.cpp:59-111); a drop-in caller therefore
 // passes ordinary malloc'd memory.  A DMA engine can only read page-locked
-// memory, so such a copy goes through pinned memory either way.  Here each
-// handle owns two pinned bounce buffers: while the DMA engine moves one
-// buffer, host threads of a process-wide pool copy the next chunk into (or
-// out of) the other, so the host-side copies and the PCIe transfers overlap.
+// memory, so such a copy goes through pinned memory either way.  Large copies
+// use two pinned bounce buffers that each handle owns: while the DMA engine
+// moves one buffer, host threads of a process-wide pool copy the next chunk
+// into (or out of) the other, so the host-side copies and the PCIe transfers
+// overlap.  Operands below the size of such a pipeline take 1 MiB chunks of
+// a small process-wide pool of pinned memory instead, copied by the same
+// threads (the driver copies them on one thread: 11 to 14 GB/s; a product of
+// 1024 x 768 x 512 on host arrays takes 287 us so, 510 through the driver).
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstring>
-#include <deque>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -23,11 +27,26 @@ namespace iclb {
 namespace {
 
 constexpr size_t kBounceBytes = (size_t)32 << 20;   // one bounce buffer
-constexpr size_t kSliceBytes = (size_t)2 << 20;     // host-copy work per thread and task
+constexpr size_t kSliceBytes = (size_t)128 << 10;   // least host-copy work per thread and copy
+constexpr int kSpinUs = 50;                         // a worker looks for the next copy this long before it sleeps
 
-// Process-wide pool of host threads for large memcpy calls (started on first
-// use).  A call splits its copy into slices, queues all but one, copies one
-// itself and waits for its own slices only.
+inline void cpu_pause()
+{
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#else
+    std::this_thread::yield();
+#endif
+}
+
+// Process-wide pool of host threads for memcpy calls (started on first use).
+// One copy at a time is shared out: the slices of it that are still to be
+// done are handed out by an atomic counter, to the workers that come and to
+// the caller itself, so the caller never waits for a thread that has yet to
+// wake up, and no lock is taken on the way (with a locked queue, eight
+// workers waking up for a 1 MiB copy cost more than the copy).  A caller that
+// finds the pool taken copies on its own thread.  Workers spin for kSpinUs
+// after a copy: the next chunk of the same call finds them awake.
 class CopyPool {
 public:
     static CopyPool& get()
@@ -38,52 +57,43 @@ public:
 
     void copy(void* dst, const void* src, size_t bytes)
     {
-        const size_t nslices = std::min<size_t>(workers_.size() + 1, (bytes + kSliceBytes - 1) / kSliceBytes);
-        if (nslices <= 1) {
+        const size_t n = std::min<size_t>(workers_.size() + 1, (bytes + kSliceBytes - 1) / kSliceBytes);
+        std::unique_lock<std::mutex> mine(owner_, std::defer_lock);
+        if (n <= 1 || !mine.try_lock()) {
             std::memcpy(dst, src, bytes);
             return;
         }
-        Batch b;
-        b.left.store((int)nslices - 1);
-        const size_t per = (bytes + nslices - 1) / nslices;
-        {
+        dst_ = (char*)dst;
+        src_ = (const char*)src;
+        bytes_ = bytes;
+        per_ = ((bytes + n - 1) / n + 63) & ~(size_t)63;
+        slices_ = (int)((bytes + per_ - 1) / per_);
+        next_.store(0);
+        done_.store(0);
+        open_.store(true);      // workers may enter
+        copies_.fetch_add(1);   // and know there is something new
+        if (sleeping_.load() > 0) {
             std::lock_guard<std::mutex> lock(mu_);
-            for (size_t i = 1; i < nslices; ++i) {
-                const size_t off = i * per;
-                if (off >= bytes) {
-                    b.left.fetch_sub(1);
-                    continue;
-                }
-                q_.push_back(Task{(char*)dst + off, (const char*)src + off, std::min(per, bytes - off), &b});
-            }
+            cv_.notify_all();
         }
-        cv_.notify_all();
-        std::memcpy(dst, src, std::min(per, bytes));
-        std::unique_lock<std::mutex> lock(mu_);
-        done_.wait(lock, [&] { return b.left.load() == 0; });
+        work();
+        while (done_.load() < slices_) cpu_pause();
+        // no worker may look at this copy once the next one is set up
+        open_.store(false);
+        while (inside_.load() > 0) cpu_pause();
     }
 
     ~CopyPool()
     {
         {
             std::lock_guard<std::mutex> lock(mu_);
-            stop_ = true;
+            stop_.store(true);
         }
         cv_.notify_all();
         for (auto& t : workers_) t.join();
     }
 
 private:
-    struct Batch {
-        std::atomic<int> left{0};
-    };
-    struct Task {
-        char* dst;
-        const char* src;
-        size_t bytes;
-        Batch* batch;
-    };
-
     CopyPool()
     {
         const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
@@ -91,26 +101,105 @@ private:
         for (unsigned i = 0; i < n; ++i) workers_.emplace_back([this] { run(); });
     }
 
-    void run()
+    void work()
     {
-        std::unique_lock<std::mutex> lock(mu_);
-        for (;;) {
-            cv_.wait(lock, [&] { return stop_ || !q_.empty(); });
-            if (stop_ && q_.empty()) return;
-            Task t = q_.front();
-            q_.pop_front();
-            lock.unlock();
-            std::memcpy(t.dst, t.src, t.bytes);
-            lock.lock();
-            if (t.batch->left.fetch_sub(1) == 1) done_.notify_all();
+        for (int i = next_.fetch_add(1); i < slices_; i = next_.fetch_add(1)) {
+            const size_t off = (size_t)i * per_;
+            std::memcpy(dst_ + off, src_ + off, std::min(per_, bytes_ - off));
+            done_.fetch_add(1);
         }
     }
 
+    void run()
+    {
+        unsigned seen = 0;
+        for (;;) {
+            const auto t0 = std::chrono::steady_clock::now();
+            while (copies_.load() == seen && !stop_.load() &&
+                   std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(kSpinUs))
+                cpu_pause();
+            if (copies_.load() == seen) {
+                std::unique_lock<std::mutex> lock(mu_);
+                sleeping_.fetch_add(1);
+                cv_.wait(lock, [&] { return stop_.load() || copies_.load() != seen; });
+                sleeping_.fetch_sub(1);
+            }
+            if (stop_.load()) return;
+            seen = copies_.load();
+            // the caller closes the copy and then waits for inside_ == 0: a
+            // worker that still finds it open is waited for
+            inside_.fetch_add(1);
+            if (open_.load()) work();
+            inside_.fetch_sub(1);
+        }
+    }
+
+    std::mutex owner_;  // held by the caller whose copy is shared out
+    char* dst_ = nullptr;
+    const char* src_ = nullptr;
+    size_t bytes_ = 0, per_ = 0;
+    int slices_ = 0;
+    std::atomic<int> next_{0}, done_{0}, inside_{0}, sleeping_{0};
+    std::atomic<unsigned> copies_{0};
+    std::atomic<bool> open_{false}, stop_{false};
     std::mutex mu_;
-    std::condition_variable cv_, done_;
-    std::deque<Task> q_;
+    std::condition_variable cv_;
     std::vector<std::thread> workers_;
-    bool stop_ = false;
+};
+
+// Process-wide pool of pinned chunks for small copies: at most kMaxChunks, made
+// as they are needed, given back to the system when the last handle goes.  A
+// call holds a chunk until its DMA is over; with none left the caller copies
+// through the driver.
+class PinnedPool {
+public:
+    static PinnedPool& get()
+    {
+        static PinnedPool* pool = new PinnedPool();  // never destroyed: handles may outlive static objects
+        return *pool;
+    }
+    void retain()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        ++handles_;
+    }
+    void release()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (--handles_ > 0) return;
+        for (void* c : free_)
+            if (cudaFreeHost(c) != cudaSuccess) cudaGetLastError();
+        made_ -= (int)free_.size();
+        free_.clear();
+    }
+    void* take()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (!free_.empty()) {
+            void* c = free_.back();
+            free_.pop_back();
+            return c;
+        }
+        if (made_ >= kMaxChunks) return nullptr;
+        void* c = nullptr;
+        if (cudaHostAlloc(&c, kPinnedChunk, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        ++made_;
+        return c;
+    }
+    void give(void* c)
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        free_.push_back(c);
+    }
+
+private:
+    static constexpr int kMaxChunks = 16;
+    std::mutex mu_;
+    std::vector<void*> free_;
+    int made_ = 0, handles_ = 0;
 };
 
 cudaError_t ensure_bounce(iclblasHandle_t h)
@@ -134,6 +223,11 @@ cudaError_t bounce_free(iclblasHandle_t h, int b)
 }
 
 }  // namespace
+
+void pinned_retain() { PinnedPool::get().retain(); }
+void pinned_release() { PinnedPool::get().release(); }
+void* pinned_take() { return PinnedPool::get().take(); }
+void pinned_give(void* chunk) { PinnedPool::get().give(chunk); }
 
 void host_copy(void* dst, const void* src, size_t bytes) { CopyPool::get().copy(dst, src, bytes); }
 

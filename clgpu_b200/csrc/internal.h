@@ -169,6 +169,13 @@ private:
 cudaError_t copy_pageable_h2d(iclblasHandle_t h, void* dst_dev, const void* src_host, size_t bytes);
 cudaError_t copy_pageable_d2h(iclblasHandle_t h, void* dst_host, const void* src_dev, size_t bytes);
 cudaError_t free_bounce(iclblasHandle_t h);
+// Pinned chunks of kPinnedChunk bytes from a bounded process-wide pool
+// (nullptr: none left), kept while any handle exists.
+constexpr size_t kPinnedChunk = (size_t)1 << 20;
+void pinned_retain();
+void pinned_release();
+void* pinned_take();
+void pinned_give(void* chunk);
 // memcpy between host buffers on the process-wide pool of copy threads.
 void host_copy(void* dst, const void* src, size_t bytes);
 
