@@ -1098,9 +1098,11 @@ __global__ void __launch_bounds__(THREADS, 1)
 // Logical operand L (R x K): L[r][k] = S[r*rs + k*ks] (conj if requested).
 // Output planes are K-major with row pitch kpad elements.
 // Real:    plane[l][r*kpad + k]            (k >= K: zero)
-// Complex A: plane[l][r*kpad + k] = re, [r*kpad + K + k] = im       (kpad >= 2K)
-// Complex B: plane[l][(2r)*kpad + k] = re, [(2r)*kpad + K + k] = -im,
-//            plane[l][(2r+1)*kpad + k] = im, [(2r+1)*kpad + K + k] = re
+// Complex, Kp = K rounded up to 8 (16-byte stores of the second half), zeros
+// between K and Kp and past 2 Kp:
+//   A: plane[l][r*kpad + k] = re, [r*kpad + Kp + k] = im
+//   B: plane[l][(2r)*kpad + k] = re, [(2r)*kpad + Kp + k] = -im,
+//      plane[l][(2r+1)*kpad + k] = im, [(2r+1)*kpad + Kp + k] = re
 enum SplitMode { kReal = 0, kCplxA = 1, kCplxB = 2 };
 
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& hi, __nv_bfloat16& mid, __nv_bfloat16& lo)
@@ -1126,17 +1128,43 @@ struct SplitOut {
     long kpad;
 };
 
-__device__ __forceinline__ void put(const SplitOut& o, long idx, float x)
+// One operand to split (the kernels below).
+struct SplitJob {
+    const void* S;
+    int R, K;
+    long rs, ks;
+    SplitOut o;
+    long kw;             // K values written per row (real)
+    int tri, unit;       // real
+    long szs, dzs;       // real, several equal operands
+    int vin, vout;       // real
+    int mode, conj;      // complex
+};
+
+// Eight consecutive K values of one row: the levels of x at element off of
+// every plane (16-byte aligned there).
+__device__ __forceinline__ void put8(const SplitOut& o, long off, const float (&x)[8])
 {
     if (o.tf32) {
-        ((float*)o.plane[0])[idx] = to_tf32(x);
+        float4* d = reinterpret_cast<float4*>((float*)o.plane[0] + off);
+        d[0] = make_float4(to_tf32(x[0]), to_tf32(x[1]), to_tf32(x[2]), to_tf32(x[3]));
+        d[1] = make_float4(to_tf32(x[4]), to_tf32(x[5]), to_tf32(x[6]), to_tf32(x[7]));
         return;
     }
-    __nv_bfloat16 h, m, l;
-    split3(x, h, m, l);
-    ((__nv_bfloat16*)o.plane[0])[idx] = h;
-    if (o.nlev > 1) ((__nv_bfloat16*)o.plane[1])[idx] = m;
-    if (o.nlev > 2) ((__nv_bfloat16*)o.plane[2])[idx] = l;
+    uint32_t w[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        __nv_bfloat16 ha, ma, la, hb, mb, lb;
+        split3(x[2 * e], ha, ma, la);
+        split3(x[2 * e + 1], hb, mb, lb);
+        w[0][e] = (uint32_t)__bfloat16_as_ushort(ha) | ((uint32_t)__bfloat16_as_ushort(hb) << 16);
+        w[1][e] = (uint32_t)__bfloat16_as_ushort(ma) | ((uint32_t)__bfloat16_as_ushort(mb) << 16);
+        w[2][e] = (uint32_t)__bfloat16_as_ushort(la) | ((uint32_t)__bfloat16_as_ushort(lb) << 16);
+    }
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+        if (l < o.nlev)
+            *reinterpret_cast<uint4*>((__nv_bfloat16*)o.plane[l] + off) = make_uint4(w[l][0], w[l][1], w[l][2], w[l][3]);
 }
 
 // Real operands: 64 rows x 64 K per block (256 threads).  Bound by HBM (4
@@ -1150,17 +1178,26 @@ __device__ __forceinline__ void put(const SplitOut& o, long idx, float x)
 // Row r goes to plane + r * o.kpad, K values [0, kw) (zeros for k >= K; kw
 // even).  `tri` masks L to a triangle (1: keep k <= r, 2: keep k >= r; `unit`
 // puts 1 on the diagonal); tiles wholly outside the kept triangle are left
-// unwritten.  blockIdx.z selects one of several equal operands: source
-// + z * szs, destination row offset + z * dzs.
-__global__ void __launch_bounds__(256) split_real_kernel(int R, int K, const float* __restrict__ S, long rs, long ks,
-                                                         SplitOut o, long kw, int tri, int unit, long szs, long dzs,
-                                                         int vin, int vout)
+// unwritten.  `two`: blockIdx.z selects the operand, a or b (both of a
+// product in one launch); else it selects one of several equal operands a:
+// source + z * szs, destination row offset + z * dzs.
+__global__ void __launch_bounds__(256) split_real_kernel(const __grid_constant__ SplitJob a,
+                                                         const __grid_constant__ SplitJob b, int two)
 {
     __shared__ float tile[64][65];
+    const bool sb = two && blockIdx.z;
+    const SplitOut o = sb ? b.o : a.o;
+    const float* S = (const float*)(sb ? b.S : a.S);
+    const int R = sb ? b.R : a.R, K = sb ? b.K : a.K;
+    const long rs = sb ? b.rs : a.rs, ks = sb ? b.ks : a.ks, kw = sb ? b.kw : a.kw;
+    const int vin = sb ? b.vin : a.vin, vout = sb ? b.vout : a.vout;
+    const int tri = a.tri, unit = a.unit;  // (0 for a product's operands)
     const int k0 = blockIdx.x * 64, r0 = blockIdx.y * 64, t = threadIdx.x;
+    if (r0 >= R || k0 >= kw) return;
     if ((tri == 1 && k0 > r0 + 63) || (tri == 2 && k0 + 63 < r0)) return;
-    S += (long)blockIdx.z * szs;
-    const long dz = (long)blockIdx.z * dzs;
+    const long z = two ? 0 : blockIdx.z;
+    S += z * a.szs;
+    const long dz = z * a.dzs;
     // f runs along the contiguous dimension of the source, g across it
     const bool rc = rs == 1;
     const int f0 = rc ? r0 : k0, nf = rc ? R : K, g0 = rc ? k0 : r0, ng = rc ? K : R;
@@ -1210,55 +1247,105 @@ __global__ void __launch_bounds__(256) split_real_kernel(int R, int K, const flo
             }
         }
         const long off = ((long)r + dz) * o.kpad + k;  // even: 4- and 8-byte aligned pairs
-        if (o.tf32) {
-            float* d = (float*)o.plane[0] + off;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] = to_tf32(x[e]);
-            if (vout) {
-                reinterpret_cast<float4*>(d)[0] = make_float4(x[0], x[1], x[2], x[3]);
-                reinterpret_cast<float4*>(d)[1] = make_float4(x[4], x[5], x[6], x[7]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; e += 2)
-                    if (k + e < kw) *reinterpret_cast<float2*>(d + e) = make_float2(x[e], x[e + 1]);
-            }
+        if (vout) {
+            put8(o, off, x);
         } else {
-            uint32_t w[3][4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                __nv_bfloat16 ha, ma, la, hb, mb, lb;
-                split3(x[2 * e], ha, ma, la);
-                split3(x[2 * e + 1], hb, mb, lb);
-                w[0][e] = (uint32_t)__bfloat16_as_ushort(ha) | ((uint32_t)__bfloat16_as_ushort(hb) << 16);
-                w[1][e] = (uint32_t)__bfloat16_as_ushort(ma) | ((uint32_t)__bfloat16_as_ushort(mb) << 16);
-                w[2][e] = (uint32_t)__bfloat16_as_ushort(la) | ((uint32_t)__bfloat16_as_ushort(lb) << 16);
-            }
-#pragma unroll
-            for (int l = 0; l < 3; ++l) {
-                if (l >= o.nlev) break;
-                __nv_bfloat16* d = (__nv_bfloat16*)o.plane[l] + off;
-                if (vout) {
-                    *reinterpret_cast<uint4*>(d) = make_uint4(w[l][0], w[l][1], w[l][2], w[l][3]);
+            for (int e = 0; e < 8; e += 2) {
+                if (k + e >= kw) break;
+                if (o.tf32) {
+                    *reinterpret_cast<float2*>((float*)o.plane[0] + off + e) =
+                        make_float2(to_tf32(x[e]), to_tf32(x[e + 1]));
                 } else {
+                    __nv_bfloat16 ha, ma, la, hb, mb, lb;
+                    split3(x[e], ha, ma, la);
+                    split3(x[e + 1], hb, mb, lb);
+                    const __nv_bfloat162 v[3] = {__halves2bfloat162(ha, hb), __halves2bfloat162(ma, mb),
+                                                 __halves2bfloat162(la, lb)};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (k + 2 * e < kw) reinterpret_cast<uint32_t*>(d)[e] = w[l][e];
+                    for (int l = 0; l < 3; ++l)
+                        if (l < o.nlev)
+                            *reinterpret_cast<__nv_bfloat162*>((__nv_bfloat16*)o.plane[l] + off + e) = v[l];
                 }
             }
         }
     }
 }
 
-// Launches split_real_kernel: nz operands of R rows, K values [0, kw) each.
-cudaError_t launch_split_real(cudaStream_t st, const float* S, int R, int K, long rs, long ks, const SplitOut& o,
-                              long kw, int tri, int unit, int nz, long szs, long dzs)
+// Complex operands of a product, both in one launch (blockIdx.z): 64 rows x
+// 64 K per block, the same scheme: 16 loads a thread in flight, 8
+// consecutive K of a row a store.  (32 x 32 tiles with 2-byte stores, a
+// launch per operand and two more for the padding, took two thirds of a
+// 1969 x 1300 x 313 3xBF16 call.)
+__global__ void __launch_bounds__(256) split_cplx_kernel(const __grid_constant__ SplitJob a,
+                                                         const __grid_constant__ SplitJob b)
 {
-    const int vin = ((uintptr_t)S & 15) == 0 && ((rs == 1 ? ks : rs) & 3) == 0 && (szs & 3) == 0;
+    __shared__ float2 tile[64][65];
+    const bool sb = blockIdx.z != 0;
+    const SplitOut o = sb ? b.o : a.o;
+    const float2* S = (const float2*)(sb ? b.S : a.S);
+    const int R = sb ? b.R : a.R, K = sb ? b.K : a.K, Kp = (K + 7) & ~7;
+    const long rs = sb ? b.rs : a.rs, ks = sb ? b.ks : a.ks;
+    const bool conj = (sb ? b.conj : a.conj) != 0, amode = (sb ? b.mode : a.mode) == kCplxA;
+    const int k0 = blockIdx.x * 64, r0 = blockIdx.y * 64, t = threadIdx.x;
+    if (r0 >= R || k0 >= Kp) return;
+    const bool rc = rs == 1;
+    const int f0 = rc ? r0 : k0, nf = rc ? R : K, g0 = rc ? k0 : r0, ng = rc ? K : R;
+    const long gs = rc ? ks : rs;
+    float2 v[16];
+    const int f = t % 64;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int g = t / 64 + 4 * u;
+        v[u] = (f0 + f < nf && g0 + g < ng) ? __ldg(S + (long)(g0 + g) * gs + f0 + f) : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int g = t / 64 + 4 * u;
+        tile[rc ? f : g][rc ? g : f] = v[u];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int rr = t / 8 + 32 * u, kk = (t % 8) * 8;
+        const int r = r0 + rr, k = k0 + kk;
+        if (r >= R || k >= Kp) continue;
+        float re[8], im[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 w = tile[rr][kk + e];
+            re[e] = w.x;
+            im[e] = conj ? -w.y : w.y;
+        }
+        if (amode) {
+            put8(o, (long)r * o.kpad + k, re);
+            put8(o, (long)r * o.kpad + Kp + k, im);
+        } else {
+            put8(o, (2L * r) * o.kpad + k, re);
+            put8(o, (2L * r + 1) * o.kpad + k, im);
+            put8(o, (2L * r + 1) * o.kpad + Kp + k, re);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) im[e] = -im[e];
+            put8(o, (2L * r) * o.kpad + Kp + k, im);
+        }
+    }
+    // zeros past both halves, by the blocks of the last K tile
+    const int tail = (int)(o.kpad - 2L * Kp) / 8;
+    if (k0 + 64 >= Kp && tail > 0) {
+        const float zero[8] = {};
+        const int rows = min(64, R - r0) * (amode ? 1 : 2);
+        for (int i = t; i < rows * tail; i += 256)
+            put8(o, ((amode ? 1L : 2L) * r0 + i / tail) * o.kpad + 2L * Kp + 8 * (i % tail), zero);
+    }
+}
+
+SplitJob real_job(const float* S, int R, int K, long rs, long ks, const SplitOut& o, long kw, int tri = 0,
+                  int unit = 0, long szs = 0, long dzs = 0)
+{
     bool vout = (kw & 7) == 0 && (o.kpad & 7) == 0;
     for (int l = 0; l < (o.tf32 ? 1 : o.nlev); ++l) vout = vout && ((uintptr_t)o.plane[l] & 15) == 0;
-    dim3 grid((unsigned)ceil_div(kw, 64L), (unsigned)ceil_div(R, 64), (unsigned)nz);
-    split_real_kernel<<<grid, 256, 0, st>>>(R, K, S, rs, ks, o, kw, tri, unit, szs, dzs, vin, (int)vout);
-    return cudaGetLastError();
+    const int vin = ((uintptr_t)S & 15) == 0 && ((rs == 1 ? ks : rs) & 3) == 0 && (szs & 3) == 0;
+    return SplitJob{S, R, K, rs, ks, o, kw, tri, unit, szs, dzs, vin, (int)vout, 0, 0};
 }
 
 // IEEE half operands (HGEMM): 32 x 64 tiles, values copied into
@@ -1288,71 +1375,6 @@ __global__ void __launch_bounds__(256) pack_half_kernel(int R, int K, const __ha
         const int r = r0 + rr, k = k0 + 2 * kp;
         if (r >= R || k >= kpad) continue;
         *reinterpret_cast<__half2*>(plane + (long)r * kpad + k) = __halves2half2(tile[rr][2 * kp], tile[rr][2 * kp + 1]);
-    }
-}
-
-// Complex operands: 32 x 32 tile of L per block (blockDim 32 x 8), transposed
-// through shared memory when the source is contiguous along r, so that both
-// the reads of S and the K-contiguous writes are coalesced.
-template <class T>
-__global__ void __launch_bounds__(256) split_kernel(int R, int K, const T* __restrict__ S, long rs, long ks, int conj,
-                                                    int mode, SplitOut o)
-{
-    __shared__ T tile[32][33];
-    const int k0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    // load tile[rr][kk] = L[r0+rr][k0+kk]
-    if (rs == 1) {  // contiguous along r
-        for (int kk = ty; kk < 32; kk += 8) {
-            const int r = r0 + tx, k = k0 + kk;
-            T v{};
-            if (r < R && k < K) v = S[(long)r + (long)k * ks];
-            tile[tx][kk] = v;
-        }
-    } else {
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            T v{};
-            if (r < R && k < K) v = S[(long)r * rs + (long)k];
-            tile[rr][tx] = v;
-        }
-    }
-    __syncthreads();
-    for (int rr = ty; rr < 32; rr += 8) {
-        const int r = r0 + rr, k = k0 + tx;
-        if (r >= R) continue;
-        const T v = tile[rr][tx];
-        if constexpr (sizeof(T) == sizeof(float)) {
-            // real: K is padded to a multiple of the block by the grid; k >= K writes zeros
-            if (k < o.kpad) put(o, (long)r * o.kpad + k, k < K ? (float)*(const float*)&v : 0.f);
-        } else {
-            const float re = ((const float*)&v)[0];
-            const float im = (conj ? -1.f : 1.f) * ((const float*)&v)[1];
-            if (k >= K) continue;
-            if (mode == kCplxA) {
-                put(o, (long)r * o.kpad + k, re);
-                put(o, (long)r * o.kpad + K + k, im);
-            } else {
-                put(o, (long)(2 * r) * o.kpad + k, re);
-                put(o, (long)(2 * r) * o.kpad + K + k, -im);
-                put(o, (long)(2 * r + 1) * o.kpad + k, im);
-                put(o, (long)(2 * r + 1) * o.kpad + K + k, re);
-            }
-        }
-    }
-}
-
-// zero the K padding columns [kfrom, kpad) of every row (complex layouts)
-__global__ void zero_pad_kernel(long rows, long kfrom, SplitOut o)
-{
-    const long w = o.kpad - kfrom;
-    const long total = rows * w;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-        const long r = e / w, k = kfrom + e % w;
-        const long idx = r * o.kpad + k;
-        if (o.tf32) ((float*)o.plane[0])[idx] = 0.f;
-        else
-            for (int l = 0; l < o.nlev; ++l) ((__nv_bfloat16*)o.plane[l])[idx] = __float2bfloat16_rn(0.f);
     }
 }
 
@@ -1485,24 +1507,14 @@ void set_mode_params(Params& p, const ModeInfo& mi, long kext)
     }
 }
 
-template <class T>
-cudaError_t run_split(iclblasHandle_t h, const T* S, int R, int K, long rs, long ks, int conj, int mode,
-                      const SplitOut& o, long out_rows)
+// Both operands of a product, one launch.
+cudaError_t run_split_pair(iclblasHandle_t h, bool cplx, const SplitJob& a, const SplitJob& b)
 {
-    if (std::is_same<T, float>::value) {
-        return launch_split_real(h->stream, (const float*)S, R, K, rs, ks, o, o.kpad, 0, 0, 1, 0, 0);
-    }
-    dim3 grid(ceil_div(K, 32), ceil_div(R, 32));
-    split_kernel<T><<<grid, dim3(32, 8), 0, h->stream>>>(R, K, S, rs, ks, conj, mode, o);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (!std::is_same<T, float>::value && o.kpad > 2L * K) {
-        const long total = out_rows * (o.kpad - 2L * K);
-        const int g = (int)std::min<long>((total + 255) / 256, (long)h->sm_count * 8);
-        zero_pad_kernel<<<g, 256, 0, h->stream>>>(out_rows, 2L * K, o);
-        e = cudaGetLastError();
-    }
-    return e;
+    auto k_of = [&](const SplitJob& j) { return cplx ? (long)((j.K + 7) & ~7) : j.kw; };
+    const dim3 grid((unsigned)ceil_div(std::max(k_of(a), k_of(b)), 64L), (unsigned)ceil_div(std::max(a.R, b.R), 64), 2);
+    if (cplx) split_cplx_kernel<<<grid, 256, 0, h->stream>>>(a, b);
+    else split_real_kernel<<<grid, 256, 0, h->stream>>>(a, b, 1);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1664,7 +1676,7 @@ cudaError_t gemm_tc(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T al
     const ModeInfo mi = mode_info(h->math);
     const int esize = mi.tf32 ? 4 : 2;
     const int kblk = ROW_BYTES / esize;
-    const long kreal = cplx ? 2L * k : (long)k;
+    const long kreal = cplx ? 2L * ((k + 7) & ~7) : (long)k;
     const long kpad = (kreal + kblk - 1) / kblk * kblk;
     const long rows_a = m, rows_b = cplx ? 2L * n : (long)n;
     const size_t plane_a = (size_t)rows_a * kpad * esize, plane_b = (size_t)rows_b * kpad * esize;
@@ -1682,10 +1694,14 @@ cudaError_t gemm_tc(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T al
     }
     // A: L[r=m][k] ; op N: S[m + k*lda] ; op T/C: S[k + m*lda]
     const bool at = ta != ICLBLAS_OP_N, bt = tb != ICLBLAS_OP_N;
-    cudaError_t e = run_split<T>(h, A, m, k, at ? lda : 1, at ? 1 : lda, ta == ICLBLAS_OP_C, kCplxA, oa, rows_a);
-    if (e != cudaSuccess) return e;
     // B: L[r=n][k] = op(B)[k][n] ; op N: S[k + n*ldb] ; op T/C: S[n + k*ldb]
-    e = run_split<T>(h, B, n, k, bt ? 1 : ldb, bt ? ldb : 1, tb == ICLBLAS_OP_C, kCplxB, ob, rows_b);
+    SplitJob ja = real_job((const float*)A, m, k, at ? lda : 1, at ? 1 : lda, oa, kpad);
+    SplitJob jb = real_job((const float*)B, n, k, bt ? 1 : ldb, bt ? ldb : 1, ob, kpad);
+    ja.mode = kCplxA;
+    jb.mode = kCplxB;
+    ja.conj = ta == ICLBLAS_OP_C;
+    jb.conj = tb == ICLBLAS_OP_C;
+    cudaError_t e = run_split_pair(h, cplx, ja, jb);
     if (e != cudaSuccess) return e;
 
     Params p{};
@@ -1823,7 +1839,10 @@ cudaError_t split_planes_tc(iclblasHandle_t h, const float* S, int R, int K, lon
     o.tf32 = dst.tf32;
     o.kpad = dst.pitch;
     for (int l = 0; l < dst.nlev; ++l) o.plane[l] = (char*)dst.plane[l] + (row0 * dst.pitch + k0) * esize;
-    return launch_split_real(h->stream, S, R, K, rs, ks, o, kw, tri, unit, nz, szs, dzs);
+    const SplitJob j = real_job(S, R, K, rs, ks, o, kw, tri, unit, szs, dzs);
+    const dim3 grid((unsigned)ceil_div(kw, 64L), (unsigned)ceil_div(R, 64), (unsigned)nz);
+    split_real_kernel<<<grid, 256, 0, h->stream>>>(j, j, 0);
+    return cudaGetLastError();
 }
 
 template cudaError_t gemm_tc<float>(iclblasHandle_t, int, int, int, int, int, float, const float*, int, const float*,
