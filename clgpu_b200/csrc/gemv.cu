@@ -405,6 +405,47 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_kernel(int m, int n, T alpha
     }
 }
 
+// Tall columns without 16-byte alignment: a block a column, its rows in eight
+// runs, one a warp, 8 loads of each operand in flight, the warps' sums added
+// in shared memory.  Against a warp a column, in slices whose sums go through
+// global memory and an atomic (us, operands in L2): real 3001 x 1777 11.1,
+// 7.3; 5000 x 100 9.4, 3.1; complex 5000 x 5001 55, 43; but 600 x 9000 6.9,
+// 14.2 and real 9001 x 9000 74, 79.
+template <class T, bool CONJ>
+__global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha, const T* __restrict__ A, long lda,
+                                                                 const T* __restrict__ x, long incx, T beta,
+                                                                 T* __restrict__ y, long incy, int seg)
+{
+    constexpr int W = kTThreads / 32, U = 8;
+    __shared__ T part[W];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long col = blockIdx.x;
+    const T* Ac = A + col * lda;
+    const int r1 = min(m, (w + 1) * seg);
+    T acc = zero_of(T());
+    for (int r = w * seg + lane; r < r1; r += U * 32) {
+        T v[U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = r + u * 32 < r1;
+            v[u] = in ? ldg_of(Ac + r + u * 32) : zero_of(T());
+            xv[u] = in ? ldg_of(x + (long)(r + u * 32) * incx) : zero_of(T());
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (r + u * 32 < r1) madd<CONJ>(acc, v[u], xv[u]);
+    }
+    acc = warp_sum_t(acc);
+    if (lane == 0) part[w] = acc;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    T sum = part[0];
+#pragma unroll
+    for (int k = 1; k < W; ++k) sum = add(sum, part[k]);
+    T* yp = y + col * incy;
+    *yp = axpby(alpha, sum, beta, yp);
+}
+
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 template <class T>
@@ -452,6 +493,15 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     }
     // op T / C: columns of A are dot products with x
     const bool vec = aligned16(A) && ((long)lda * sizeof(T)) % 16 == 0 && incx == 1 && aligned16(x);
+    const bool conj = (trans == ICLBLAS_OP_C) && sizeof(T) == sizeof(cfloat);
+    if (!vec && m >= 1024 && n <= 6000) {
+        const int seg = ceil_div(ceil_div(m, kTThreads / 32), 32) * 32;
+        if (conj)
+            gemv_t_block_kernel<T, true><<<n, kTThreads, 0, h->stream>>>(m, alpha, A, lda, x, incx, beta, y, incy, seg);
+        else
+            gemv_t_block_kernel<T, false><<<n, kTThreads, 0, h->stream>>>(m, alpha, A, lda, x, incx, beta, y, incy, seg);
+        return cudaGetLastError();
+    }
     const int warps_target = target * (kTThreads / 32);
     int S = 1;
     // (a real scalar load brings a quarter as much: shorter slices)
@@ -467,7 +517,6 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     }
     const long warps = (long)n * S;
     const int grid = (int)((warps * 32 + kTThreads - 1) / kTThreads);
-    const bool conj = (trans == ICLBLAS_OP_C) && sizeof(T) == sizeof(cfloat);
 #define LAUNCH(C, V)                                                                                         \
     gemv_t_kernel<T, C, V><<<grid, kTThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, S, \
                                                               rps, partial, h->ws.counters)
