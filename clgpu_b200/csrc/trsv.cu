@@ -15,6 +15,7 @@
 // Every wait is bounded: a CTA that gives up records kDevWaitTimeout in the
 // device status word and returns, and so do the CTAs that wait for it; the
 // host reports EXECUTION_FAILED.
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <type_traits>
@@ -784,6 +785,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 // step no shorter: the hand-off, not the products, sets it).
 constexpr int NB = 64;
 constexpr int kBStages = 3;
+// CTAs of a cluster: up to 16 for solves of at most kBWide blocks (fewer
+// hand-offs through global memory: real n = 2048 41 us with 8, 38 with 16,
+// n = 3072 55 and 50, complex n = 3072 68 and 66), up to 8 for longer ones,
+// whose clusters of 16 wait for GPCs with 16 free SMs (complex n = 4096 89
+// and 93, real n = 8192 172 and 179).
+constexpr int kBCluster = 16, kBWide = 48;
 
 struct alignas(16) dcomplex {
     double re, im;
@@ -855,12 +862,12 @@ __device__ __forceinline__ int bpitch(int op)
 template <class T>
 struct alignas(16) BlockSmem {
     T stage[kBStages][NB * kBPitch];   // tiles, [column][row] (op N) or [row][column]
-    T xin[kMaxCluster][kBEntries<T>];  // solved blocks of earlier CTAs of this cluster (st.async)
+    T xin[kBCluster][kBEntries<T>];    // solved blocks of earlier CTAs of this cluster (st.async)
     T xs[2][kBEntries<T>];             // a solved block from the published words
     T y2[kBEntries<T>];                // b - the products of the earlier blocks
     wide_t<T> Y[NB][NB + 1];  // FP64 inverse of the diagonal block (the other triangle: doubling temporaries)
     T D[NB][NB + 1];          // the diagonal block of op(A)
-    uint64_t xbar[kMaxCluster];
+    uint64_t xbar[kBCluster];
     unsigned s, epoch, cl;
 };
 static_assert(sizeof(BlockSmem<cfloat>) <= 232448 && 2 * (sizeof(BlockSmem<float>) + 1024) <= 233472,
@@ -1158,11 +1165,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     asm volatile("cp.async.wait_all;" ::: "memory");
 
     // ---- this block's step of the chain
-    // hand-off: lane cg sends this thread's two rows to rank + 1 + cg
-    uint32_t dx = 0, db = 0;
-    if (cl > 1 && rank + 1 + cg < (unsigned)cl && cfirst + (int)rank + 1 + cg < nb) {
-        dx = map_to(&S.xin[rank][bidx<T>(R0)], rank + 1 + cg);
-        db = map_to(&S.xbar[rank], rank + 1 + cg);
+    // hand-off: lane cg sends this thread's two rows to rank + 1 + cg and rank + 9 + cg
+    uint32_t dx[2] = {0, 0}, db[2] = {0, 0};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const unsigned d = rank + 1 + cg + 8 * u;
+        if (cl > 1 && d < (unsigned)cl && cfirst + (int)d < nb) {
+            dx[u] = map_to(&S.xin[rank][bidx<T>(R0)], d);
+            db[u] = map_to(&S.xbar[rank], d);
+        }
     }
     // the solved entries of block s-1, once they are known (every thread calls it)
     auto last_x = [&]() -> const T* {
@@ -1214,9 +1225,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         for (int k = 0; k < 2; ++k)
             if (R0 + 8 * k >= nr) o[k] = zero_v(T());
         // the hand-offs first, then the published words; the output x last
-        if (db != 0 && cg == 0) st_async_pair(dx, o[0], o[1], db);
+        if (db[0] != 0 && cg == 0) st_async_pair(dx[0], o[0], o[1], db[0]);
         __syncwarp();
-        if (db != 0 && cg != 0) st_async_pair(dx, o[0], o[1], db);
+        if (db[0] != 0 && cg != 0) st_async_pair(dx[0], o[0], o[1], db[0]);
+        if (db[1] != 0) st_async_pair(dx[1], o[0], o[1], db[1]);
         const int k = cg / kW, row = R0 + 8 * k;
         if (cg < 2 * kW && row < nr) {
             const T v = k == 0 ? o[0] : o[1];
@@ -1382,7 +1394,7 @@ cudaError_t strsv_tma(iclblasHandle_t h, int uplo, int trans, int diag, int n, c
 template <class T>
 int trsv_block_capacity(int device, int cl)
 {
-    static std::atomic<int> cap[64][kMaxCluster + 1];  // capacity + 1; 0: not asked yet
+    static std::atomic<int> cap[64][kBCluster + 1];  // capacity + 1; 0: not asked yet
     std::atomic<int>& c = cap[device & 63][cl];
     int v = c.load();
     if (v == 0) {
@@ -1426,14 +1438,17 @@ cudaError_t trsv_block(iclblasHandle_t h, int uplo, int trans, int diag, int n, 
     if (!(smem_set.load() & bit)) {
         e = cudaFuncSetAttribute(trsv_block_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(BlockSmem<T>));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(trsv_block_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         smem_set.fetch_or(bit);
     }
-    // the cluster size as for strsv_tma_kernel: the largest for which every
-    // cluster of the launch is resident at once, else 8, else none
+    // the cluster size as for strsv_tma_kernel: the largest (up to the number
+    // of blocks) for which every cluster of the launch is resident at once,
+    // else 8, else none
     int cl = 1;
     if (nb > 1) {
-        for (int c = kMaxCluster; c >= 2 && cl == 1; --c) {
+        for (int c = std::min(nb, nb <= kBWide ? kBCluster : kMaxCluster); c >= 2 && cl == 1; --c) {
             const int cap = trsv_block_capacity<T>(h->device, c);
             if (cap > 0 && cap * c >= nb) cl = c;
         }
