@@ -40,3 +40,45 @@ def test_split_modes(handle, cuda, mode, m, n, k):
 def test_hgemm(handle, cuda, m, n, k):
     import torch
     check(handle, B.iclblasHgemm, m, n, k, 5e-4, torch.float16, torch)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("mode", list(BARS))
+@pytest.mark.parametrize("n", [192, 640, 1664])
+def test_back_to_back_products(handle, cuda, mode, n, captured):
+    """Each product reads what the launch before it wrote, with no host
+    synchronisation between them, live and replayed: the same bits as with one
+    after every call (the kernels overlap their prologues, not their reads)."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    X0, W = ((torch.rand(n, n, generator=gen, device="cuda") * 2 - 1) / 16 for _ in range(2))
+    steps = 6
+    X = [X0.clone()] + [torch.empty_like(X0) for _ in range(steps)]
+    want = [X0.clone()] + [torch.empty_like(X0) for _ in range(steps)]
+    handle.set_math_mode(mode)
+
+    def chain(bufs, sync):
+        for i in range(steps):
+            assert B.iclblasSgemm(handle, 0, 0, n, n, n, 1.0, W, n, bufs[i], n, 0.0, bufs[i + 1], n) == B.SUCCESS
+            if sync:
+                assert handle.synchronize() == B.SUCCESS
+
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    handle.set_stream(s)
+    with torch.cuda.stream(s):
+        chain(want, True)
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                chain(X, False)
+            for _ in range(3):
+                for t in X[1:]:
+                    t.fill_(float("nan"))
+                g.replay()
+        else:
+            chain(X, False)
+    s.synchronize()
+    assert handle.synchronize() == B.SUCCESS
+    for got, ref in zip(X, want):
+        assert torch.equal(got, ref)
