@@ -64,6 +64,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace iclb {
 namespace tc {
@@ -156,14 +157,6 @@ __device__ __forceinline__ unsigned long long global_ns()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-// Programmatic dependent launch: a split kernel lets the GEMM behind it start
-// (its CTAs set up barriers, TMEM and tensor maps as SMs come free), and the
-// GEMM touches global memory only once everything before it in the stream has
-// finished.  Without the launch attribute both are no-ops.  Measured: HGEMM
-// 25088 x 128 x 512 14.3 -> 12.4 us, STRSM 8192 x 4096 in 3xBF16 3993 -> 3887.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Bounded wait: false when 2 s passed or another role gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
@@ -1195,7 +1188,8 @@ __global__ void __launch_bounds__(256) split_real_kernel(const __grid_constant__
                                                          const __grid_constant__ SplitJob b, int two)
 {
     __shared__ float tile[64][65];
-    pdl_launch_dependents();
+    pdl_wait();
+    pdl_trigger();
     const bool sb = two && blockIdx.z;
     const SplitOut o = sb ? b.o : a.o;
     const float* S = (const float*)(sb ? b.S : a.S);
@@ -1292,7 +1286,8 @@ __global__ void __launch_bounds__(256) split_cplx_kernel(const __grid_constant__
                                                          const __grid_constant__ SplitJob b)
 {
     __shared__ float2 tile[64][65];
-    pdl_launch_dependents();
+    pdl_wait();
+    pdl_trigger();
     const bool sb = blockIdx.z != 0;
     const SplitOut o = sb ? b.o : a.o;
     const float2* S = (const float2*)(sb ? b.S : a.S);
@@ -1519,14 +1514,18 @@ void set_mode_params(Params& p, const ModeInfo& mi, long kext)
     }
 }
 
-// Both operands of a product, one launch.
+// Both operands of a product, one launch.  A chain split -> GEMM -> split
+// overlaps each kernel's start with the end of the one before it: STRSM
+// 8192 x 4096 in 3xBF16 3993 us with plain launches, 3887 with the GEMM
+// launched dependent, 3814 with the splits too.  The splits trigger the GEMM
+// behind them; the GEMM doesn't trigger the next split (3968: split blocks
+// then sit on SMs whose GEMM tiles are still running).
 cudaError_t run_split_pair(iclblasHandle_t h, bool cplx, const SplitJob& a, const SplitJob& b)
 {
     auto k_of = [&](const SplitJob& j) { return cplx ? (long)((j.K + 7) & ~7) : j.kw; };
     const dim3 grid((unsigned)ceil_div(std::max(k_of(a), k_of(b)), 64L), (unsigned)ceil_div(std::max(a.R, b.R), 64), 2);
-    if (cplx) split_cplx_kernel<<<grid, 256, 0, h->stream>>>(a, b);
-    else split_real_kernel<<<grid, 256, 0, h->stream>>>(a, b, 1);
-    return cudaGetLastError();
+    if (cplx) return pdl_launch(split_cplx_kernel, grid, 256, 0, h->stream, 1, a, b);
+    return pdl_launch(split_real_kernel, grid, 256, 0, h->stream, 1, a, b, 1);
 }
 
 }  // namespace
@@ -1630,24 +1629,9 @@ cudaError_t launch_engine(iclblasHandle_t h, const ModeInfo& mi, const Operand* 
         auto run2 = [&](auto kernel) -> cudaError_t {
             const KernelFacts f = kernel_facts(kernel, smem, true, h);
             if (f.status != cudaSuccess) return f.status;
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 2;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[1].val.programmaticStreamSerializationAllowed = 1;
-            cfg.blockDim = dim3(THREADS);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = h->stream;
-            cfg.attrs = attr;
-            cfg.numAttrs = 2;
             // as many pairs as can be resident at once (persistent), at most one per tile
-            cfg.gridDim = dim3(2 * std::min(pair_tiles, f.max_clusters));
-            const cudaError_t r = cudaLaunchKernelEx(&cfg, kernel, ma[0], ma[1], ma[2], mb[0], mb[1], mb[2], mc, p);
-            if (r != cudaSuccess) return r;
-            return cudaGetLastError();
+            return pdl_launch(kernel, dim3(2 * std::min(pair_tiles, f.max_clusters)), THREADS, smem, h->stream, 2, ma[0],
+                              ma[1], ma[2], mb[0], mb[1], mb[2], mc, p);
         };
         if (p.out_half) return run2(gemm_tc2_kernel<false, OUT_F16, true>);
         if (mi.tf32)
@@ -1661,18 +1645,8 @@ cudaError_t launch_engine(iclblasHandle_t h, const ModeInfo& mi, const Operand* 
     auto run = [&](auto kernel) -> cudaError_t {
         const KernelFacts f = kernel_facts(kernel, smem, false, h);
         if (f.status != cudaSuccess) return f.status;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = h->stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const cudaError_t r = cudaLaunchKernelEx(&cfg, kernel, ma[0], ma[1], ma[2], mb[0], mb[1], mb[2], mc, p);
-        return r != cudaSuccess ? r : cudaGetLastError();
+        return pdl_launch(kernel, dim3((unsigned)grid), THREADS, smem, h->stream, 1, ma[0], ma[1], ma[2], mb[0], mb[1],
+                          mb[2], mc, p);
     };
     // instantiations: TF32 and HGEMM always single-chunk; the BF16 modes
     // single-chunk when the whole K fits one chunk (K <= 64 * chunk)
@@ -1865,8 +1839,7 @@ cudaError_t split_planes_tc(iclblasHandle_t h, const float* S, int R, int K, lon
     for (int l = 0; l < dst.nlev; ++l) o.plane[l] = (char*)dst.plane[l] + (row0 * dst.pitch + k0) * esize;
     const SplitJob j = real_job(S, R, K, rs, ks, o, kw, tri, unit, szs, dzs);
     const dim3 grid((unsigned)ceil_div(kw, 64L), (unsigned)ceil_div(R, 64), (unsigned)nz);
-    split_real_kernel<<<grid, 256, 0, h->stream>>>(j, j, 0);
-    return cudaGetLastError();
+    return pdl_launch(split_real_kernel, grid, 256, 0, h->stream, 1, j, j, 0);
 }
 
 template cudaError_t gemm_tc<float>(iclblasHandle_t, int, int, int, int, int, float, const float*, int, const float*,
