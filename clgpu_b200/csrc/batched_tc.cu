@@ -981,8 +981,8 @@ struct MmaArgs {
 };
 
 // A solve is a chain of some 30 of these launches, each a few tiles an SM: a
-// CTA of the next launch sets up as soon as the SM's CTA of this one ends (64
-// instances up to 2048 columns in 6xBF16: 2555 -> 2468 us).
+// CTA of the next launch sets up as soon as the SM's CTA of this one ends (512
+// instances of order up to 1024, forward and adjoint in 6xBF16: 2555 -> 2468 us).
 template <bool TF32>
 cudaError_t launch_mma(const MmaLaunch& p, int kind, int grid, cudaStream_t st)
 {

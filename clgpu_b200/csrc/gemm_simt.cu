@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace iclb {
 namespace {
@@ -205,6 +206,11 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     constexpr int WX = TX / 8;  // warps along n
     const int ty = (warp / WX) * 4 + lane / 8, tx = (warp % WX) * 8 + lane % 8;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    pdl_wait();
+    PDL_FRESH(A);
+    PDL_FRESH(B);
+    PDL_FRESH(C);
+    pdl_trigger();
     // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed;
     // tiles wholly outside it have no work
     if ((tri == 1 && m0 + BM - 1 < n0) || (tri == 2 && m0 > n0 + BN - 1)) return;
@@ -342,8 +348,8 @@ cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alp
         }
     }
     dim3 grid(ceil_div(m, BM), ceil_div(n, BN));
-    kern<<<grid, CF::NT, CF::SMEM, h->stream>>>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri);
-    return cudaGetLastError();
+    return pdl_launch(kern, grid, CF::NT, CF::SMEM, h->stream, 1,
+                      ta, tb, m, n, k, alpha, A, (long)lda, B, (long)ldb, beta, C, (long)ldc, tri);
 }
 
 }  // namespace

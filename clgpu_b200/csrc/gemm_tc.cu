@@ -1213,7 +1213,7 @@ __global__ void __launch_bounds__(256) split_real_kernel(const __grid_constant__
         for (int u = 0; u < 4; ++u) {
             const int f = (t % 16) * 4, g = t / 16 + 16 * u;
             float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (g0 + g < ng) w = __ldg(reinterpret_cast<const float4*>(S + (long)(g0 + g) * gs + f0 + f));
+            if (g0 + g < ng) w = *reinterpret_cast<const float4*>(S + (long)(g0 + g) * gs + f0 + f);
             v[4 * u] = w.x;
             v[4 * u + 1] = w.y;
             v[4 * u + 2] = w.z;
@@ -1228,7 +1228,7 @@ __global__ void __launch_bounds__(256) split_real_kernel(const __grid_constant__
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const int f = t % 64, g = t / 64 + 4 * u;
-            v[u] = (f0 + f < nf && g0 + g < ng) ? __ldg(S + (long)(g0 + g) * gs + f0 + f) : 0.f;
+            v[u] = (f0 + f < nf && g0 + g < ng) ? S[(long)(g0 + g) * gs + f0 + f] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
@@ -1304,7 +1304,7 @@ __global__ void __launch_bounds__(256) split_cplx_kernel(const __grid_constant__
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
         const int g = t / 64 + 4 * u;
-        v[u] = (f0 + f < nf && g0 + g < ng) ? __ldg(S + (long)(g0 + g) * gs + f0 + f) : make_float2(0.f, 0.f);
+        v[u] = (f0 + f < nf && g0 + g < ng) ? S[(long)(g0 + g) * gs + f0 + f] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < 16; ++u) {

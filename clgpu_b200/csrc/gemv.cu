@@ -9,9 +9,13 @@
 //         last block of each row tile adds them in slice order (deterministic)
 //         and applies alpha/beta;
 //   op T/C: one warp per column (a column is contiguous), 128-bit loads down
-//         the column, shuffle-tree sum.
+//         the column, shuffle-tree sum; one block per column where tall
+//         columns allow only scalar loads.
+// Operands without 16-byte alignment are read by scalar loads, a warp's rows
+// consecutive, several columns' loads issued together.
 // beta == 0 means y is written without being read (Sgemv_naive.cl:34,54).
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace iclb {
 namespace {
@@ -57,6 +61,14 @@ __device__ __forceinline__ float ldg_of(const float* p) { return __ldg(p); }
 __device__ __forceinline__ cfloat ldg_of(const cfloat* p)
 {
     const float2 v = __ldg((const float2*)p);
+    return cfloat{v.x, v.y};
+}
+// for kernels whose launch may start before the one ahead of it has ended:
+// their inputs aren't constant data
+__device__ __forceinline__ float ld_of(const float* p) { return *p; }
+__device__ __forceinline__ cfloat ld_of(const cfloat* p)
+{
+    const float2 v = *(const float2*)p;
     return cfloat{v.x, v.y};
 }
 // another block's partial sum, past this SM's L1
@@ -184,6 +196,12 @@ __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T a
                                                                T* __restrict__ y, long incy, int cps,
                                                                T* __restrict__ partial, unsigned* counters)
 {
+    pdl_wait();
+    PDL_FRESH(A);
+    PDL_FRESH(x);
+    PDL_FRESH(y);
+    PDL_FRESH(partial);
+    pdl_trigger();
     constexpr int R = 16 / sizeof(T);
     constexpr int RS = VEC ? 1 : kNThreads;  // rows of a thread: row0 + r * RS
     constexpr int XC = 256;  // x values staged per chunk
@@ -249,7 +267,7 @@ __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T a
                     for (int u = 0; u < 8; ++u)
 #pragma unroll
                         for (int r = 0; r < R; ++r)
-                            v[u][r] = row0 + r * RS < m ? ldg_of(Ac + (long)(c + u) * lda + r * RS) : zero_of(T());
+                            v[u][r] = row0 + r * RS < m ? ld_of(Ac + (long)(c + u) * lda + r * RS) : zero_of(T());
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
 #pragma unroll
@@ -416,6 +434,11 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha,
                                                                  const T* __restrict__ x, long incx, T beta,
                                                                  T* __restrict__ y, long incy, int seg)
 {
+    pdl_wait();
+    PDL_FRESH(A);
+    PDL_FRESH(x);
+    PDL_FRESH(y);
+    pdl_trigger();
     constexpr int W = kTThreads / 32, U = 8;
     __shared__ T part[W];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -428,8 +451,8 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha,
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const bool in = r + u * 32 < r1;
-            v[u] = in ? ldg_of(Ac + r + u * 32) : zero_of(T());
-            xv[u] = in ? ldg_of(x + (long)(r + u * 32) * incx) : zero_of(T());
+            v[u] = in ? ld_of(Ac + r + u * 32) : zero_of(T());
+            xv[u] = in ? ld_of(x + (long)(r + u * 32) * incx) : zero_of(T());
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -481,8 +504,8 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
         }
         dim3 grid(rt, splits);
 #define LAUNCH(V, G)                                                                                       \
-    gemv_n_kernel<T, V, G><<<grid, kNThreads * G, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, \
-                                                                  cps, partial, h->ws.counters)
+    return pdl_launch(gemv_n_kernel<T, V, G>, dim3(grid), kNThreads * G, 0, h->stream, dependent((long)m * n),   \
+                      m, n, alpha, A, lda, x, incx, beta, y, incy, cps, partial, h->ws.counters)
         if (small) { if (vec) LAUNCH(true, 4); else LAUNCH(false, 4); }
         else if (!vec) LAUNCH(false, 1);
         else
@@ -497,10 +520,11 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     if (!vec && m >= 1024 && n <= 6000) {
         const int seg = ceil_div(ceil_div(m, kTThreads / 32), 32) * 32;
         if (conj)
-            gemv_t_block_kernel<T, true><<<n, kTThreads, 0, h->stream>>>(m, alpha, A, lda, x, incx, beta, y, incy, seg);
+            return pdl_launch(gemv_t_block_kernel<T, true>, dim3(n), kTThreads, 0, h->stream, dependent((long)m * n),
+                              m, alpha, A, lda, x, incx, beta, y, incy, seg);
         else
-            gemv_t_block_kernel<T, false><<<n, kTThreads, 0, h->stream>>>(m, alpha, A, lda, x, incx, beta, y, incy, seg);
-        return cudaGetLastError();
+            return pdl_launch(gemv_t_block_kernel<T, false>, dim3(n), kTThreads, 0, h->stream, dependent((long)m * n),
+                              m, alpha, A, lda, x, incx, beta, y, incy, seg);
     }
     const int warps_target = target * (kTThreads / 32);
     int S = 1;

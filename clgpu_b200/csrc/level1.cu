@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace iclb {
 namespace {
@@ -56,9 +57,16 @@ __host__ RedShape red_shape(iclblasHandle_t h, long n, long units, int per_sm)
 // computes this_y += alpha*this_x, Saxpy_noinc.cl).  The n % 4 last elements
 // go to the first threads of the same launch: a launch of their own costs a
 // short vector about 3 us, as much as the whole of its other work.
+template <bool DEP>
 __global__ void __launch_bounds__(kThreads) saxpy_vec(long n, float alpha, const float4* __restrict__ x,
                                                       float4* __restrict__ y)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(y);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x, n4 = n >> 2;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid < (n & 3)) {
@@ -76,16 +84,29 @@ __global__ void __launch_bounds__(kThreads) saxpy_vec(long n, float alpha, const
     }
 }
 
+template <bool DEP>
 __global__ void __launch_bounds__(kThreads) saxpy_strided(long n, float alpha, const float* __restrict__ x, long incx,
                                                           float* __restrict__ y, long incy)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(y);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
         y[i * incy] = fmaf(alpha, x[i * incx], y[i * incy]);
 }
 
+template <bool DEP>
 __global__ void __launch_bounds__(kThreads) sscal_vec(long n, float alpha, float4* __restrict__ x)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x, n4 = n >> 2;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (tid < (n & 3)) ((float*)(x + n4))[tid] *= alpha;
@@ -96,8 +117,14 @@ __global__ void __launch_bounds__(kThreads) sscal_vec(long n, float alpha, float
     }
 }
 
+template <bool DEP>
 __global__ void __launch_bounds__(kThreads) sscal_strided(long n, float alpha, float* __restrict__ x, long incx)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i * incx] *= alpha;
 }
@@ -120,10 +147,16 @@ __device__ __forceinline__ cfloat cmul_d(cfloat x, cfloat a)
     return cfloat{(float)re, (float)im};
 }
 
-template <bool VEC>
+template <bool VEC, bool DEP>
 __global__ void __launch_bounds__(kThreads) caxpy_kernel(long n, cfloat alpha, const cfloat* __restrict__ x, long incx,
                                                          cfloat* __restrict__ y, long incy)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(y);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x;
     if (VEC) {
         const float4* x4 = (const float4*)x;
@@ -142,9 +175,14 @@ __global__ void __launch_bounds__(kThreads) caxpy_kernel(long n, cfloat alpha, c
     }
 }
 
-template <bool VEC>
+template <bool VEC, bool DEP>
 __global__ void __launch_bounds__(kThreads) cscal_kernel(long n, cfloat alpha, cfloat* __restrict__ x, long incx)
 {
+    if (DEP) {
+        pdl_wait();
+        PDL_FRESH(x);
+        pdl_trigger();
+    }
     const long stride = (long)gridDim.x * blockDim.x;
     if (VEC) {
         float4* x4 = (float4*)x;
@@ -177,6 +215,13 @@ __global__ void __launch_bounds__(NT) sreduce_kernel(long n, const float* __rest
                                                            double* __restrict__ partials, unsigned* counter,
                                                            float* __restrict__ result)
 {
+    if (NT == 1024) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(y);
+        PDL_FRESH(partials);
+        pdl_trigger();
+    }
     __shared__ double sh[32];
     const long stride = (long)gridDim.x * blockDim.x;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -251,6 +296,12 @@ __global__ void __launch_bounds__(NT) creduce_kernel(long n, const cfloat* __res
                                                            double* __restrict__ partials, unsigned* counter,
                                                            float* __restrict__ result)
 {
+    if (NT == 1024) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(partials);
+        pdl_trigger();
+    }
     __shared__ double sh[32];
     const long stride = (long)gridDim.x * blockDim.x;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -304,6 +355,13 @@ __global__ void __launch_bounds__(NT) cdot_kernel(long n, const cfloat* __restri
                                                         double* __restrict__ partials, unsigned* counter,
                                                         cfloat* __restrict__ result)
 {
+    if (NT == 1024) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(y);
+        PDL_FRESH(partials);
+        pdl_trigger();
+    }
     __shared__ double sh[32];
     const long stride = (long)gridDim.x * blockDim.x;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -426,6 +484,12 @@ __global__ void __launch_bounds__(NT) iamax_kernel(long n, const T* __restrict__
                                                          Cand* __restrict__ partials, unsigned* counter,
                                                          int* __restrict__ result)
 {
+    if (NT == 1024) {
+        pdl_wait();
+        PDL_FRESH(x);
+        PDL_FRESH(partials);
+        pdl_trigger();
+    }
     __shared__ Cand sh[32];
     const long stride = (long)gridDim.x * blockDim.x;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -490,9 +554,11 @@ __global__ void __launch_bounds__(NT) iamax_kernel(long n, const T* __restrict__
 cudaError_t saxpy(iclblasHandle_t h, int n, float alpha, const float* x, int incx, float* y, int incy)
 {
     if (incx == 1 && incy == 1 && aligned16(x) && aligned16(y)) {
-        saxpy_vec<<<l1_grid(h, n >> 2, 4), kThreads, 0, h->stream>>>(n, alpha, (const float4*)x, (float4*)y);
+        return pdl_launch(dependent(n) ? saxpy_vec<true> : saxpy_vec<false>, dim3(l1_grid(h, n >> 2, 4)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, (const float4*)x, (float4*)y);
     } else {
-        saxpy_strided<<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx, y, incy);
+        return pdl_launch(dependent(n) ? saxpy_strided<true> : saxpy_strided<false>, dim3(l1_grid(h, n)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, incx, y, incy);
     }
     return cudaGetLastError();
 }
@@ -500,9 +566,11 @@ cudaError_t saxpy(iclblasHandle_t h, int n, float alpha, const float* x, int inc
 cudaError_t sscal(iclblasHandle_t h, int n, float alpha, float* x, int incx)
 {
     if (incx == 1 && aligned16(x)) {
-        sscal_vec<<<l1_grid(h, n >> 2), kThreads, 0, h->stream>>>(n, alpha, (float4*)x);
+        return pdl_launch(dependent(n) ? sscal_vec<true> : sscal_vec<false>, dim3(l1_grid(h, n >> 2)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, (float4*)x);
     } else {
-        sscal_strided<<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx);
+        return pdl_launch(dependent(n) ? sscal_strided<true> : sscal_strided<false>, dim3(l1_grid(h, n)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, incx);
     }
     return cudaGetLastError();
 }
@@ -510,19 +578,25 @@ cudaError_t sscal(iclblasHandle_t h, int n, float alpha, float* x, int incx)
 cudaError_t caxpy(iclblasHandle_t h, int n, cfloat alpha, const cfloat* x, int incx, cfloat* y, int incy)
 {
     if (incx == 1 && incy == 1 && aligned16(x) && aligned16(y))
-        caxpy_kernel<true><<<l1_grid(h, (long)n / 2 + 1), kThreads, 0, h->stream>>>(n, alpha, x, 1, y, 1);
+        return pdl_launch(dependent(n) ? caxpy_kernel<true, true> : caxpy_kernel<true, false>,
+                          dim3(l1_grid(h, (long)n / 2 + 1)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, 1, y, 1);
     else
-        caxpy_kernel<false><<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx, y, incy);
-    return cudaGetLastError();
+        return pdl_launch(dependent(n) ? caxpy_kernel<false, true> : caxpy_kernel<false, false>,
+                          dim3(l1_grid(h, n)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, incx, y, incy);
 }
 
 cudaError_t cscal(iclblasHandle_t h, int n, cfloat alpha, cfloat* x, int incx)
 {
     if (incx == 1 && aligned16(x))
-        cscal_kernel<true><<<l1_grid(h, (long)n / 2 + 1), kThreads, 0, h->stream>>>(n, alpha, x, 1);
+        return pdl_launch(dependent(n) ? cscal_kernel<true, true> : cscal_kernel<true, false>,
+                          dim3(l1_grid(h, (long)n / 2 + 1)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, 1);
     else
-        cscal_kernel<false><<<l1_grid(h, n), kThreads, 0, h->stream>>>(n, alpha, x, incx);
-    return cudaGetLastError();
+        return pdl_launch(dependent(n) ? cscal_kernel<false, true> : cscal_kernel<false, false>,
+                          dim3(l1_grid(h, n)), kThreads, 0,
+                          h->stream, dependent(n), n, alpha, x, incx);
 }
 
 cudaError_t sreduce(iclblasHandle_t h, Red op, int n, const float* x, int incx, const float* y, int incy,
@@ -537,9 +611,11 @@ cudaError_t sreduce(iclblasHandle_t h, Red op, int n, const float* x, int incx, 
 #define LAUNCH(OP, V)                                                                                            \
     do {                                                                                                         \
         if (g.grid > 1)                                                                                          \
-            sreduce_kernel<OP, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+            return pdl_launch(sreduce_kernel<OP, V>, dim3(g.grid), g.threads, 0, h->stream, 0,        \
+                              n, x, incx, y, incy, partials, ctr, result);                                       \
         else                                                                                                     \
-            sreduce_kernel<OP, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+            return pdl_launch(sreduce_kernel<OP, V, 1024>, dim3(1), g.threads, 0, h->stream, 1,       \
+                              n, x, incx, y, incy, partials, ctr, result);                                       \
     } while (0)
     switch (op) {
     case Red::Dot: if (vec) LAUNCH(Red::Dot, true); else LAUNCH(Red::Dot, false); break;
@@ -634,23 +710,21 @@ cudaError_t sdot_noalloc(iclblasHandle_t h, int n, const float* x, int incx, con
     if (e != cudaSuccess) return e;
     if (g.grid == 1) {
         if (vec)
-            sreduce_kernel<Red::Dot, true, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                                 &sc->counter, result);
+            return pdl_launch(sreduce_kernel<Red::Dot, true, 1024>, dim3(1), g.threads, 0, h->stream, 1,
+                              n, x, incx, y, incy, sc->partials, &sc->counter, result);
         else
-            sreduce_kernel<Red::Dot, false, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                                  &sc->counter, result);
-        return cudaGetLastError();
+            return pdl_launch(sreduce_kernel<Red::Dot, false, 1024>, dim3(1), g.threads, 0, h->stream, 1,
+                              n, x, incx, y, incy, sc->partials, &sc->counter, result);
     }
     // the array keeps the previous call's contents: the ticket must start at 0
     e = cudaMemsetAsync(&sc->counter, 0, sizeof(unsigned), h->stream);
     if (e != cudaSuccess) return e;
     if (vec)
-        sreduce_kernel<Red::Dot, true><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                            &sc->counter, result);
+        return pdl_launch(sreduce_kernel<Red::Dot, true>, dim3(g.grid), g.threads, 0, h->stream, 0,
+                              n, x, incx, y, incy, sc->partials, &sc->counter, result);
     else
-        sreduce_kernel<Red::Dot, false><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, sc->partials,
-                                                                             &sc->counter, result);
-    return cudaGetLastError();
+        return pdl_launch(sreduce_kernel<Red::Dot, false>, dim3(g.grid), g.threads, 0, h->stream, 0,
+                              n, x, incx, y, incy, sc->partials, &sc->counter, result);
 }
 
 cudaError_t creduce_real(iclblasHandle_t h, Red op, int n, const cfloat* x, int incx, float* result)
@@ -664,9 +738,11 @@ cudaError_t creduce_real(iclblasHandle_t h, Red op, int n, const cfloat* x, int 
 #define LAUNCH(OP, V)                                                                                        \
     do {                                                                                                     \
         if (g.grid > 1)                                                                                      \
-            creduce_kernel<OP, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);   \
+            return pdl_launch(creduce_kernel<OP, V>, dim3(g.grid), g.threads, 0, h->stream, 0,        \
+                              n, x, incx, partials, ctr, result);                                                \
         else                                                                                                 \
-            creduce_kernel<OP, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);  \
+            return pdl_launch(creduce_kernel<OP, V, 1024>, dim3(1), g.threads, 0, h->stream, 1,       \
+                              n, x, incx, partials, ctr, result);                                                \
     } while (0)
     if (op == Red::Asum) { if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false); }
     else { if (vec) LAUNCH(Red::Nrm2, true); else LAUNCH(Red::Nrm2, false); }
@@ -686,9 +762,11 @@ cudaError_t cdot(iclblasHandle_t h, bool conj, int n, const cfloat* x, int incx,
 #define LAUNCH(C, V)                                                                                           \
     do {                                                                                                       \
         if (g.grid > 1)                                                                                        \
-            cdot_kernel<C, V><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+            return pdl_launch(cdot_kernel<C, V>, dim3(g.grid), g.threads, 0, h->stream, 0,            \
+                              n, x, incx, y, incy, partials, ctr, result);                                       \
         else                                                                                                   \
-            cdot_kernel<C, V, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, y, incy, partials, ctr, result); \
+            return pdl_launch(cdot_kernel<C, V, 1024>, dim3(1), g.threads, 0, h->stream, 1,           \
+                              n, x, incx, y, incy, partials, ctr, result);                                       \
     } while (0)
     if (conj) { if (vec) LAUNCH(true, true); else LAUNCH(true, false); }
     else { if (vec) LAUNCH(false, true); else LAUNCH(false, false); }
@@ -709,9 +787,11 @@ cudaError_t iamax_impl(iclblasHandle_t h, int n, const T* x, int incx, int* resu
 #define LAUNCH(V)                                                                                                \
     do {                                                                                                         \
         if (g.grid > 1)                                                                                          \
-            iamax_kernel<T, V, MIN><<<g.grid, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);     \
+            return pdl_launch(iamax_kernel<T, V, MIN>, dim3(g.grid), g.threads, 0, h->stream, 0,      \
+                              n, x, incx, partials, ctr, result);                                                \
         else                                                                                                     \
-            iamax_kernel<T, V, MIN, 1024><<<1, g.threads, 0, h->stream>>>(n, x, incx, partials, ctr, result);    \
+            return pdl_launch(iamax_kernel<T, V, MIN, 1024>, dim3(1), g.threads, 0, h->stream, 1,     \
+                              n, x, incx, partials, ctr, result);                                                \
     } while (0)
     if (vec) LAUNCH(true); else LAUNCH(false);
 #undef LAUNCH
