@@ -121,17 +121,17 @@ ICLBLAS_API iclblasStatus_t iclblasSdot(iclblasHandle_t handle, int n, float* x,
  *     (INVALID_VALUE otherwise: staging host data would allocate, and a
  *     kernel cannot read another GPU's memory); the call is asynchronous on the
  *     handle's stream and its result equals iclblasSdot's;
- *   - a call needing more than 4096 partials -- one per block, with
- *     min(ceil(n/1024), 8 x SM count) blocks for unit-stride 16-byte-aligned
- *     operands and min(ceil(n/256), 8 x SM count) otherwise -- returns
- *     NOT_SUPPORTED;
+ *   - a call needing more than 4096 partials -- one per block, with one
+ *     block up to n = 16384, else min(ceil(n/1024), 8 x SM count) blocks for
+ *     unit-stride 16-byte-aligned operands and min(ceil(n/256), 8 x SM count)
+ *     otherwise -- returns NOT_SUPPORTED;
  *   - the first call on each device looks up the array's device address
  *     (cudaGetSymbolAddress) in the CUDA runtime's context of that device
  *     (its primary context; a context made current through the driver API is
  *     not supported), and looks it up again once that context has changed
  *     (after cudaDeviceReset); make that first call before any stream capture;
  *   - all calls share the one array, which keeps the previous call's
- *     contents (the counter is cleared at the start of each call): calls that
+ *     contents (a call of several blocks clears the counter first): calls that
  *     overlap on the GPU (other streams or handles at the same time) race and
  *     give wrong results, so serialize them. */
 ICLBLAS_API iclblasStatus_t iclblasSdotNoAlloc(iclblasHandle_t handle, int n, const float* x, int incx, const float* y,

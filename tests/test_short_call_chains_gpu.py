@@ -1,0 +1,58 @@
+"""Chains of short calls, each reading what the launch before it wrote, with no
+host synchronisation between them: on the legacy stream, on a stream of its own,
+and replayed from a CUDA graph, over aligned, odd and strided operands.  The
+same bits as with a synchronisation after every call are expected: launches may
+start early, but read only finished results."""
+import pytest
+
+from clgpu_b200 import iclblas as B
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("where", ["legacy", "stream", "graph"])
+@pytest.mark.parametrize("n,lda,inc", [(64, 64, 1), (301, 303, 1), (1536, 1537, 1), (1100, 1101, 2), (1024, 1024, 1)])
+def test_chain(handle, cuda, n, lda, inc, where):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n + inc)
+    A = ((torch.rand(n, lda, generator=gen, device="cuda") * 2 - 1) / n ** 0.5).contiguous()
+    v0 = torch.rand(n * inc, generator=gen, device="cuda")
+    handle.set_math_mode(0)
+    steps = 8
+
+    def chain(v, w, r, M, sync):
+        def done(status):
+            assert status == B.SUCCESS
+            if sync:
+                assert handle.synchronize() == B.SUCCESS
+        for i in range(steps):
+            done(B.iclblasSgemv(handle, i % 2, n, n, 1.0, A, lda, v, inc, 0.0, w, inc))
+            done(B.iclblasSaxpy(handle, n, 0.5, v, inc, w, inc))
+            done(B.iclblasSscal(handle, n, 0.75, w, inc))
+            done(B.iclblasSdot(handle, n, v, inc, w, inc, r[i:]))
+            done(B.iclblasSgemm(handle, 0, 0, n, 1, n, 1.0, A, lda, w, n, 0.0, M[i], n))
+            v, w = w, v
+
+    def bufs():
+        return v0.clone(), torch.zeros_like(v0), torch.zeros(steps, device="cuda"), torch.zeros(steps, n, device="cuda")
+
+    want, got = bufs(), bufs()
+    s = torch.cuda.current_stream() if where == "legacy" else torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle.set_stream(s)
+    with torch.cuda.stream(s):
+        chain(*want, True)
+        if where == "graph":
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                chain(*got, False)
+            for _ in range(3):
+                got[0].copy_(v0)
+                for t in got[1:]:
+                    t.zero_()
+                g.replay()
+        else:
+            chain(*got, False)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
