@@ -56,3 +56,43 @@ def test_chain(handle, cuda, n, lda, inc, where):
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("mode", [B.MATH_PLAIN_FP32, B.MATH_BF16X3])
+def test_after_copies_and_fills_in_a_graph(handle, cuda, mode):
+    """Captured calls behind copy and fill nodes, and a solve that forks onto
+    the handle's second stream."""
+    import torch
+    n, nrhs = 1536, 1024
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.rand(n, n, generator=gen, device="cuda") / n
+    A.diagonal().add_(1.0)
+    X0 = torch.rand(nrhs, n, generator=gen, device="cuda")
+    handle.set_math_mode(mode)
+
+    def run(X, C):
+        X.copy_(X0)
+        assert B.iclblasStrsm(handle, 0, 1, 0, 0, n, nrhs, 1.0, A, n, X, n) == B.SUCCESS
+        C.zero_()
+        assert B.iclblasSgemm(handle, 0, 0, n, nrhs, n, 1.0, A, n, X, n, 1.0, C, n) == B.SUCCESS
+        X0b = X.clone()
+        assert B.iclblasSscal(handle, X0b.numel(), 0.5, X0b, 1) == B.SUCCESS
+        C.add_(X0b)
+
+    want, got = [[torch.empty_like(X0) for _ in range(2)] for _ in range(2)]
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle.set_stream(s)
+    with torch.cuda.stream(s):
+        run(*want)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            run(*got)
+        for _ in range(2):
+            for t in got:
+                t.fill_(float("nan"))
+            g.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
