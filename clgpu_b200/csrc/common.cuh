@@ -80,6 +80,10 @@ __device__ __forceinline__ bool last_block_of(unsigned* counter, unsigned total)
     return is_last;
 }
 
+// Complex operands are pairs of floats: any multiple of 4 is a legal address,
+// and only those at a multiple of 8 may be read an element at a time.
+inline bool aligned8(const void* p) { return ((uintptr_t)p & 7u) == 0; }
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace iclb

@@ -50,7 +50,8 @@ cudaError_t cgemm(iclblasHandle_t h, int ta, int tb, int m, int n, int k, cfloat
                   const cfloat* B, int ldb, cfloat beta, cfloat* C, int ldc)
 {
     if (m == 0 || n == 0) return cudaSuccess;
-    if (h->math != ICLBLAS_MATH_PLAIN_FP32 && k > 0)
+    // (the tensor-core epilogue moves whole elements of C)
+    if (h->math != ICLBLAS_MATH_PLAIN_FP32 && k > 0 && aligned8(C))
         return tc::gemm_tc<cfloat>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0);
     return cgemm_simt(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }

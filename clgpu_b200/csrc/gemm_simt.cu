@@ -127,6 +127,17 @@ __device__ __forceinline__ void cp_async_elem(cfloat* dst, const cfloat* src, bo
                  "r"(in ? 8 : 0)
                  : "memory");
 }
+// HALF: a complex element as its two floats (operands at 4 modulo 8)
+template <bool HALF, class T>
+__device__ __forceinline__ void cp_async_from(T* dst, const T* src, bool in)
+{
+    if constexpr (HALF) {
+        cp_async_elem(&dst->re, &src->re, in);
+        cp_async_elem(&dst->im, &src->im, in);
+    } else {
+        cp_async_elem(dst, src, in);
+    }
+}
 
 // Threads: (BM/TM) x (BN/TN).  Each thread owns TM x TN outputs in runs of VA
 // rows and VB columns (16 bytes, or all it has) spread evenly over the tile,
@@ -153,7 +164,7 @@ struct Cfg {
 
 // Copies of one operand's BX x BK tile into [kk][i] (pitch PX).  CONTIG_K:
 // element (i, kk) at p[i*ld + kk], else at p[kk*ld + i].
-template <class T, int BX, int BK, int NT, int PX>
+template <class T, int BX, int BK, int NT, int PX, bool HALF>
 struct TileCopy {
     static constexpr int PER = BX * BK / NT;
     const T* base;   // first element this thread copies, at k = 0
@@ -176,7 +187,7 @@ struct TileCopy {
             for (int q = 0; q < PER; ++q) {
                 const int kk = 8 * (q % KH), i = (q / KH) * RS;
                 const bool in = i0 + i < rows && k0 + kk0 + kk < k;
-                cp_async_elem(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)i * ld + kk : base, in);
+                cp_async_from<HALF>(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)i * ld + kk : base, in);
             }
         } else {
             constexpr int KS = NT >= BX ? NT / BX : 1, IP = NT >= BX ? 1 : BX / NT;   // k per pass; row passes
@@ -185,13 +196,13 @@ struct TileCopy {
             for (int q = 0; q < PER; ++q) {
                 const int kk = (q / IP) * KS, i = (q % IP) * NT;
                 const bool in = i0 + i < rows && k0 + kk0 + kk < k;
-                cp_async_elem(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)kk * ld + i : base, in);
+                cp_async_from<HALF>(dst + (kk0 + kk) * PX + i0 + i, in ? src + (long)kk * ld + i : base, in);
             }
         }
     }
 };
 
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB>
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF>
 __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     gemm_simt_kernel(int ta, int tb, int m, int n, int k, T alpha, const T* __restrict__ A, long lda,
                      const T* __restrict__ B, long ldb, T beta, T* __restrict__ C, long ldc, int tri)
@@ -215,8 +226,8 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     // tiles wholly outside it have no work
     if ((tri == 1 && m0 + BM - 1 < n0) || (tri == 2 && m0 > n0 + BN - 1)) return;
     const bool a_conj = ta == ICLBLAS_OP_C, b_conj = tb == ICLBLAS_OP_C;
-    const TileCopy<T, BM, BK, NT, PA> ca(A, lda, ta != ICLBLAS_OP_N, m0, m);
-    const TileCopy<T, BN, BK, NT, PB> cb(B, ldb, tb == ICLBLAS_OP_N, n0, n);
+    const TileCopy<T, BM, BK, NT, PA, HALF> ca(A, lda, ta != ICLBLAS_OP_N, m0, m);
+    const TileCopy<T, BN, BK, NT, PB, HALF> cb(B, ldb, tb == ICLBLAS_OP_N, n0, n);
 
     // float: accumulators in pairs along the longer dimension of the thread's
     // outputs (fewer values of the other operand to duplicate)
@@ -331,12 +342,12 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     }
 }
 
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB>
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF = false>
 cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alpha, const T* A, int lda, const T* B,
                    int ldb, T beta, T* C, int ldc, int tri)
 {
     using CF = Cfg<T, BM, BN, BK, TM, TN, ST>;
-    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB>;
+    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB, HALF>;
     if (CF::SMEM > 48 * 1024) {
         // the attribute belongs to the current device's copy of the kernel
         static std::atomic<unsigned long long> smem_set{0};
@@ -411,7 +422,12 @@ cudaError_t cgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, c
                        const cfloat* B, int ldb, cfloat beta, cfloat* C, int ldc)
 {
 #define LAUNCH(...) launch<cfloat, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0)
-    switch (pick_tile(kCplxTiles, h->sm_count, m, n, false)) {
+    const int tile = pick_tile(kCplxTiles, h->sm_count, m, n, false);
+    if (!aligned8(A) || !aligned8(B)) {
+        // two copies an element: the small tile is not worth a third of these
+        return tile == 0 ? LAUNCH(64, 64, 8, 8, 4, 4, 3, true) : LAUNCH(32, 32, 16, 4, 2, 3, 4, true);
+    }
+    switch (tile) {
     case 0:
         // 4096 x 4096 x 2048 (28 tiles an SM): 8 x 8 outputs a thread 6226 us,
         // 8 x 4 6653; 2048^3 (7): 8 x 4 1684 us, 8 x 8 slower than 1716

@@ -1140,7 +1140,7 @@ struct SplitJob {
     long kw;             // K values written per row (real)
     int tri, unit;       // real
     long szs, dzs;       // real, several equal operands
-    int vin, vout;       // real
+    int vin, vout;       // vin: S takes vector loads (real: 16 bytes, complex: an element); vout: real
     int mode, conj;      // complex
 };
 
@@ -1290,7 +1290,8 @@ __global__ void __launch_bounds__(256) split_cplx_kernel(const __grid_constant__
     pdl_trigger();
     const bool sb = blockIdx.z != 0;
     const SplitOut o = sb ? b.o : a.o;
-    const float2* S = (const float2*)(sb ? b.S : a.S);
+    const float* S = (const float*)(sb ? b.S : a.S);
+    const int vin = sb ? b.vin : a.vin;
     const int R = sb ? b.R : a.R, K = sb ? b.K : a.K, Kp = (K + 7) & ~7;
     const long rs = sb ? b.rs : a.rs, ks = sb ? b.ks : a.ks;
     const bool conj = (sb ? b.conj : a.conj) != 0, amode = (sb ? b.mode : a.mode) == kCplxA;
@@ -1304,7 +1305,9 @@ __global__ void __launch_bounds__(256) split_cplx_kernel(const __grid_constant__
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
         const int g = t / 64 + 4 * u;
-        v[u] = (f0 + f < nf && g0 + g < ng) ? S[(long)(g0 + g) * gs + f0 + f] : make_float2(0.f, 0.f);
+        const float* e = S + 2 * ((long)(g0 + g) * gs + f0 + f);
+        v[u] = make_float2(0.f, 0.f);
+        if (f0 + f < nf && g0 + g < ng) v[u] = vin ? *(const float2*)e : make_float2(e[0], e[1]);
     }
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
@@ -1695,6 +1698,10 @@ cudaError_t gemm_tc(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T al
     // B: L[r=n][k] = op(B)[k][n] ; op N: S[k + n*ldb] ; op T/C: S[n + k*ldb]
     SplitJob ja = real_job((const float*)A, m, k, at ? lda : 1, at ? 1 : lda, oa, kpad);
     SplitJob jb = real_job((const float*)B, n, k, bt ? 1 : ldb, bt ? ldb : 1, ob, kpad);
+    if (cplx) {
+        ja.vin = aligned8(A);
+        jb.vin = aligned8(B);
+    }
     ja.mode = kCplxA;
     jb.mode = kCplxB;
     ja.conj = ta == ICLBLAS_OP_C;

@@ -58,16 +58,17 @@ __device__ __forceinline__ cfloat axpby(cfloat alpha, cfloat s, cfloat beta, con
 }
 
 __device__ __forceinline__ float ldg_of(const float* p) { return __ldg(p); }
-__device__ __forceinline__ cfloat ldg_of(const cfloat* p)
-{
-    const float2 v = __ldg((const float2*)p);
-    return cfloat{v.x, v.y};
-}
 // for kernels whose launch may start before the one ahead of it has ended:
-// their inputs aren't constant data
-__device__ __forceinline__ float ld_of(const float* p) { return *p; }
+// their inputs aren't constant data.  HALF: complex data at 4 modulo 8.
+template <bool HALF = false>
+__device__ __forceinline__ float ld_of(const float* p)
+{
+    return *p;
+}
+template <bool HALF = false>
 __device__ __forceinline__ cfloat ld_of(const cfloat* p)
 {
+    if (HALF) return cfloat{((const float*)p)[0], ((const float*)p)[1]};
     const float2 v = *(const float2*)p;
     return cfloat{v.x, v.y};
 }
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kNThreads) gemv_n_stream_kernel(int m, int n, 
 // Measured (us, before and after, operands in L2): real 256 x 256 10.7, 4.2;
 // 423 x 9911, lda 425, 41, 9.1; 4096 x 4096 19.0, 12.3; 5000 x 5001 42, 15.8;
 // 9001 x 9000 (G = 1) 78, 61; complex 3001 x 1777, lda 3003, 18.2, 9.1.
-template <class T, bool VEC, int G>
+template <class T, bool VEC, int G, bool HALF = false>
 __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T alpha, const T* __restrict__ A, long lda,
                                                                const T* __restrict__ x, long incx, T beta,
                                                                T* __restrict__ y, long incy, int cps,
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T a
                     for (int u = 0; u < 8; ++u)
 #pragma unroll
                         for (int r = 0; r < R; ++r)
-                            v[u][r] = row0 + r * RS < m ? ld_of(Ac + (long)(c + u) * lda + r * RS) : zero_of(T());
+                            v[u][r] = row0 + r * RS < m ? ld_of<HALF>(Ac + (long)(c + u) * lda + r * RS) : zero_of(T());
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
 #pragma unroll
@@ -503,11 +504,14 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
             if (!partial) return cudaErrorMemoryAllocation;
         }
         dim3 grid(rt, splits);
-#define LAUNCH(V, G)                                                                                       \
-    return pdl_launch(gemv_n_kernel<T, V, G>, dim3(grid), kNThreads * G, 0, h->stream, dependent((long)m * n),   \
+#define LAUNCH(V, G, HALF)                                                                                       \
+    return pdl_launch(gemv_n_kernel<T, V, G, HALF>, dim3(grid), kNThreads * G, 0, h->stream, dependent((long)m * n), \
                       m, n, alpha, A, lda, x, incx, beta, y, incy, cps, partial, h->ws.counters)
-        if (small) { if (vec) LAUNCH(true, 4); else LAUNCH(false, 4); }
-        else if (!vec) LAUNCH(false, 1);
+        if constexpr (sizeof(T) == sizeof(cfloat)) {
+            if (!aligned8(A)) { if (small) LAUNCH(false, 4, true); else LAUNCH(false, 1, true); }
+        }
+        if (small) { if (vec) LAUNCH(true, 4, false); else LAUNCH(false, 4, false); }
+        else if (!vec) LAUNCH(false, 1, false);
         else
             gemv_n_stream_kernel<T><<<grid, kNThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, cps,
                                                                        partial, h->ws.counters);
@@ -517,7 +521,8 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     // op T / C: columns of A are dot products with x
     const bool vec = aligned16(A) && ((long)lda * sizeof(T)) % 16 == 0 && incx == 1 && aligned16(x);
     const bool conj = (trans == ICLBLAS_OP_C) && sizeof(T) == sizeof(cfloat);
-    if (!vec && m >= 1024 && n <= 6000) {
+    const bool elems = sizeof(T) == sizeof(float) || (aligned8(A) && aligned8(x));  // else only a float at a time
+    if (!vec && elems && m >= 1024 && n <= 6000) {
         const int seg = ceil_div(ceil_div(m, kTThreads / 32), 32) * 32;
         if (conj)
             return pdl_launch(gemv_t_block_kernel<T, true>, dim3(n), kTThreads, 0, h->stream, dependent((long)m * n),
