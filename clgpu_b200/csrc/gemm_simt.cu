@@ -380,7 +380,9 @@ constexpr TileCost kRealTiles[] = {{128, 128, 209, 184}, {128, 64, 120, 97}, {64
                                    {16, 16, 26, 13}};
 constexpr TileCost kCplxTiles[] = {{64, 64, 260, 205}, {32, 32, 92, 58}, {16, 16, 58, 27}};
 
-// the tile of the least estimated time
+// the tile of the least estimated time, of those whose columns fit the grid's
+// 65,535 blocks in y (the largest tile of a table, the first, may not: n above
+// 8.3 million real or 4.1 million complex columns)
 template <int N>
 int pick_tile(const TileCost (&c)[N], int sms, int m, int n, bool tri)
 {
@@ -388,6 +390,7 @@ int pick_tile(const TileCost (&c)[N], int sms, int m, int n, bool tri)
     double best_t = 0;
     for (int q = 0; q < N; ++q) {
         const long tm = ceil_div(m, c[q].bm), tn = ceil_div(n, c[q].bn);
+        if (q > 0 && tn > 65535) continue;
         const long tiles = tri ? (tm * tn + std::max(tm, tn)) / 2 : tm * tn;
         const double t = std::max((double)c[q].alone, (double)ceil_div(tiles, sms) * c[q].each);
         if (q == 0 || t < best_t) {

@@ -47,3 +47,26 @@ def test_cgemm_tiles(handle, m, n, k):
         O.cgemm(ta, tb, m, n, k, 1.25 - 0.5j, A, ra + pad, Bm, rb + pad, 0.5j, want, m + pad)
         assert B.iclblasCgemm(handle, ta, tb, m, n, k, 1.25 - 0.5j, A, ra + pad, Bm, rb + pad, 0.5j, C, m + pad) == B.SUCCESS
         assert O.rel_fro(C, want) <= 1e-5
+
+
+# flat products of millions of columns: more column tiles of the small sizes
+# than a grid has in y
+def test_sgemm_flat(handle):
+    m, n, k = 4, 2_100_000, 4
+    rng = np.random.default_rng(1)
+    A, Bm, C = (O.colmajor(r, c, r, rng) for r, c in ((m, k), (k, n), (m, n)))
+    want = C.copy()
+    O.sgemm(0, 0, m, n, k, 1.25, A, m, Bm, k, 0.5, want, m)
+    assert B.iclblasSgemm(handle, 0, 0, m, n, k, 1.25, A, m, Bm, k, 0.5, C, m) == B.SUCCESS
+    assert np.array_equal(C, want)
+
+
+@pytest.mark.parametrize("m,n", [(4, 1_100_000), (20, 2_100_000)])
+def test_cgemm_flat(handle, m, n):
+    k = 3
+    rng = np.random.default_rng(m)
+    A, Bm, C = (O.colmajor(r, c, r, rng, np.complex64) for r, c in ((m, k), (k, n), (m, n)))
+    want = C.copy()
+    O.cgemm(0, 0, m, n, k, 1.25, A, m, Bm, k, 0.5j, want, m)
+    assert B.iclblasCgemm(handle, 0, 0, m, n, k, 1.25, A, m, Bm, k, 0.5j, C, m) == B.SUCCESS
+    assert O.rel_fro(C, want) <= 1e-5
