@@ -25,8 +25,8 @@
 // 8192 x 8192 x 4096 NN 11981, 11112, TN 11978, 10524; 2000 x 1500 x 3001 TN
 // with odd leading dimensions 670, 463; 1000^3 98.4, 68.6; 512^3 34.9, 18.5;
 // 256^3 18.5, 8.3; 128 x 100 x 3000 171, 41.  Complex: 4096 x 4096 x 2048 NN
-// 6185, 6226, TN 6456, 6004; 1000 x 750 x 1500 TN 375, 301; 500^3 61.5, 41.0;
-// (re, im) pairs updated by fma.rn.f32x2 measured 10 % slower than scalar
+// 6185, 5430, TN 6456, 5195; 500 x 10000 x 2000 NN 1959, 1734; 2048^2 x 2000
+// NN 1551, 1527; (re, im) pairs updated by fma.rn.f32x2 measured 10 % slower than scalar
 // FMAs there.
 #include <algorithm>
 #include <atomic>
@@ -202,7 +202,10 @@ struct TileCopy {
     }
 };
 
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF>
+// HALF: complex operands at 4 modulo 8.  CONJ: an operand may be conjugated
+// (choosing inside the k loop costs 12 selects per 32 complex products, and a
+// fifth of the time: 4096 x 4096 x 2048 NN 6656 us with, 5430 without).
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF, bool CONJ>
 __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     gemm_simt_kernel(int ta, int tb, int m, int n, int k, T alpha, const T* __restrict__ A, long lda,
                      const T* __restrict__ B, long ldb, T beta, T* __restrict__ C, long ldc, int tri)
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
             if (kk + 1 < BK) read(kk + 1);
             T* fa = a[kk & 1];
             T* fb = b[kk & 1];
-            if constexpr (!std::is_same<T, float>::value) {
+            if constexpr (CONJ) {
 #pragma unroll
                 for (int i = 0; i < TM; ++i) fa[i] = conj_if(fa[i], a_conj);
 #pragma unroll
@@ -342,12 +345,12 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     }
 }
 
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF = false>
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF = false, bool CONJ = false>
 cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alpha, const T* A, int lda, const T* B,
                    int ldb, T beta, T* C, int ldc, int tri)
 {
     using CF = Cfg<T, BM, BN, BK, TM, TN, ST>;
-    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB, HALF>;
+    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB, HALF, CONJ>;
     if (CF::SMEM > 48 * 1024) {
         // the attribute belongs to the current device's copy of the kernel
         static std::atomic<unsigned long long> smem_set{0};
@@ -428,14 +431,17 @@ cudaError_t cgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, c
     const int tile = pick_tile(kCplxTiles, h->sm_count, m, n, false);
     if (!aligned8(A) || !aligned8(B)) {
         // two copies an element: the small tile is not worth a third of these
-        return tile == 0 ? LAUNCH(64, 64, 8, 8, 4, 4, 3, true) : LAUNCH(32, 32, 16, 4, 2, 3, 4, true);
+        return tile == 0 ? LAUNCH(64, 64, 8, 8, 4, 4, 3, true, true) : LAUNCH(32, 32, 16, 4, 2, 3, 4, true, true);
+    }
+    if (ta == ICLBLAS_OP_C || tb == ICLBLAS_OP_C) {
+        switch (tile) {
+        case 0: return LAUNCH(64, 64, 8, 8, 4, 4, 3, false, true);
+        case 1: return LAUNCH(32, 32, 16, 4, 2, 3, 4, false, true);
+        default: return LAUNCH(16, 16, 16, 2, 2, 3, 4, false, true);
+        }
     }
     switch (tile) {
-    case 0:
-        // 4096 x 4096 x 2048 (28 tiles an SM): 8 x 8 outputs a thread 6226 us,
-        // 8 x 4 6653; 2048^3 (7): 8 x 4 1684 us, 8 x 8 slower than 1716
-        if ((long)ceil_div(m, 64) * ceil_div(n, 64) >= 16L * h->sm_count) return LAUNCH(64, 64, 8, 8, 8, 4, 2);
-        return LAUNCH(64, 64, 8, 8, 4, 4, 3);
+    case 0: return LAUNCH(64, 64, 8, 8, 4, 4, 3);
     case 1: return LAUNCH(32, 32, 16, 4, 2, 3, 4);
     default: return LAUNCH(16, 16, 16, 2, 2, 3, 4);
     }
