@@ -224,7 +224,10 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     PDL_FRESH(A);
     PDL_FRESH(B);
     PDL_FRESH(C);
-    pdl_trigger();
+    // no pdl_trigger(): blocks of the next launch would take the free places of
+    // an SM before this one's end, so that an even grid of that launch came to
+    // lie unevenly (1000 x 2000 x 2000, two 128 x 64 tiles an SM: 328 us in a
+    // chain of such calls, 229 without; 512^3 the same either way)
     // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed;
     // tiles wholly outside it have no work
     if ((tri == 1 && m0 + BM - 1 < n0) || (tri == 2 && m0 > n0 + BN - 1)) return;
@@ -369,25 +372,28 @@ cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alp
 }  // namespace
 
 namespace {
-// Estimated SM cycles per k step of a product whose busiest SM works on
-// `ctas` tiles: a lone CTA is bound by its latency, several by throughput.
-// Both constants per tile are measured (B200, k of 1000 to 3000).
-// The complex 16 x 16 tile takes 25 cycles at four tiles an SM and 36 at
-// eight, so it is for three or fewer: 581 x 489 x 283 44.1 us with it, 34.5
-// with 32 x 32; 400 x 300 x 900 47.3 and 44.0.
+// Estimated SM cycles of a product: a lone tile on an SM takes alone0 (its
+// first copies and its stores) + alone * k, bound by latency; several take
+// each0 + each * k apiece, bound by throughput.  Measured from grids of 1 to
+// 500 tiles an SM at k = 4, 100 and 2000.  (Without the constant terms, us,
+// the tile taken so and the one of the table: 1000 x 2000 x 4 10.5, 8.0; 1400 x 700 x 4
+// 7.1, 4.7; 1000 x 2000 x 48 14.6, 11.6.)
 struct TileCost {
     int bm, bn;
-    int alone, each;
+    double alone0, alone, each0, each;
 };
-constexpr TileCost kRealTiles[] = {{128, 128, 209, 184}, {128, 64, 120, 97}, {64, 64, 105, 62}, {32, 32, 41, 24},
-                                   {16, 16, 26, 13}};
-constexpr TileCost kCplxTiles[] = {{64, 64, 260, 205}, {32, 32, 92, 58}, {16, 16, 58, 27}};
+constexpr TileCost kRealTiles[] = {{128, 128, 10000, 207, 10400, 190},
+                                   {128, 64, 8200, 120, 5600, 104},
+                                   {64, 64, 8800, 123, 2860, 55},
+                                   {32, 32, 600, 41, 743, 21},
+                                   {16, 16, 300, 26, 397, 10.5}};
+constexpr TileCost kCplxTiles[] = {{64, 64, 5900, 228, 5200, 191}, {32, 32, 800, 76, 1580, 53}, {16, 16, 300, 50, 465, 20}};
 
 // the tile of the least estimated time, of those whose columns fit the grid's
 // 65,535 blocks in y (the largest tile of a table, the first, may not: n above
 // 8.3 million real or 4.1 million complex columns)
 template <int N>
-int pick_tile(const TileCost (&c)[N], int sms, int m, int n, bool tri)
+int pick_tile(const TileCost (&c)[N], int sms, int m, int n, int k, bool tri)
 {
     int best = 0;
     double best_t = 0;
@@ -395,7 +401,7 @@ int pick_tile(const TileCost (&c)[N], int sms, int m, int n, bool tri)
         const long tm = ceil_div(m, c[q].bm), tn = ceil_div(n, c[q].bn);
         if (q > 0 && tn > 65535) continue;
         const long tiles = tri ? (tm * tn + std::max(tm, tn)) / 2 : tm * tn;
-        const double t = std::max((double)c[q].alone, (double)ceil_div(tiles, sms) * c[q].each);
+        const double t = std::max(c[q].alone0 + c[q].alone * k, ceil_div(tiles, sms) * (c[q].each0 + c[q].each * k));
         if (q == 0 || t < best_t) {
             best = q;
             best_t = t;
@@ -409,12 +415,14 @@ cudaError_t sgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, f
                        const float* B, int ldb, float beta, float* C, int ldc, int tri)
 {
 #define LAUNCH(...) launch<float, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri)
-    switch (pick_tile(kRealTiles, h->sm_count, m, n, tri != 0)) {
+    switch (pick_tile(kRealTiles, h->sm_count, m, n, k, tri != 0)) {
     case 0:
         // 16 x 8 outputs a thread read less shared memory per product, 8 x 8
-        // hide latency with twice the warps: 4096^3 51.3 against 49.1
-        // TFLOP/s, 3000 x 3000 x 1000 (4 tiles an SM) 39.7 against 41.8
-        if ((long)ceil_div(m, 128) * ceil_div(n, 128) >= 6L * h->sm_count) return LAUNCH(128, 128, 16, 16, 8, 3, 2);
+        // hide latency with twice the warps: 4000 x 4000 (7 tiles an SM) x
+        // 2000 1368 us against 1399, x 1000 712 and 711, x 500 384 and 372,
+        // x 48 76 and 54; 3000 x 3000 x 1000 (4 tiles an SM) 39.7 TFLOP/s
+        // against 41.8
+        if (k >= 1000 && (long)ceil_div(m, 128) * ceil_div(n, 128) >= 6L * h->sm_count) return LAUNCH(128, 128, 16, 16, 8, 3, 2);
         return LAUNCH(128, 128, 16, 8, 8, 3, 2);
     case 1: return LAUNCH(128, 64, 16, 8, 8, 4, 3);
     case 2: return LAUNCH(64, 64, 16, 8, 8, 4, 6);
@@ -428,7 +436,7 @@ cudaError_t cgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, c
                        const cfloat* B, int ldb, cfloat beta, cfloat* C, int ldc)
 {
 #define LAUNCH(...) launch<cfloat, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0)
-    const int tile = pick_tile(kCplxTiles, h->sm_count, m, n, false);
+    const int tile = pick_tile(kCplxTiles, h->sm_count, m, n, k, false);
     if (!aligned8(A) || !aligned8(B)) {
         // two copies an element: the small tile is not worth a third of these
         return tile == 0 ? LAUNCH(64, 64, 8, 8, 4, 4, 3, true, true) : LAUNCH(32, 32, 16, 4, 2, 3, 4, true, true);
