@@ -17,6 +17,7 @@
 // host reports EXECUTION_FAILED.
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <cstddef>
 #include <type_traits>
 
@@ -50,12 +51,13 @@ __device__ __forceinline__ float addv(float a, float b) { return a + b; }
 __device__ __forceinline__ cfloat addv(cfloat a, cfloat b) { return cfloat{a.re + b.re, a.im + b.im}; }
 __device__ __forceinline__ float subv(float a, float b) { return a - b; }
 __device__ __forceinline__ cfloat subv(cfloat a, cfloat b) { return cfloat{a.re - b.re, a.im - b.im}; }
-__device__ __forceinline__ float divv(float a, float d) { return a / d; }
-// complex quotient through |d|^2 (the reference's cdiv, core/src/ocl/complex.h.cl:36)
-__device__ __forceinline__ cfloat divv(cfloat a, cfloat d)
+__device__ __forceinline__ float quot(float a, float d) { return a / d; }
+// complex quotient through |d|^2 (the reference's cdiv, core/src/ocl/complex.h.cl:36),
+// in FP64, whose range no square of an FP32 number leaves
+__device__ __forceinline__ cfloat quot(cfloat a, cfloat d)
 {
-    float q = fmaf(d.re, d.re, d.im * d.im);
-    return cfloat{fmaf(a.re, d.re, a.im * d.im) / q, fmaf(a.im, d.re, -a.re * d.im) / q};
+    const double re = d.re, im = d.im, q = 1.0 / fma(re, re, im * im);
+    return cfloat{(float)(fma((double)a.re, re, a.im * im) * q), (float)(fma((double)a.im, re, -(double)a.re * im) * q)};
 }
 __device__ __forceinline__ float shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 __device__ __forceinline__ cfloat shfl(cfloat v, int src)
@@ -774,9 +776,19 @@ __global__ void __launch_bounds__(kThreads, 1)
 //     strsv_tma_kernel: by st.async inside a cluster, as (value, epoch) words
 //     between clusters.  A thread's two rows make one remote store, and those
 //     to the next CTA of the cluster, which waits for them, go first.
-// A block whose inverse or right-hand side holds an infinity or a NaN is
-// solved by substitution instead, so that those reach exactly the entries
-// that substitution gives them to.
+// A block is solved by substitution instead, as accurate as that is,
+//   - when its inverse or right-hand side holds an infinity or a NaN, so that
+//     those reach exactly the entries that substitution gives them to;
+//   - when the largest row sum of |inv(D)| |D| is above kBGrowth: the residual
+//     of a product with the inverse grows with it, substitution's does not.
+//     (FP32 blocks of order 64, residual over |D| |x|, product and
+//     substitution: factors of random matrices by LU, 300 to 550, 2.5e-7 and
+//     9e-8, by Cholesky at condition 1e4, 620, 1.2e-7 and 7e-8; unit triangles
+//     of entries up to 0.5, 750, 3.5e-7 and 1.1e-7, up to 1, 5e4 and more,
+//     2.1e-5 and 9e-8; the error of x is below substitution's in all but the
+//     last.)
+//   - when nonzero entries of its inverse lie below FP32's normal range and
+//     what they lack could show in an entry of x.
 // Measured (us; before: one substitution warp per block and a flag per
 // block): complex n = 3001 512, 88; n = 4096 88; n = 512 25; real with an odd
 // leading dimension n = 4096 67, n = 16384 354.  A step of the chain takes
@@ -791,6 +803,7 @@ constexpr int kBStages = 3;
 // whose clusters of 16 wait for GPCs with 16 free SMs (complex n = 4096 89
 // and 93, real n = 8192 172 and 179).
 constexpr int kBCluster = 16, kBWide = 48;
+constexpr float kBGrowth = 1024.f;
 
 struct alignas(16) dcomplex {
     double re, im;
@@ -822,6 +835,12 @@ __device__ __forceinline__ dcomplex dmul(dcomplex a, dcomplex b)
 {
     return dcomplex{fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re)};
 }
+__device__ __forceinline__ float abs_max(float v) { return fabsf(v); }
+__device__ __forceinline__ float abs_max(cfloat v) { return fmaxf(fabsf(v.re), fabsf(v.im)); }
+__device__ __forceinline__ float abs_sum(float v) { return fabsf(v); }
+__device__ __forceinline__ float abs_sum(cfloat v) { return fabsf(v.re) + fabsf(v.im); }
+__device__ __forceinline__ bool is_zero(double v) { return v == 0.0; }
+__device__ __forceinline__ bool is_zero(dcomplex v) { return v.re == 0.0 && v.im == 0.0; }
 __device__ __forceinline__ bool finite_v(float v) { return isfinite(v); }
 __device__ __forceinline__ bool finite_v(cfloat v) { return isfinite(v.re) && isfinite(v.im); }
 __device__ __forceinline__ void madd_v(float& acc, float a, float x) { acc = fmaf(a, x, acc); }
@@ -991,6 +1010,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     for (int i = 0; i < kBStages - 1; ++i) fetch(i);
 
     // ---- diagonal block: D, then its FP64 inverse
+    float* const rowsum = reinterpret_cast<float*>(S.xs[0]);  // of |D|
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
         const int f = lane + 32 * (q & 1), g = warp * 8 + (q >> 1);
@@ -1033,6 +1053,17 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) S.Y[o + i][o + j] = y[i];
+    } else if (t < 3 * NB) {
+        // meanwhile the row sums of |D|, two threads a row
+        const int r = (t - NB) >> 1, h = (t & 1) * 32;
+        float v = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+            const int c = h + i;
+            v += (lower_op ? c > r : c < r) ? 0.f : c == r && unit ? 1.f : abs_sum(S.D[r][c]);
+        }
+        v = xor_add(v, 1);
+        rowsum[r] = v;
     }
     __syncthreads();
     // the product C Y11 (lower; C Y22 upper) waits in the block's mirror
@@ -1092,22 +1123,31 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     doubling(std::integral_constant<int, 32>{});
 
     T iv[2][8], tc[2][8];
-    // element (r, c) of the inverse
-    auto inv_at = [&](int r, int c) {
-        return r < nr && c < nr && (lower_op ? c <= r : c >= r) ? narrow(S.Y[r][c]) : zero_v(T());
-    };
-    bool fin = true;
+    bool fin = true, low = false;
+    float sum[2] = {0.f, 0.f};  // row sums of |inv(D)| |D|
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            iv[k][j] = inv_at(R0 + 8 * k, cg + 8 * j);
+            const int r = R0 + 8 * k, c = cg + 8 * j;
+            const bool in = r < nr && c < nr && (lower_op ? c <= r : c >= r);
+            const W w = S.Y[r][c];
+            iv[k][j] = in ? narrow(w) : zero_v(T());
             fin = fin && finite_v(iv[k][j]);
+            low = low || (in && abs_max(iv[k][j]) < FLT_MIN && !is_zero(w));
+            sum[k] = fmaf(abs_sum(iv[k][j]), rowsum[c], sum[k]);
         }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) sum[k] = xor_add(sum[k], o);
+    fin = fin && sum[0] <= kBGrowth && sum[1] <= kBGrowth;
     asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 1) : "memory");
     __syncthreads();  // the tile next to D has arrived
     read_tile(kBStages - 1, tc);
-    const bool inv_ok = __syncthreads_and(fin);
+    // inv_ok: neither; low: only the last of the three reasons to substitute
+    const bool inv_ok = __syncthreads_and(fin && !low);
+    if (!inv_ok) low = __syncthreads_and(fin);
     // a[k] += row R0 + 8k of this thread's columns of M times its entries of v
     auto load_x = [&](const T* v, T(&q)[8]) {
         alignas(16) T w[8];
@@ -1201,21 +1241,30 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         yr = subv(brow, cg == 0 ? acc[0] : acc[1]);
         S.y2[bidx<T>(R0 + 8 * cg)] = yr;
     }
-    // a wait failed, or a non-finite right-hand side
-    const int vote = __syncthreads_or((bad ? 1 : 0) | (finite_v(yr) && inv_ok ? 0 : 2));
+    // a wait failed, or the inverse may not do
+    const int vote = __syncthreads_or(bad || !inv_ok || !finite_v(yr));
     if (vote == 0) {
         mul(iv, S.y2, o);
         share(o);
     } else {
         bad = __syncthreads_or(bad);
-        if (!bad) {
+        // an inverse with entries below the normal range leaves out at most
+        // 64 * 2^-126 max|y| an entry: nothing that shows where |y| <= 2^60 and
+        // |x| >= 2^-30
+        bool sub = __syncthreads_or(!low || !finite_v(yr) || abs_max(yr) > 0x1p60f);
+        if (!sub) {
+            mul(iv, S.y2, o);
+            share(o);
+            sub = __syncthreads_or((R0 < nr && abs_max(o[0]) < 0x1p-30f) || (R0 + 8 < nr && abs_max(o[1]) < 0x1p-30f));
+        }
+        if (!bad && sub) {
             // substitution by one warp: each lane owns rows lane and lane + 32
             if (warp == 0) {
                 T b0 = S.y2[bidx<T>(lane)], b1 = S.y2[bidx<T>(lane + 32)];
                 for (int kk = 0; kk < nr; ++kk) {
                     const int k = lower_op ? kk : nr - 1 - kk;
                     T bk = (k < 32) ? shfl(b0, k & 31) : shfl(b1, k & 31);
-                    if (!unit) bk = divv(bk, S.D[k][k]);
+                    if (!unit) bk = quot(bk, S.D[k][k]);
                     if (lane == (k & 31)) { if (k < 32) b0 = bk; else b1 = bk; }
                     const bool u0 = lower_op ? lane > k : lane < k, u1 = lower_op ? lane + 32 > k : lane + 32 < k;
                     if (u0 && lane < nr) msub(b0, S.D[lane][k], bk);

@@ -100,3 +100,71 @@ def test_first_call_captured_and_replayed(handle, cuda):
         assert O.rel_fro(x.cpu().numpy(), x_ref) <= TOL
     handle.set_stream(torch.cuda.current_stream())
     del g
+
+
+def forms(dtype):
+    """(n, lda): complex, real that TMA cannot address, and short aligned real solves."""
+    return ((130, 131), (200, 200)) + (() if dtype == np.complex64 else ((512, 512),))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+@pytest.mark.parametrize("uplo", [0, 1])
+def test_growth(handle, dtype, uplo):
+    """Unit triangles with entries of size 1, whose diagonal blocks have large
+    inverses: substitution leaves a residual of about sqrt(n) roundings of
+    |T| |x|, a product with an FP32 inverse hundreds of them."""
+    for n, lda in ((130, 131), (200, 200)) + (() if dtype == np.complex64 else ((256, 256),)):
+        rng = np.random.default_rng(n)
+        A = O.colmajor(n, n, lda, rng, dtype)
+        T = A.reshape(n, lda).T[:n].astype(np.complex128 if dtype == np.complex64 else np.float64)
+        T = (np.tril(T, -1) if uplo == 1 else np.triu(T, 1)) + np.eye(n)
+        b = (T @ rng.uniform(-1, 1, n)).astype(dtype)
+        x = b.copy()
+        assert solve(handle, dtype, uplo, 0, 1, n, A, lda, x, 1) == B.SUCCESS
+        assert np.isfinite(x).all()
+        res = np.abs(T @ x - b).max() / (np.abs(T) @ np.abs(x)).max()
+        assert res <= 2 * np.sqrt(n) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+@pytest.mark.parametrize("uplo", [0, 1])
+def test_inverse_below_normal_range(handle, dtype, uplo):
+    """Diagonals so large that the inverse's other entries vanish in FP32: each
+    entry of x is still right to a few roundings."""
+    d, e, f = (3e18, 1e-3, 1e18) if dtype == np.complex64 else (1e23, 1.0, 1e23)
+    for n, lda in forms(dtype):
+        rng = np.random.default_rng(n)
+        A = (O.colmajor(n, n, lda, rng, dtype) * dtype(e)).astype(dtype)
+        M = A.reshape(n, lda).T[:n]
+        M[np.arange(n), np.arange(n)] = d
+        b = np.zeros(n, dtype)
+        b[::64] = f
+        if uplo == 0:
+            b = b[::-1].copy()
+        wide = np.complex128 if dtype == np.complex64 else np.float64
+        want = b.astype(wide)
+        T = M.astype(wide)
+        for i in range(n) if uplo == 1 else range(n - 1, -1, -1):
+            want[i] /= T[i, i]
+            rest = slice(i + 1, n) if uplo == 1 else slice(0, i)
+            want[rest] -= T[rest, i] * want[i]
+        assert (np.abs(want) > 1e-36).all()
+        x = b.copy()
+        assert solve(handle, dtype, uplo, 0, 0, n, A, lda, x, 1) == B.SUCCESS
+        assert (np.abs(x - want) <= 1e-4 * np.abs(want)).all()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+def test_narrow_band(handle, dtype):
+    """An inverse that falls off below FP32's range, harmlessly."""
+    for n, lda in forms(dtype):
+        rng = np.random.default_rng(n)
+        A = np.zeros(lda * n, dtype)
+        M = A.reshape(n, lda).T[:n]
+        M[np.arange(n), np.arange(n)] = 4096
+        M[np.arange(1, n), np.arange(n - 1)] = 1
+        x = O.colmajor(n, 1, n, rng, dtype)
+        x_ref = x.copy()
+        want(dtype, 1, 0, 0, n, A, lda, x_ref, 1)
+        assert solve(handle, dtype, 1, 0, 0, n, A, lda, x, 1) == B.SUCCESS
+        assert O.rel_fro(x, x_ref) <= TOL
