@@ -7,7 +7,8 @@
 // n rows are cut into blocks, one CTA per block; the CTAs draw tickets from
 // an atomic counter and own blocks in solve order (forward for a lower
 // op(A), backward for an upper one), so a CTA only ever waits for CTAs that
-// are already running.  Two kernels share that structure:
+// are already running.  Two kernels share that structure, and solves of up to
+// 128 rows are one CTA's substitution (trsv_small_kernel):
 //   - strsv_tma_kernel: long real solves that TMA can address, 128-row blocks;
 //   - trsv_block_kernel: everything else (complex data, short solves, any
 //     base address and leading dimension), 64-row blocks fetched element by
@@ -51,6 +52,17 @@ __device__ __forceinline__ float addv(float a, float b) { return a + b; }
 __device__ __forceinline__ cfloat addv(cfloat a, cfloat b) { return cfloat{a.re + b.re, a.im + b.im}; }
 __device__ __forceinline__ float subv(float a, float b) { return a - b; }
 __device__ __forceinline__ cfloat subv(cfloat a, cfloat b) { return cfloat{a.re - b.re, a.im - b.im}; }
+__device__ __forceinline__ float shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ cfloat shfl(cfloat v, int src)
+{
+    return cfloat{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+}
+
+__device__ __forceinline__ int ld_volatile(const int* p) { return *(const volatile int*)p; }
+
+// ---------------------------------------------------------------- substitution
+__device__ __forceinline__ float abs_max(float v) { return fabsf(v); }
+__device__ __forceinline__ float abs_max(cfloat v) { return fmaxf(fabsf(v.re), fabsf(v.im)); }
 __device__ __forceinline__ float quot(float a, float d) { return a / d; }
 // complex quotient through |d|^2 (the reference's cdiv, core/src/ocl/complex.h.cl:36),
 // in FP64, whose range no square of an FP32 number leaves
@@ -59,13 +71,126 @@ __device__ __forceinline__ cfloat quot(cfloat a, cfloat d)
     const double re = d.re, im = d.im, q = 1.0 / fma(re, re, im * im);
     return cfloat{(float)(fma((double)a.re, re, a.im * im) * q), (float)(fma((double)a.im, re, -(double)a.re * im) * q)};
 }
-__device__ __forceinline__ float shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ cfloat shfl(cfloat v, int src)
+// 1 / d as hi + lo
+__device__ __forceinline__ void recip(float d, float& hi, float& lo)
 {
-    return cfloat{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+    const double w = 1.0 / d;
+    hi = (float)w;
+    lo = (float)(w - (double)hi);
+}
+__device__ __forceinline__ void recip(cfloat d, cfloat& hi, cfloat& lo)
+{
+    const double re = d.re, im = d.im, q = 1.0 / fma(re, re, im * im);
+    hi = cfloat{(float)(re * q), (float)(-im * q)};
+    lo = cfloat{(float)(re * q - (double)hi.re), (float)(-im * q - (double)hi.im)};
+}
+// v / d for 1 / d = hi + lo, right to less than a rounding where nothing
+// leaves the normal range
+__device__ __forceinline__ float times(float v, float hi, float lo) { return fmaf(v, hi, v * lo); }
+__device__ __forceinline__ cfloat times(cfloat v, cfloat hi, cfloat lo)
+{
+    return cfloat{fmaf(v.re, hi.re, fmaf(-v.im, hi.im, fmaf(v.re, lo.re, -v.im * lo.im))),
+                  fmaf(v.re, hi.im, fmaf(v.im, hi.re, fmaf(v.re, lo.im, v.im * lo.re)))};
 }
 
-__device__ __forceinline__ int ld_volatile(const int* p) { return *(const volatile int*)p; }
+// One warp solves the nr x nr lower triangle with element (r, k) at
+// D[r * sr + k * sc] (shared memory, sr odd) in place of v: lane l holds rows
+// l + 32 q, those past nr anything.  (An upper triangle is a lower one with rows
+// and columns in reverse order.)  Bound by the chain of nr steps, each a
+// quotient, a shuffle and an update; so that no division lies in it, the
+// diagonal's reciprocals are formed first, as two floats each, wherever they
+// are in range.
+template <class T, int R, bool FAST>
+__device__ __forceinline__ void substitute_steps(const T* D, int sr, int sc, int nr, bool unit, const T (&hi)[R],
+                                                 const T (&lo)[R], T (&v)[R])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int steps = min(32, nr - 32 * q);
+#pragma unroll 1
+        for (int l = 0; l < steps; ++l) {
+            T x = v[q];
+            if (!unit) x = FAST ? times(x, hi[q], lo[q]) : quot(x, hi[q]);
+            x = shfl(x, l);
+            if (lane == l) v[q] = x;
+#pragma unroll
+            for (int p = q; p < R; ++p)
+                if ((p > q || lane > l) && lane + 32 * p < nr)
+                    msub(v[p], D[(lane + 32 * p) * sr + (l + 32 * q) * sc], x);
+        }
+    }
+}
+template <class T, int R>
+__device__ __forceinline__ void substitute(const T* D, int sr, int sc, int nr, bool unit, T (&v)[R])
+{
+    const int lane = threadIdx.x & 31;
+    T hi[R], lo[R];
+    bool fast = true;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        hi[q] = lo[q] = zero_v(T());
+        if (unit || lane + 32 * q >= nr) continue;
+        hi[q] = D[(lane + 32 * q) * (sr + sc)];
+        fast = fast && abs_max(hi[q]) >= 0x1p-100f && abs_max(hi[q]) <= 0x1p100f;
+    }
+    if (__all_sync(0xffffffffu, fast)) {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (!unit) recip(hi[q], hi[q], lo[q]);
+        substitute_steps<T, R, true>(D, sr, sc, nr, unit, hi, lo, v);
+    } else {
+        substitute_steps<T, R, false>(D, sr, sc, nr, unit, hi, lo, v);
+    }
+}
+
+// Solves of up to kSmall rows, a CTA: the triangle goes to shared memory, the
+// first warp substitutes.  R: rows of a lane.
+// Measured (us, 64-row block kernel and this one): real n = 1 8.5, 2.0, n = 64
+// 12.4, 5.7, n = 128 16.4, 13.3; complex n = 1 12.5, 2.3, n = 64 16.9, 6.7,
+// n = 128 18.2, 15.3; n = 129 14.9 and 19.7 in the block kernel.
+constexpr int kSmall = 128;
+template <class T, int R>
+__global__ void __launch_bounds__(kThreads) trsv_small_kernel(int n, int lower_op, int op, int unit,
+                                                              const T* __restrict__ A, long lda, T* x, long incx)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* const D = reinterpret_cast<T*>(smem_raw);
+    const int P = n | 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // consecutive lanes read consecutive addresses, rows of a column of A; a
+    // lane's elements of 8 columns are in flight at once (one column at a time
+    // n = 65 took 15 us)
+    const bool lower_a = (op == 0) == (lower_op != 0);
+    for (int c0 = warp; c0 < n; c0 += 8 * (kThreads / 32)) {
+        T e[8][R];
+        auto in = [&](int r, int c) { return r < n && c < n && (lower_a ? r >= c : r <= c); };
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int r = lane + 32 * q, c = c0 + u * (kThreads / 32);
+                e[u][q] = in(r, c) ? A[(long)c * lda + r] : zero_v(T());
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int r = lane + 32 * q, c = c0 + u * (kThreads / 32);  // (r, c) of A, (r, c) or (c, r) of op(A)
+                if (in(r, c)) D[op == 0 ? r * P + c : c * P + r] = op == 2 ? conj_v(e[u][q]) : e[u][q];
+            }
+    }
+    T v[R];
+    auto row = [&](int q) { return lower_op ? lane + 32 * q : n - 1 - lane - 32 * q; };
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = warp == 0 && lane + 32 * q < n ? x[(long)row(q) * incx] : zero_v(T());
+    __syncthreads();
+    if (warp != 0) return;
+    const int sg = lower_op ? 1 : -1;
+    substitute<T, R>(lower_op ? D : D + (n - 1) * (P + 1), sg * P, sg, n, unit != 0, v);
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (lane + 32 * q < n) x[(long)row(q) * incx] = v[q];
+}
 
 // ---------------------------------------------------------------- STRSV, TMA path
 // Float TRSV when A is 16-byte aligned with lda a multiple of 4 and >= n
@@ -835,8 +960,6 @@ __device__ __forceinline__ dcomplex dmul(dcomplex a, dcomplex b)
 {
     return dcomplex{fma(a.re, b.re, -a.im * b.im), fma(a.re, b.im, a.im * b.re)};
 }
-__device__ __forceinline__ float abs_max(float v) { return fabsf(v); }
-__device__ __forceinline__ float abs_max(cfloat v) { return fmaxf(fabsf(v.re), fabsf(v.im)); }
 __device__ __forceinline__ float abs_sum(float v) { return fabsf(v); }
 __device__ __forceinline__ float abs_sum(cfloat v) { return fabsf(v.re) + fabsf(v.im); }
 __device__ __forceinline__ bool is_zero(double v) { return v == 0.0; }
@@ -1258,20 +1381,13 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
             sub = __syncthreads_or((R0 < nr && abs_max(o[0]) < 0x1p-30f) || (R0 + 8 < nr && abs_max(o[1]) < 0x1p-30f));
         }
         if (!bad && sub) {
-            // substitution by one warp: each lane owns rows lane and lane + 32
             if (warp == 0) {
-                T b0 = S.y2[bidx<T>(lane)], b1 = S.y2[bidx<T>(lane + 32)];
-                for (int kk = 0; kk < nr; ++kk) {
-                    const int k = lower_op ? kk : nr - 1 - kk;
-                    T bk = (k < 32) ? shfl(b0, k & 31) : shfl(b1, k & 31);
-                    if (!unit) bk = quot(bk, S.D[k][k]);
-                    if (lane == (k & 31)) { if (k < 32) b0 = bk; else b1 = bk; }
-                    const bool u0 = lower_op ? lane > k : lane < k, u1 = lower_op ? lane + 32 > k : lane + 32 < k;
-                    if (u0 && lane < nr) msub(b0, S.D[lane][k], bk);
-                    if (u1 && lane + 32 < nr) msub(b1, S.D[lane + 32][k], bk);
-                }
-                S.y2[bidx<T>(lane)] = b0;
-                S.y2[bidx<T>(lane + 32)] = b1;
+                // (rows past nr, lower: 0; upper: the order starts at nr - 1)
+                const int sg = lower_op ? 1 : -1, ra = lower_op ? lane : nr - 1 - lane, rb = ra + 32 * sg;
+                T v[2] = {ra >= 0 ? S.y2[bidx<T>(ra)] : zero_v(T()), rb >= 0 ? S.y2[bidx<T>(rb)] : zero_v(T())};
+                substitute<T, 2>(lower_op ? &S.D[0][0] : &S.D[nr - 1][nr - 1], sg * (NB + 1), sg, nr, unit != 0, v);
+                if (ra >= 0) S.y2[bidx<T>(ra)] = v[0];
+                if (rb >= 0) S.y2[bidx<T>(rb)] = v[1];
             }
             __syncthreads();
             o[0] = S.y2[bidx<T>(R0)];
@@ -1530,10 +1646,41 @@ cudaError_t trsv_block(iclblasHandle_t h, int uplo, int trans, int diag, int n, 
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+template <class T, int R>
+cudaError_t trsv_small_launch(iclblasHandle_t h, int n, int lower_op, int op, int unit, const T* A, int lda, T* x,
+                              int incx)
+{
+    const int smem = n * (n | 1) * (int)sizeof(T);
+    if (smem > 48 * 1024) {
+        static std::atomic<unsigned long long> smem_set{0};
+        const unsigned long long bit = 1ull << (h->device & 63);
+        if (!(smem_set.load() & bit)) {
+            const cudaError_t e = cudaFuncSetAttribute(trsv_small_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       kSmall * (kSmall | 1) * (int)sizeof(T));
+            if (e != cudaSuccess) return e;
+            smem_set.fetch_or(bit);
+        }
+    }
+    trsv_small_kernel<T, R><<<1, kThreads, smem, h->stream>>>(n, lower_op, op, unit, A, lda, x, incx);
+    return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t trsv_small(iclblasHandle_t h, int uplo, int trans, int diag, int n, const T* A, int lda, T* x, int incx)
+{
+    const int op = trans == ICLBLAS_OP_N ? 0 : (trans == ICLBLAS_OP_C && sizeof(T) == sizeof(cfloat)) ? 2 : 1;
+    const bool lower = uplo == ICLBLAS_FILL_MODE_LOWER;
+    const int lower_op = (op == 0) ? lower : !lower, unit = diag == ICLBLAS_DIAG_UNIT;
+    if (n <= 32) return trsv_small_launch<T, 1>(h, n, lower_op, op, unit, A, lda, x, incx);
+    if (n <= 64) return trsv_small_launch<T, 2>(h, n, lower_op, op, unit, A, lda, x, incx);
+    return trsv_small_launch<T, 4>(h, n, lower_op, op, unit, A, lda, x, incx);
+}
+
 }  // namespace
 
 cudaError_t strsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const float* A, int lda, float* x, int incx)
 {
+    if (n <= kSmall) return trsv_small<float>(h, uplo, trans, diag, n, A, lda, x, incx);
     // short solves are bound by the time to the first block's inverse, which
     // 64-row blocks have sooner (n = 512: 19 us against 30 with 128-row
     // blocks, n = 1024 25 and 34, n = 2048 41 and 42, n = 3072 55 and 52)
@@ -1548,6 +1695,7 @@ cudaError_t strsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const
 cudaError_t ctrsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const cfloat* A, int lda, cfloat* x,
                   int incx)
 {
+    if (n <= kSmall) return trsv_small<cfloat>(h, uplo, trans, diag, n, A, lda, x, incx);
     return aligned8(A) ? trsv_block<cfloat, false>(h, uplo, trans, diag, n, A, lda, x, incx)
                        : trsv_block<cfloat, true>(h, uplo, trans, diag, n, A, lda, x, incx);
 }

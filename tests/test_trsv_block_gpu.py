@@ -1,5 +1,7 @@
-"""TRSV's 64-row block kernel (complex data, and real data that TMA cannot
-address) at the edges of its blocks and clusters, against the oracle.
+"""TRSV's 64-row block kernel (complex data, short solves, and real data that
+TMA cannot address) at the edges of its blocks and clusters, and the one-CTA
+substitution of up to 128 rows at the edges of its warps' rows, against the
+oracle.
 
 Tolerance: relative Frobenius error <= 1e-5 against the FP64-accumulating
 oracle, the bar of the other TRSV tests."""
@@ -31,8 +33,9 @@ def want(dtype, *args):
     (O.ctrsv if dtype == np.complex64 else O.strsv)(*args)
 
 
-# one block, its edges, two blocks, a cluster's 8 blocks and the first of the next, several clusters
-@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 129, 511, 512, 513, 577, 1333])
+# one CTA with one, two and four rows a lane; then blocks and their edges, a cluster's 8 blocks and the first of
+# the next, several clusters
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 97, 127, 128, 129, 511, 512, 513, 577, 1333])
 @pytest.mark.parametrize("dtype", [np.float32, np.complex64])
 def test_block_edges(handle, n, dtype):
     rng = np.random.default_rng(n)
@@ -55,15 +58,14 @@ def test_block_edges(handle, n, dtype):
 def test_non_finite(handle, dtype, uplo):
     """A NaN or an infinity in b and a zero on the diagonal make exactly the
     entries non-finite that substitution makes so."""
-    n = 201
     rng = np.random.default_rng(5 + uplo)
-    for what in ("nan", "inf", "zero"):
+    for n, what in ((n, what) for n in (201, 50) for what in ("nan", "inf", "zero")):
         A = tri(n, n, uplo == 1, rng, dtype)
         x = O.colmajor(n, 1, n, rng, dtype)
         if what == "zero":
-            A[100 * n + 100] = 0
+            A[n // 2 * n + n // 2] = 0
         else:
-            x[100] = np.nan if what == "nan" else np.inf
+            x[n // 2] = np.nan if what == "nan" else np.inf
         x_ref = x.copy()
         with np.errstate(all="ignore"):
             want(dtype, uplo, 0, 0, n, A, n, x_ref, 1)
@@ -104,7 +106,7 @@ def test_first_call_captured_and_replayed(handle, cuda):
 
 def forms(dtype):
     """(n, lda): complex, real that TMA cannot address, and short aligned real solves."""
-    return ((130, 131), (200, 200)) + (() if dtype == np.complex64 else ((512, 512),))
+    return ((100, 101), (130, 131), (200, 200)) + (() if dtype == np.complex64 else ((512, 512),))
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.complex64])
@@ -131,8 +133,9 @@ def test_growth(handle, dtype, uplo):
 def test_inverse_below_normal_range(handle, dtype, uplo):
     """Diagonals so large that the inverse's other entries vanish in FP32: each
     entry of x is still right to a few roundings."""
-    d, e, f = (3e18, 1e-3, 1e18) if dtype == np.complex64 else (1e23, 1.0, 1e23)
-    for n, lda in forms(dtype):
+    mid = (3e18, 1e-3, 1e18) if dtype == np.complex64 else (1e23, 1.0, 1e23)
+    # (70: diagonals whose reciprocals the one-CTA substitution does not form either)
+    for n, lda, (d, e, f) in [(n, lda, mid) for n, lda in forms(dtype)] + [(70, 71, (1e32, 1.0, 1e32))]:
         rng = np.random.default_rng(n)
         A = (O.colmajor(n, n, lda, rng, dtype) * dtype(e)).astype(dtype)
         M = A.reshape(n, lda).T[:n]
