@@ -122,7 +122,7 @@ ICLBLAS_API iclblasStatus_t iclblasSdot(iclblasHandle_t handle, int n, float* x,
  *     kernel cannot read another GPU's memory); the call is asynchronous on the
  *     handle's stream and its result equals iclblasSdot's;
  *   - a call needing more than 4096 partials -- one per block, with one
- *     block up to n = 16384, else min(ceil(n/1024), 8 x SM count) blocks for
+ *     block for short vectors, else min(ceil(n/1024), 8 x SM count) blocks for
  *     unit-stride 16-byte-aligned operands and min(ceil(n/256), 8 x SM count)
  *     otherwise -- returns NOT_SUPPORTED;
  *   - the first call on each device looks up the array's device address

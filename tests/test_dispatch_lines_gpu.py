@@ -52,3 +52,19 @@ def test_trsv_of_one_row(us, cuda, cplx):
     f = B.iclblasCtrsv if cplx else B.iclblasStrsv
     one, full = (us(lambda h: f(h, 1, 0, 0, n, A, 65, x, 1)) for n in (1, 64))
     assert one <= 0.5 * full
+
+
+@pytest.mark.parametrize("inc,shift", [(1, 0), (1, 1), (2, 0), (17, 0)])
+def test_reductions_of_short_vectors(us, cuda, inc, shift):
+    """Half the elements never take much longer (one block or several)."""
+    import torch
+    big = 18000
+    x, y = buf(big * inc + 4, False, cuda)[shift:], buf(big * inc + 4, False, cuda)[shift:]
+    xc, yc = buf(big * inc + 4, True, cuda)[shift:], buf(big * inc + 4, True, cuda)[shift:]
+    r, ri = torch.zeros(1, dtype=torch.complex64, device=cuda), torch.zeros(1, dtype=torch.int32, device=cuda)
+    for call in (lambda h, n: B.iclblasSdot(h, n, x, inc, y, inc, r), lambda h, n: B.iclblasSasum(h, n, x, inc, r),
+                 lambda h, n: B.iclblasIsamax(h, n, x, inc, ri), lambda h, n: B.iclblasCdotc(h, n, xc, inc, yc, inc, r),
+                 lambda h, n: B.iclblasScnrm2(h, n, xc, inc, r), lambda h, n: B.iclblasIcamax(h, n, xc, inc, ri)):
+        several = us(lambda h: call(h, big))
+        for n in (2048, 4096, 8192, 12000, 16384):
+            assert us(lambda h: call(h, n)) <= 1.3 * several, n
