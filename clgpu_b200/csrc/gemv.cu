@@ -57,7 +57,6 @@ __device__ __forceinline__ cfloat axpby(cfloat alpha, cfloat s, cfloat beta, con
     return r;
 }
 
-__device__ __forceinline__ float ldg_of(const float* p) { return __ldg(p); }
 // for kernels whose launch may start before the one ahead of it has ended:
 // their inputs aren't constant data.  HALF: complex data at 4 modulo 8.
 template <bool HALF = false>
@@ -331,7 +330,7 @@ __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T a
 
 // ------------------------------------------------------------------ op T / C
 // Warp w of the grid handles column col = w / S, row slice w % S of S.
-template <class T, bool CONJ, bool VEC>
+template <class T, bool CONJ, bool VEC, int U>
 __global__ void __launch_bounds__(kTThreads) gemv_t_kernel(int m, int n, T alpha, const T* __restrict__ A, long lda,
                                                            const T* __restrict__ x, long incx, T beta,
                                                            T* __restrict__ y, long incy, int S, int rps,
@@ -381,20 +380,19 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_kernel(int m, int n, T alpha
         for (int k = 0; k < R; ++k)
             if (r + k < r1) madd<CONJ>(acc, Ac[r + k], x[r + k]);
     } else {
-        // real data: 8 loads of each operand in flight, the last ones
-        // predicated (9001 x 9000 147 us with one at a time, 74 so; 1000 x 1000
-        // 9.0, 3.4); complex data measured slower that way
-        if constexpr (sizeof(T) == sizeof(float)) {
-            for (int r = r0 + lane; r < r1; r += 8 * 32) {
-                T v[8], xv[8];
+        // U > 1 (real data): U loads of each operand in flight, the last ones
+        // predicated
+        if constexpr (U > 1) {
+            for (int r = r0 + lane; r < r1; r += U * 32) {
+                T v[U], xv[U];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
+                for (int u = 0; u < U; ++u) {
                     const bool in = r + u * 32 < r1;
-                    v[u] = in ? ldg_of(Ac + r + u * 32) : zero_of(T());
-                    xv[u] = in ? ldg_of(x + (long)(r + u * 32) * incx) : zero_of(T());
+                    v[u] = in ? __ldg(Ac + r + u * 32) : zero_of(T());
+                    xv[u] = in ? __ldg(x + (long)(r + u * 32) * incx) : zero_of(T());
                 }
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
+                for (int u = 0; u < U; ++u)
                     if (r + u * 32 < r1) madd<CONJ>(acc, v[u], xv[u]);
             }
         } else {
@@ -426,10 +424,8 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_kernel(int m, int n, T alpha
 
 // Tall columns without 16-byte alignment: a block a column, its rows in eight
 // runs, one a warp, 8 loads of each operand in flight, the warps' sums added
-// in shared memory.  Against a warp a column, in slices whose sums go through
-// global memory and an atomic (us, operands in L2): real 3001 x 1777 11.1,
-// 7.3; 5000 x 100 9.4, 3.1; complex 5000 x 5001 55, 43; but 600 x 9000 6.9,
-// 14.2 and real 9001 x 9000 74, 79.
+// in shared memory.  Against warps that each take a slice of a column, whose
+// sums go through global memory and an atomic, see block_columns().
 template <class T, bool CONJ>
 __global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha, const T* __restrict__ A, long lda,
                                                                  const T* __restrict__ x, long incx, T beta,
@@ -471,6 +467,23 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha,
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+// Whether op T / C of an unaligned m x n matrix takes a block a column: for
+// columns that are long enough for eight warps, yet no longer than one block
+// reads in the time the slices' sums cost, and not many more than the SMs
+// hold blocks.  Measured against the slices (us, operands in L2): real 1025 x
+// 1025 3.0, 3.6; 3000 x 1777 6.8, 8.8; 6000 x 6000 35, 39; but 1500 x 6000
+// 11.2, 9.4; 100000 x 33 23, 9.3; 1000000 x 4 215, 25.  Complex 1025 x 1025
+// 3.9, 5.2; 3000 x 1777 8.8, 10.3; 10000 x 600 9.2, 11.2; 30000 x 600 32, 41;
+// but 1500 x 3000 8.3, 7.5; 3000 x 6000 42, 38; 30000 x 33 12.3, 8.0; 100000 x
+// 200 80, 48.
+bool block_columns(bool cplx, int m, int n)
+{
+    if (m < 1024 || n > 6000) return false;
+    if (!cplx) return m < 2048 ? n <= 2048 : m <= 32768;
+    if (m < 4096) return n <= (m < 2048 ? 1600 : 4096);
+    return m <= 12288 || (m <= 49152 && n >= 300);
+}
 
 template <class T>
 cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const T* A, int lda, const T* x, int incx,
@@ -522,7 +535,7 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     const bool vec = aligned16(A) && ((long)lda * sizeof(T)) % 16 == 0 && incx == 1 && aligned16(x);
     const bool conj = (trans == ICLBLAS_OP_C) && sizeof(T) == sizeof(cfloat);
     const bool elems = sizeof(T) == sizeof(float) || (aligned8(A) && aligned8(x));  // else only a float at a time
-    if (!vec && elems && m >= 1024 && n <= 6000) {
+    if (!vec && elems && block_columns(sizeof(T) == sizeof(cfloat), m, n)) {
         const int seg = ceil_div(ceil_div(m, kTThreads / 32), 32) * 32;
         if (conj)
             return pdl_launch(gemv_t_block_kernel<T, true>, dim3(n), kTThreads, 0, h->stream, dependent((long)m * n),
@@ -533,9 +546,7 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     }
     const int warps_target = target * (kTThreads / 32);
     int S = 1;
-    // (a real scalar load brings a quarter as much: shorter slices)
-    if (n < warps_target && n <= kCounterWords)
-        S = min(ceil_div(warps_target, n), max(1, m / (vec || sizeof(T) != sizeof(float) ? 1024 : 512)));
+    if (n < warps_target && n <= kCounterWords) S = min(ceil_div(warps_target, n), max(1, m / 1024));
     int rps = ceil_div(m, S);
     rps = (rps + 32 * R - 1) / (32 * R) * (32 * R);
     S = ceil_div(m, rps);
@@ -546,11 +557,20 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
     }
     const long warps = (long)n * S;
     const int grid = (int)((warps * 32 + kTThreads - 1) / kTThreads);
-#define LAUNCH(C, V)                                                                                         \
-    gemv_t_kernel<T, C, V><<<grid, kTThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, S, \
-                                                              rps, partial, h->ws.counters)
-    if (conj) { if (vec) LAUNCH(true, true); else LAUNCH(true, false); }
-    else { if (vec) LAUNCH(false, true); else LAUNCH(false, false); }
+#define LAUNCH(C, V, U)                                                                                         \
+    gemv_t_kernel<T, C, V, U><<<grid, kTThreads, 0, h->stream>>>(m, n, alpha, A, lda, x, incx, beta, y, incy, S, \
+                                                                 rps, partial, h->ws.counters)
+    if (conj) { if (vec) LAUNCH(true, true, 1); else LAUNCH(true, false, 1); return cudaGetLastError(); }
+    if constexpr (sizeof(T) == sizeof(float)) {
+        // batches of loads, unless many columns keep the SMs busy and most of a
+        // column's last batch would be empty: 1025 x 30000 69 us with one load
+        // at a time, 31 in batches, 100 x 100 2.5, 1.9, 100 x 30000 9.3, 8.8; but
+        // 300 x 30000 9.9, 13.4, 33 x 30000 6.3, 8.5
+        const int rows = min(m, rps);
+        const bool empty = rows <= 64 || (rows > 256 && rows < 512);
+        if (!vec && (n <= 2048 || !empty)) { LAUNCH(false, false, 8); return cudaGetLastError(); }
+    }
+    if (vec) LAUNCH(false, true, 1); else LAUNCH(false, false, 1);
 #undef LAUNCH
     return cudaGetLastError();
 }

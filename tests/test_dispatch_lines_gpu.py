@@ -68,3 +68,13 @@ def test_reductions_of_short_vectors(us, cuda, inc, shift):
         several = us(lambda h: call(h, big))
         for n in (2048, 4096, 8192, 12000, 16384):
             assert us(lambda h: call(h, n)) <= 1.3 * several, n
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_gemv_t_of_tall_and_of_short_columns(us, cuda, cplx):
+    """Unaligned columns against aligned ones: a few tall ones, many short ones."""
+    f = B.iclblasCgemv if cplx else B.iclblasSgemv
+    for m, n, factor in ((1_000_000, 4, 2.0), (100_000, 33, 2.0), (4, 100_000, 1.3), (33, 100_000, 1.3)):
+        A, x, y = buf((m + 4) * n, cplx, cuda), buf(m, cplx, cuda), buf(n, cplx, cuda)
+        odd, aligned = (us(lambda h: f(h, 1, m, n, 1.0, A, lda, x, 1, 0.0, y, 1)) for lda in (m | 1, m + -m % 4))
+        assert odd <= factor * aligned + 1, (m, n)
