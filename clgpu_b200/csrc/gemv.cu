@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kNThreads * G) gemv_n_kernel(int m, int n, T a
             } else {
                 int c = 8 * g;
                 // (VEC: the few rows past the last whole vector)
-                for (; !VEC && c + 8 <= cn; c += 8 * G) {
+                for (; c + 8 <= cn; c += 8 * G) {
                     T v[8][R];
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
@@ -498,12 +498,18 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
         // bandwidth-bound: enough blocks of 64 columns and more to fill the
         // GPU (one group a block); else four groups a block and as many
         // slices as the SMs hold blocks, at least one batch of columns a
-        // group (16384 x 16384 with four groups: 297 us against 159)
-        const bool small = (long)rt * max(1, n / 64) < target;
+        // group (16384 x 16384 with four groups: 297 us against 159).  Up to
+        // 128 columns are one slice: adding slices costs more than a few
+        // batches (3000 x 33 4.1 us with two, 2.4), and so they are where the
+        // row tiles nearly fill the GPU (100000 x 200 12.5, 8.9); with a batch
+        // or two of columns three groups would be idle (complex 1000000 x 4
+        // 17 us with four groups, 5.8 with one; 100000 x 4 3.3, 2.4)
+        const bool wide = rt >= 96, few = n <= 16 && (!vec || rt > 2 * h->sm_count);
+        const bool small = (long)rt * max(1, n / 64) < target && !few && !(wide && n > 320);
         int splits = 1, unit = 8;
         if (small) {
             unit = 32;
-            splits = max(1, min(ceil_div(2 * h->sm_count, rt), ceil_div(n, unit)));
+            if (n > 128 && !wide) splits = min(ceil_div(2 * h->sm_count, rt), ceil_div(n, unit));
         } else if (rt < target && rt <= kCounterWords) {
             splits = ceil_div(target, rt);
             splits = min(splits, max(1, n / 64));

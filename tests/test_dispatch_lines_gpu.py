@@ -78,3 +78,12 @@ def test_gemv_t_of_tall_and_of_short_columns(us, cuda, cplx):
         A, x, y = buf((m + 4) * n, cplx, cuda), buf(m, cplx, cuda), buf(n, cplx, cuda)
         odd, aligned = (us(lambda h: f(h, 1, m, n, 1.0, A, lda, x, 1, 0.0, y, 1)) for lda in (m | 1, m + -m % 4))
         assert odd <= factor * aligned + 1, (m, n)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_gemv_n_of_few_columns(us, cuda, cplx):
+    """One column more than a batch of 32 is no other slice."""
+    f = B.iclblasCgemv if cplx else B.iclblasSgemv
+    A, x, y = buf(3000 * 33, cplx, cuda), buf(33, cplx, cuda), buf(3000, cplx, cuda)
+    t33, t32 = (us(lambda h: f(h, 0, 3000, n, 1.0, A, 3000, x, 1, 0.0, y, 1)) for n in (33, 32))
+    assert t33 <= 1.35 * t32

@@ -34,3 +34,29 @@ def test_unaligned(handle, cuda, m, n, dtype):
             xd, yd = torch.from_numpy(x).to(cuda), torch.from_numpy(y).to(cuda)
             assert f(handle, trans, m, n, 1.25, Ad[shift:], lda, xd, inc, beta, yd, inc) == B.SUCCESS
             assert O.rel_fro(yd.cpu().numpy(), y_ref) <= 1e-5
+
+
+# (the widest single slice, and unaligned columns below two slices)
+@pytest.mark.parametrize("trans,m,n,lda", [(0, 700, 127, 700), (0, 2001, 127, 2001), (1, 2047, 6100, 2047)])
+def test_first_call_captured(cuda, trans, m, n, lda):
+    """Calls that need no scratch may be a handle's first, and captured."""
+    import torch
+    rng = np.random.default_rng(n)
+    xl, yl = (n, m) if trans == 0 else (m, n)
+    A, x, y = (O.colmajor(r, c, r, rng) for r, c in ((lda, n), (xl, 1), (yl, 1)))
+    want = y.copy()
+    O.sgemv(trans, m, n, 1.25, A, lda, x, 1, 0.5, want, 1)
+    Ad, xd, yd = (torch.from_numpy(v).to(cuda) for v in (A, x, y))
+    h = B.Handle()
+    s = torch.cuda.Stream()
+    h.set_stream(s)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        status = B.iclblasSgemv(h, trans, m, n, 1.25, Ad, lda, xd, 1, 0.5, yd, 1)
+    assert status == B.SUCCESS
+    g.replay()
+    torch.cuda.synchronize()
+    assert O.rel_fro(yd.cpu().numpy(), want) <= 1e-5
+    del g
+    h.destroy()
