@@ -13,139 +13,26 @@
 // threads (the driver copies them on one thread: 11 to 14 GB/s; a product of
 // 1024 x 768 x 512 on host arrays takes 287 us so, 510 through the driver).
 #include <algorithm>
-#include <atomic>
-#include <chrono>
-#include <condition_variable>
 #include <cstring>
 #include <mutex>
 #include <thread>
 #include <vector>
 
+#include "copy_pool.h"
 #include "internal.h"
 
 namespace iclb {
 namespace {
 
 constexpr size_t kBounceBytes = (size_t)32 << 20;   // one bounce buffer
-constexpr size_t kSliceBytes = (size_t)128 << 10;   // least host-copy work per thread and copy
-constexpr int kSpinUs = 50;                         // a worker looks for the next copy this long before it sleeps
 
-inline void cpu_pause()
+// The process-wide pool of copy threads, started on first use.
+CopyPool& copy_pool()
 {
-#if defined(__x86_64__)
-    __builtin_ia32_pause();
-#else
-    std::this_thread::yield();
-#endif
+    static CopyPool pool(std::min(8u, std::max(2u, std::thread::hardware_concurrency()) / 2),
+                         [](void* dst, const void* src, size_t bytes) { std::memcpy(dst, src, bytes); });
+    return pool;
 }
-
-// Process-wide pool of host threads for memcpy calls (started on first use).
-// One copy at a time is shared out: the slices of it that are still to be
-// done are handed out by an atomic counter, to the workers that come and to
-// the caller itself, so the caller never waits for a thread that has yet to
-// wake up, and no lock is taken on the way (with a locked queue, eight
-// workers waking up for a 1 MiB copy cost more than the copy).  A caller that
-// finds the pool taken copies on its own thread.  Workers spin for kSpinUs
-// after a copy: the next chunk of the same call finds them awake.
-class CopyPool {
-public:
-    static CopyPool& get()
-    {
-        static CopyPool pool;
-        return pool;
-    }
-
-    void copy(void* dst, const void* src, size_t bytes)
-    {
-        const size_t n = std::min<size_t>(workers_.size() + 1, (bytes + kSliceBytes - 1) / kSliceBytes);
-        std::unique_lock<std::mutex> mine(owner_, std::defer_lock);
-        if (n <= 1 || !mine.try_lock()) {
-            std::memcpy(dst, src, bytes);
-            return;
-        }
-        dst_ = (char*)dst;
-        src_ = (const char*)src;
-        bytes_ = bytes;
-        per_ = ((bytes + n - 1) / n + 63) & ~(size_t)63;
-        slices_ = (int)((bytes + per_ - 1) / per_);
-        next_.store(0);
-        done_.store(0);
-        open_.store(true);      // workers may enter
-        copies_.fetch_add(1);   // and know there is something new
-        if (sleeping_.load() > 0) {
-            std::lock_guard<std::mutex> lock(mu_);
-            cv_.notify_all();
-        }
-        work();
-        while (done_.load() < slices_) cpu_pause();
-        // no worker may look at this copy once the next one is set up
-        open_.store(false);
-        while (inside_.load() > 0) cpu_pause();
-    }
-
-    ~CopyPool()
-    {
-        {
-            std::lock_guard<std::mutex> lock(mu_);
-            stop_.store(true);
-        }
-        cv_.notify_all();
-        for (auto& t : workers_) t.join();
-    }
-
-private:
-    CopyPool()
-    {
-        const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
-        const unsigned n = std::min(8u, hw / 2);
-        for (unsigned i = 0; i < n; ++i) workers_.emplace_back([this] { run(); });
-    }
-
-    void work()
-    {
-        for (int i = next_.fetch_add(1); i < slices_; i = next_.fetch_add(1)) {
-            const size_t off = (size_t)i * per_;
-            std::memcpy(dst_ + off, src_ + off, std::min(per_, bytes_ - off));
-            done_.fetch_add(1);
-        }
-    }
-
-    void run()
-    {
-        unsigned seen = 0;
-        for (;;) {
-            const auto t0 = std::chrono::steady_clock::now();
-            while (copies_.load() == seen && !stop_.load() &&
-                   std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(kSpinUs))
-                cpu_pause();
-            if (copies_.load() == seen) {
-                std::unique_lock<std::mutex> lock(mu_);
-                sleeping_.fetch_add(1);
-                cv_.wait(lock, [&] { return stop_.load() || copies_.load() != seen; });
-                sleeping_.fetch_sub(1);
-            }
-            if (stop_.load()) return;
-            seen = copies_.load();
-            // the caller closes the copy and then waits for inside_ == 0: a
-            // worker that still finds it open is waited for
-            inside_.fetch_add(1);
-            if (open_.load()) work();
-            inside_.fetch_sub(1);
-        }
-    }
-
-    std::mutex owner_;  // held by the caller whose copy is shared out
-    char* dst_ = nullptr;
-    const char* src_ = nullptr;
-    size_t bytes_ = 0, per_ = 0;
-    int slices_ = 0;
-    std::atomic<int> next_{0}, done_{0}, inside_{0}, sleeping_{0};
-    std::atomic<unsigned> copies_{0};
-    std::atomic<bool> open_{false}, stop_{false};
-    std::mutex mu_;
-    std::condition_variable cv_;
-    std::vector<std::thread> workers_;
-};
 
 // Process-wide pool of pinned chunks for small copies: at most kMaxChunks, made
 // as they are needed, given back to the system when the last handle goes.  A
@@ -229,7 +116,7 @@ void pinned_release() { PinnedPool::get().release(); }
 void* pinned_take() { return PinnedPool::get().take(); }
 void pinned_give(void* chunk) { PinnedPool::get().give(chunk); }
 
-void host_copy(void* dst, const void* src, size_t bytes) { CopyPool::get().copy(dst, src, bytes); }
+void host_copy(void* dst, const void* src, size_t bytes) { copy_pool().copy(dst, src, bytes); }
 
 cudaError_t copy_pageable_h2d(iclblasHandle_t h, void* dst, const void* src, size_t bytes)
 {
