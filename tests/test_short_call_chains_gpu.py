@@ -96,3 +96,58 @@ def test_after_copies_and_fills_in_a_graph(handle, cuda, mode):
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("n,lda,inc", [(64, 64, 1), (301, 303, 1), (1100, 1101, 2), (1024, 1024, 1)])
+def test_complex_chain(handle, cuda, n, lda, inc, graph):
+    """The same of the complex routines."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n + inc)
+
+    def rand(*shape):
+        return torch.view_as_complex(torch.rand(*shape, 2, generator=gen, device="cuda") * 2 - 1)
+
+    A, v0 = rand(n, lda) / n ** 0.5, rand(n * inc)
+    handle.set_math_mode(0)
+    steps = 6
+
+    def chain(v, w, r, q, M, sync):
+        def done(status):
+            assert status == B.SUCCESS
+            if sync:
+                assert handle.synchronize() == B.SUCCESS
+        for i in range(steps):
+            done(B.iclblasCgemv(handle, i % 3, n, n, 1.0, A, lda, v, inc, 0.0, w, inc))
+            done(B.iclblasCaxpy(handle, n, 0.5j, v, inc, w, inc))
+            done(B.iclblasCscal(handle, n, 0.75, w, inc))
+            done(B.iclblasCdotc(handle, n, v, inc, w, inc, r[i:]))
+            done(B.iclblasScnrm2(handle, n, w, inc, q[i:]))
+            done(B.iclblasCgemm(handle, 2 * (i % 2), 0, n, 1, n, 1.0, A, lda, w, n, 0.0, M[i], n))
+            v, w = w, v
+
+    def bufs():
+        return (v0.clone(), torch.zeros_like(v0), torch.zeros(steps, dtype=v0.dtype, device="cuda"),
+                torch.zeros(steps, device="cuda"), torch.zeros(steps, n, dtype=v0.dtype, device="cuda"))
+
+    want, got = bufs(), bufs()
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle.set_stream(s)
+    with torch.cuda.stream(s):
+        chain(*want, True)
+        if graph:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                chain(*got, False)
+            for _ in range(3):
+                got[0].copy_(v0)
+                for t in got[1:]:
+                    t.zero_()
+                g.replay()
+        else:
+            chain(*got, False)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    handle.set_stream(torch.cuda.current_stream())
