@@ -915,18 +915,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 //   - when nonzero entries of its inverse lie below FP32's normal range and
 //     what they lack could show in an entry of x.
 // Measured (us; before: one substitution warp per block and a flag per
-// block): complex n = 3001 512, 88; n = 4096 88; n = 512 25; real with an odd
-// leading dimension n = 4096 67, n = 16384 354.  A step of the chain takes
-// 0.85 us (real) or 1.15 (complex).  Measured and dropped: W = inv(D) T formed
+// block): complex n = 3001 512, 84 to 89; n = 4096 603, 83; n = 512 78, 23;
+// real with an odd leading dimension n = 4096 494, 67, n = 16384 354.  A step of
+// the chain takes 0.85 us (real) or 1.15 (complex).  Measured and dropped: W = inv(D) T formed
 // beforehand for a one-product step (8 us more before the chain starts, the
 // step no shorter: the hand-off, not the products, sets it).
 constexpr int NB = 64;
 constexpr int kBStages = 3;
 // CTAs of a cluster: up to 16 for solves of at most kBWide blocks (fewer
-// hand-offs through global memory: real n = 2048 41 us with 8, 38 with 16,
-// n = 3072 55 and 50, complex n = 3072 68 and 66), up to 8 for longer ones,
-// whose clusters of 16 wait for GPCs with 16 free SMs (complex n = 4096 89
-// and 93, real n = 8192 172 and 179).
+// hand-offs through global memory; us with 8 and with 16: real n = 2048 38.5,
+// 37.0, 3072 52.5, 51.0, complex n = 1024 31.5, 30.1, 3072 66.8, 65.5), up to 8
+// for longer ones, whose clusters of 16 wait for GPCs with 16 free SMs (real n
+// = 3584 58.9, 60.5, complex 74.9, 77.0; equal from 4096 on).
 constexpr int kBCluster = 16, kBWide = 48;
 constexpr float kBGrowth = 1024.f;
 
@@ -1531,34 +1531,32 @@ cudaError_t strsv_tma(iclblasHandle_t h, int uplo, int trans, int diag, int n, c
     unsigned* ticket = h->ws.counters;
     unsigned* epoch_word = h->ws.counters + kCounterWords - 1;
     used = true;
-    if (nb > 1) {
-        // the largest cluster size, 8 down to 2, for which every cluster of
-        // the launch is resident at once (sizes need not be powers of two: a
-        // GPC that holds two clusters of 8 may hold three of 6); if none is,
-        // clusters of 8 (the most DSMEM hand-offs), else one CTA per block
-        const int caps[9] = {0,
-                             0,
-                             strsv_cluster_capacity<2>(h->device, smem),
-                             strsv_cluster_capacity<3>(h->device, smem),
-                             strsv_cluster_capacity<4>(h->device, smem),
-                             strsv_cluster_capacity<5>(h->device, smem),
-                             strsv_cluster_capacity<6>(h->device, smem),
-                             strsv_cluster_capacity<7>(h->device, smem),
-                             strsv_cluster_capacity<8>(h->device, smem)};
-        int cl = 0;
-        for (int c = 8; c >= 2 && !cl; --c)
-            if (caps[c] > 0 && caps[c] * c >= nb) cl = c;
-        if (!cl && caps[8] > 0) cl = 8;
-        switch (cl) {
-        case 8: return strsv_launch<8>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 7: return strsv_launch<7>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 6: return strsv_launch<6>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 5: return strsv_launch<5>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 4: return strsv_launch<4>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 3: return strsv_launch<3>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        case 2: return strsv_launch<2>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
-        default: break;
-        }
+    // the largest cluster size, 8 down to 2, for which every cluster of
+    // the launch is resident at once (sizes need not be powers of two: a
+    // GPC that holds two clusters of 8 may hold three of 6); if none is,
+    // clusters of 8 (the most DSMEM hand-offs), else one CTA per block
+    const int caps[9] = {0,
+                         0,
+                         strsv_cluster_capacity<2>(h->device, smem),
+                         strsv_cluster_capacity<3>(h->device, smem),
+                         strsv_cluster_capacity<4>(h->device, smem),
+                         strsv_cluster_capacity<5>(h->device, smem),
+                         strsv_cluster_capacity<6>(h->device, smem),
+                         strsv_cluster_capacity<7>(h->device, smem),
+                         strsv_cluster_capacity<8>(h->device, smem)};
+    int cl = 0;
+    for (int c = 8; c >= 2 && !cl; --c)
+        if (caps[c] > 0 && caps[c] * c >= nb) cl = c;
+    if (!cl && caps[8] > 0) cl = 8;
+    switch (cl) {
+    case 8: return strsv_launch<8>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 7: return strsv_launch<7>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 6: return strsv_launch<6>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 5: return strsv_launch<5>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 4: return strsv_launch<4>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 3: return strsv_launch<3>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    case 2: return strsv_launch<2>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
+    default: break;
     }
     return strsv_launch<1>(h, smem, nb, map, n, lower_op, op, unit, x, incx, pub, ticket, epoch_word);
 }
@@ -1598,7 +1596,6 @@ template <class T, bool HALF>
 cudaError_t trsv_block(iclblasHandle_t h, int uplo, int trans, int diag, int n, const T* A, int lda, T* x, int incx)
 {
     const int nb = (n + NB - 1) / NB;
-    if (nb > kCounterWords / 2 - 1) return cudaErrorInvalidValue;
     const int op = trans == ICLBLAS_OP_N ? 0 : (trans == ICLBLAS_OP_C && sizeof(T) == sizeof(cfloat)) ? 2 : 1;
     const bool lower = uplo == ICLBLAS_FILL_MODE_LOWER;
     const int lower_op = (op == 0) ? lower : !lower;
@@ -1682,9 +1679,11 @@ cudaError_t strsv(iclblasHandle_t h, int uplo, int trans, int diag, int n, const
 {
     if (n <= kSmall) return trsv_small<float>(h, uplo, trans, diag, n, A, lda, x, incx);
     // short solves are bound by the time to the first block's inverse, which
-    // 64-row blocks have sooner (n = 512: 19 us against 30 with 128-row
-    // blocks, n = 1024 25 and 34, n = 2048 41 and 42, n = 3072 55 and 52)
-    if (n > 2048) {
+    // 64-row blocks have sooner; 128-row blocks make half the steps (us, 64-
+    // and 128-row blocks, op N: n = 512 17.7, 27.4, 1024 22.9, 31.0, 2048 37.0,
+    // 39.8, 2560 46.2, 46.0, 3072 51.0, 49.6, 4096 65, 59; op T: 2560 45.0,
+    // 47.5, 3072 51.1, 52.5, 3584 60, 58)
+    if (n > 2560) {
         bool used = false;
         cudaError_t e = strsv_tma(h, uplo, trans, diag, n, A, lda, x, incx, used);
         if (e != cudaSuccess || used) return e;

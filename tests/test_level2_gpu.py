@@ -144,11 +144,12 @@ def test_trsv_device_pointers(handle, cuda):
     assert O.rel_fro(xd.cpu().numpy(), x_ref) <= TOL
 
 
-@pytest.mark.parametrize("n", [64, 130, 2048, 3001])
+@pytest.mark.parametrize("n", [64, 130, 2048, 2560, 2561, 2688, 3001, 4100])
 @pytest.mark.parametrize("uplo,trans", [(0, 0), (1, 0), (0, 1), (1, 2)])
 def test_strsv_tma_path_padded_lda(handle, n, uplo, trans):
-    """lda a multiple of 4 above n (the TMA-staged path), stride 2, three
-    calls in a row on one handle (each call a new epoch)."""
+    """lda a multiple of 4 above n (the TMA-staged path above n = 2560, the other
+    two kernels up to there), stride 2, three calls in a row on one handle (each
+    call a new epoch)."""
     rng = np.random.default_rng(n + 7 * uplo + trans)
     lda = (n + 4 + 3) // 4 * 4
     for diag in (0, 1, 0):

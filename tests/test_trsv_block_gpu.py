@@ -53,6 +53,22 @@ def test_block_edges(handle, n, dtype):
                     assert np.array_equal(x[1::2], x_ref[1::2])
 
 
+# more than 48 blocks: clusters of at most 8
+@pytest.mark.parametrize("n", [3072, 3073, 4100])
+@pytest.mark.parametrize("dtype", [np.float32, np.complex64])
+def test_long_solves(handle, n, dtype):
+    rng = np.random.default_rng(n)
+    lda = n | 1
+    for uplo in (0, 1):
+        A = tri(n, lda, uplo == 1, rng, dtype)
+        for trans in (0, 1, 2):
+            x = O.colmajor(n, 1, n, rng, dtype)
+            x_ref = x.copy()
+            want(dtype, uplo, trans, 0, n, A, lda, x_ref, 1)
+            assert solve(handle, dtype, uplo, trans, 0, n, A, lda, x, 1) == B.SUCCESS
+            assert O.rel_fro(x, x_ref) <= TOL
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.complex64])
 @pytest.mark.parametrize("uplo", [0, 1])
 def test_non_finite(handle, dtype, uplo):
