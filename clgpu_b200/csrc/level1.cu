@@ -574,7 +574,6 @@ cudaError_t saxpy(iclblasHandle_t h, int n, float alpha, const float* x, int inc
         return pdl_launch(dependent(n) ? saxpy_strided<true> : saxpy_strided<false>, dim3(l1_grid(h, n)), kThreads, 0,
                           h->stream, dependent(n), n, alpha, x, incx, y, incy);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t sscal(iclblasHandle_t h, int n, float alpha, float* x, int incx)
@@ -586,7 +585,6 @@ cudaError_t sscal(iclblasHandle_t h, int n, float alpha, float* x, int incx)
         return pdl_launch(dependent(n) ? sscal_strided<true> : sscal_strided<false>, dim3(l1_grid(h, n)), kThreads, 0,
                           h->stream, dependent(n), n, alpha, x, incx);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t caxpy(iclblasHandle_t h, int n, cfloat alpha, const cfloat* x, int incx, cfloat* y, int incy)
@@ -633,12 +631,11 @@ cudaError_t sreduce(iclblasHandle_t h, Red op, int n, const float* x, int incx, 
                               n, x, incx, y, incy, partials, ctr, result);                                       \
     } while (0)
     switch (op) {
-    case Red::Dot: if (vec) LAUNCH(Red::Dot, true); else LAUNCH(Red::Dot, false); break;
-    case Red::Asum: if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false); break;
-    case Red::Nrm2: if (vec) LAUNCH(Red::Nrm2, true); else LAUNCH(Red::Nrm2, false); break;
+    case Red::Dot: if (vec) LAUNCH(Red::Dot, true); else LAUNCH(Red::Dot, false);
+    case Red::Asum: if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false);
+    default: if (vec) LAUNCH(Red::Nrm2, true); else LAUNCH(Red::Nrm2, false);
     }
 #undef LAUNCH
-    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- SDOT without allocation
@@ -763,7 +760,6 @@ cudaError_t creduce_real(iclblasHandle_t h, Red op, int n, const cfloat* x, int 
     if (op == Red::Asum) { if (vec) LAUNCH(Red::Asum, true); else LAUNCH(Red::Asum, false); }
     else { if (vec) LAUNCH(Red::Nrm2, true); else LAUNCH(Red::Nrm2, false); }
 #undef LAUNCH
-    return cudaGetLastError();
 }
 
 cudaError_t cdot(iclblasHandle_t h, bool conj, int n, const cfloat* x, int incx, const cfloat* y, int incy,
@@ -788,7 +784,6 @@ cudaError_t cdot(iclblasHandle_t h, bool conj, int n, const cfloat* x, int incx,
     if (conj) { if (vec) LAUNCH(true, true); else LAUNCH(true, false); }
     else { if (vec) LAUNCH(false, true); else LAUNCH(false, false); }
 #undef LAUNCH
-    return cudaGetLastError();
 }
 
 namespace {
@@ -813,7 +808,6 @@ cudaError_t iamax_impl(iclblasHandle_t h, int n, const T* x, int incx, int* resu
     } while (0)
     if (vec) LAUNCH(true); else LAUNCH(false);
 #undef LAUNCH
-    return cudaGetLastError();
 }
 }  // namespace
 
