@@ -374,20 +374,25 @@ cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alp
 namespace {
 // Estimated SM cycles of a product: a lone tile on an SM takes alone0 (its
 // first copies and its stores) + alone * k, bound by latency; several take
-// each0 + each * k apiece, bound by throughput.  Measured from grids of 1 to
-// 500 tiles an SM at k = 4, 100 and 2000.  (Without the constant terms, us,
-// the tile taken so and the one of the table: 1000 x 2000 x 4 10.5, 8.0; 1400 x 700 x 4
-// 7.1, 4.7; 1000 x 2000 x 48 14.6, 11.6.)
+// each0 + full * (the part of the tiles inside C) + each * k apiece, bound by
+// throughput.  Fitted, near the figures of grids of one to 500 full tiles an
+// SM, to the times of every tile at 1481 real and 1478 complex shapes of 1 to a
+// million rows or columns and k of 2 to 4000: the tile so picked costs 0.24 %
+// (complex 0.34 %) more than the fastest one on average, without the constant
+// terms and `full` it was 3.0 % (1.1 %), and 60 % at 1000000 x 1 x 4 or 30 % at
+// 1000 x 2000 x 4.
 struct TileCost {
     int bm, bn;
-    double alone0, alone, each0, each;
+    double alone0, alone, each0, full, each;
 };
-constexpr TileCost kRealTiles[] = {{128, 128, 10000, 207, 10400, 190},
-                                   {128, 64, 8200, 120, 5600, 104},
-                                   {64, 64, 8800, 123, 2860, 55},
-                                   {32, 32, 600, 41, 743, 21},
-                                   {16, 16, 300, 26, 397, 10.5}};
-constexpr TileCost kCplxTiles[] = {{64, 64, 5900, 228, 5200, 191}, {32, 32, 800, 76, 1580, 53}, {16, 16, 300, 50, 465, 20}};
+constexpr TileCost kRealTiles[] = {{128, 128, 15100, 193, 523, 11900, 200},
+                                   {128, 64, 9000, 128, 709, 6300, 110},
+                                   {64, 64, 9320, 124, 296, 4210, 67.3},
+                                   {32, 32, 2410, 43.9, 200, 476, 22},
+                                   {16, 16, 293, 27.8, 270, 129, 10.2}};
+constexpr TileCost kCplxTiles[] = {{64, 64, 7410, 244, 333, 5040, 213},
+                                   {32, 32, 1600, 71, 309, 1050, 58.4},
+                                   {16, 16, 263, 42.8, 140, 253, 19.1}};
 
 // the tile of the least estimated time, of those whose columns fit the grid's
 // 65,535 blocks in y (the largest tile of a table, the first, may not: n above
@@ -401,7 +406,9 @@ int pick_tile(const TileCost (&c)[N], int sms, int m, int n, int k, bool tri)
         const long tm = ceil_div(m, c[q].bm), tn = ceil_div(n, c[q].bn);
         if (q > 0 && tn > 65535) continue;
         const long tiles = tri ? (tm * tn + std::max(tm, tn)) / 2 : tm * tn;
-        const double t = std::max(c[q].alone0 + c[q].alone * k, ceil_div(tiles, sms) * (c[q].each0 + c[q].each * k));
+        const double inside = (double)m * n / ((double)tm * c[q].bm * tn * c[q].bn);
+        const double t = std::max(c[q].alone0 + c[q].alone * k,
+                                  ceil_div(tiles, sms) * (c[q].each0 + c[q].full * inside + c[q].each * k));
         if (q == 0 || t < best_t) {
             best = q;
             best_t = t;
