@@ -41,27 +41,27 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 // Launch shape of a reduction over n elements in `units` per-thread units.
 // Short vectors take one CTA of 1024 threads, which holds the whole sum: the
 // partials, fences and ticket between CTAs cost about 2 us, half of the call.
-// One SM then does all the reading, so how short depends on what an element
-// costs it: `bytes` are those of the 32-byte sectors that hold the operands.
-// Several CTAs against one, us, at the ends of the range: unit stride n =
-// 16384 sdot 3.7, 3.0, isamax 3.9, 2.1, cdotc (192 KiB) n = 12288 4.2, 4.2;
-// stride 17 sdot n = 3000 3.8, 3.5, 4096 3.8, 4.0, 16384 3.8, 10.6; complex
-// elements one at a time (112 KiB) unit stride, not aligned, cdotc n = 8192
-// 4.2, 3.7, 12000 4.2, 4.6, stride 17 n = 1024 4.5, 3.3, 2048 4.4, 4.8, 16384
-// 4.5, 26.3.
+// One SM then does all the reading, so how short depends on the 128-byte lines
+// that the operands touch and, for complex elements, on the work an element
+// is.  Several CTAs against one, us: sdot n = 16384 unit stride 3.7, 3.0,
+// stride 2 3.6, 3.8, stride 17 n = 3000 3.8, 3.5, 4096 3.8, 4.0, 16384 3.8,
+// 10.6; isamax unit stride 16384 3.9, 2.1; cdotc aligned n = 8192 4.3, 3.5,
+// 12000 4.0, 4.4, an element at a time 8192 4.2, 3.7, 12000 4.2, 4.6, stride 17
+// n = 1024 4.5, 3.3, 2048 4.4, 4.8, 16384 4.5, 26.3; icamax an element at a time
+// 8192 3.9, 3.3, 12000 3.7, 4.3.
 struct RedShape {
     int grid, threads;
 };
+// incy: stride of the second operand, 0 for none
 template <class T>
-__host__ long sector_bytes(long n, int inc)
+__host__ RedShape red_shape(iclblasHandle_t h, long n, long units, int per_sm, int incx, int incy = 0)
 {
-    return n * std::min(32L, (long)inc * (long)sizeof(T));
-}
-template <class T>
-__host__ RedShape red_shape(iclblasHandle_t h, long n, long units, long bytes, int per_sm)
-{
-    const bool one_at_a_time = sizeof(T) == sizeof(cfloat) && units == n;
-    if (n <= 16384 && bytes <= (one_at_a_time ? 112 : 192) * 1024L)
+    const bool dot = incy != 0, one_at_a_time = units == n;
+    const long most = sizeof(T) == sizeof(float) ? 16384
+                      : one_at_a_time            ? (dot ? 8192 : 10240)
+                                                 : (dot ? 10240 : 16384);
+    auto bytes = [&](long inc) { return n * std::min(128L, inc * (long)sizeof(T)); };
+    if (n <= most && bytes(incx) + bytes(incy) <= 3400 * 128)
         return {1, (int)std::min(1024L, (units + 31) / 32 * 32)};
     return {l1_grid(h, units, per_sm), kThreads};
 }
@@ -615,8 +615,8 @@ cudaError_t sreduce(iclblasHandle_t h, Red op, int n, const float* x, int incx, 
                     float* result)
 {
     const bool vec = incx == 1 && aligned16(x) && (op != Red::Dot || (incy == 1 && aligned16(y)));
-    const long bytes = sector_bytes<float>(n, incx) + (op == Red::Dot ? sector_bytes<float>(n, incy) : 0);
-    const RedShape g = red_shape<float>(h, n, vec ? ((long)n + 3) / 4 : n, bytes, op == Red::Asum ? 6 : 8);
+    const RedShape g = red_shape<float>(h, n, vec ? ((long)n + 3) / 4 : n, op == Red::Asum ? 6 : 8, incx,
+                                        op == Red::Dot ? incy : 0);
     double* partials = nullptr;
     if (g.grid > 1 && !(partials = (double*)scratch(h, sizeof(double) * (size_t)g.grid)))
         return cudaErrorMemoryAllocation;
@@ -715,8 +715,7 @@ cudaError_t noalloc_scratch_addr(int device, SdotNoAllocScratch** out)
 cudaError_t sdot_noalloc(iclblasHandle_t h, int n, const float* x, int incx, const float* y, int incy, float* result)
 {
     const bool vec = incx == 1 && aligned16(x) && incy == 1 && aligned16(y);
-    const RedShape g = red_shape<float>(h, n, vec ? ((long)n + 3) / 4 : n,
-                                        sector_bytes<float>(n, incx) + sector_bytes<float>(n, incy), 8);
+    const RedShape g = red_shape<float>(h, n, vec ? ((long)n + 3) / 4 : n, 8, incx, incy);
     if (g.grid > kSdotNoAllocMaxBlocks) return cudaErrorNotSupported;
     SdotNoAllocScratch* sc = nullptr;
     cudaError_t e = noalloc_scratch_addr(h->device, &sc);
@@ -743,7 +742,7 @@ cudaError_t sdot_noalloc(iclblasHandle_t h, int n, const float* x, int incx, con
 cudaError_t creduce_real(iclblasHandle_t h, Red op, int n, const cfloat* x, int incx, float* result)
 {
     const bool vec = incx == 1 && aligned16(x);
-    const RedShape g = red_shape<cfloat>(h, n, vec ? ((long)n + 1) / 2 : n, sector_bytes<cfloat>(n, incx), 8);
+    const RedShape g = red_shape<cfloat>(h, n, vec ? ((long)n + 1) / 2 : n, 8, incx);
     double* partials = nullptr;
     if (g.grid > 1 && !(partials = (double*)scratch(h, sizeof(double) * (size_t)g.grid)))
         return cudaErrorMemoryAllocation;
@@ -766,8 +765,7 @@ cudaError_t cdot(iclblasHandle_t h, bool conj, int n, const cfloat* x, int incx,
                  cfloat* result)
 {
     const bool vec = incx == 1 && incy == 1 && aligned16(x) && aligned16(y);
-    const RedShape g = red_shape<cfloat>(h, n, vec ? ((long)n + 1) / 2 : n,
-                                         sector_bytes<cfloat>(n, incx) + sector_bytes<cfloat>(n, incy), 8);
+    const RedShape g = red_shape<cfloat>(h, n, vec ? ((long)n + 1) / 2 : n, 8, incx, incy);
     double* partials = nullptr;
     if (g.grid > 1 && !(partials = (double*)scratch(h, 2 * sizeof(double) * (size_t)g.grid)))
         return cudaErrorMemoryAllocation;
@@ -791,8 +789,7 @@ template <class T, bool MIN>
 cudaError_t iamax_impl(iclblasHandle_t h, int n, const T* x, int incx, int* result)
 {
     const bool vec = incx == 1 && aligned16(x);
-    const RedShape g = red_shape<T>(h, n, vec ? ((long)n + (16 / sizeof(T)) - 1) / (16 / sizeof(T)) : n,
-                                    sector_bytes<T>(n, incx), 6);
+    const RedShape g = red_shape<T>(h, n, vec ? ((long)n + (16 / sizeof(T)) - 1) / (16 / sizeof(T)) : n, 6, incx);
     Cand* partials = nullptr;
     if (g.grid > 1 && !(partials = (Cand*)scratch(h, sizeof(Cand) * (size_t)g.grid)))
         return cudaErrorMemoryAllocation;

@@ -11,7 +11,7 @@ F = np.float32
 
 
 @pytest.mark.parametrize("inc,shift", [(1, 0), (1, 1), (2, 0), (17, 0)])
-@pytest.mark.parametrize("n", [1791, 1793, 3072, 3073, 3585, 6145, 7169, 12288, 12289, 14337, 16384, 16385])
+@pytest.mark.parametrize("n", [1700, 1701, 3200, 3201, 3400, 3401, 6400, 6401, 8192, 8193, 10240, 10241, 16384, 16385])
 def test_reductions(handle, cuda, n, inc, shift):
     import torch
     handle.set_stream(torch.cuda.current_stream())
