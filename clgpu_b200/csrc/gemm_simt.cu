@@ -202,6 +202,16 @@ struct TileCopy {
     }
 };
 
+// Tiles of tile column bn that meet the lower (tri 1) or upper (2) triangle of
+// a square matrix of tm tile rows: those from row tile bn * BN / BM on, or up to
+// the one of the column's last row.
+template <int BM, int BN>
+__host__ __device__ constexpr int tri_tiles(int tri, int tm, int bn)
+{
+    const int last = (bn * BN + BN - 1) / BM + 1;
+    return tri == 1 ? tm - bn * BN / BM : (last < tm ? last : tm);
+}
+
 // HALF: complex operands at 4 modulo 8.  CONJ: an operand may be conjugated
 // (choosing inside the k loop costs 12 selects per 32 complex products, and a
 // fifth of the time: 4096 x 4096 x 2048 NN 6656 us with, 5430 without).
@@ -219,7 +229,22 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int WX = TX / 8;  // warps along n
     const int ty = (warp / WX) * 4 + lane / 8, tx = (warp % WX) * 8 + lane % 8;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    int bm = blockIdx.x, bn = blockIdx.y;
+    if (tri != 0) {
+        // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed, by
+        // a row of blocks for the tiles that meet it, column after column
+        // (blocks of the others took places on the SMs too, and the rest lay
+        // unevenly: ssyrk of 2000 x 3000, 136 tiles of 128 x 128, 583 to 647 us with
+        // them, 314 to 348 without)
+        const int tm = (m + BM - 1) / BM;
+        for (bn = 0;; ++bn) {
+            const int c = tri_tiles<BM, BN>(tri, tm, bn);
+            if (bm < c) break;
+            bm -= c;
+        }
+        if (tri == 1) bm += bn * BN / BM;
+    }
+    const int m0 = bm * BM, n0 = bn * BN;
     pdl_wait();
     PDL_FRESH(A);
     PDL_FRESH(B);
@@ -228,9 +253,6 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     // an SM before this one's end, so that an even grid of that launch came to
     // lie unevenly (1000 x 2000 x 2000, two 128 x 64 tiles an SM: 328 us in a
     // chain of such calls, 229 without; 512^3 the same either way)
-    // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed;
-    // tiles wholly outside it have no work
-    if ((tri == 1 && m0 + BM - 1 < n0) || (tri == 2 && m0 > n0 + BN - 1)) return;
     const bool a_conj = ta == ICLBLAS_OP_C, b_conj = tb == ICLBLAS_OP_C;
     const TileCopy<T, BM, BK, NT, PA, HALF> ca(A, lda, ta != ICLBLAS_OP_N, m0, m);
     const TileCopy<T, BN, BK, NT, PB, HALF> cb(B, ldb, tb == ICLBLAS_OP_N, n0, n);
@@ -365,6 +387,11 @@ cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alp
         }
     }
     dim3 grid(ceil_div(m, BM), ceil_div(n, BN));
+    if (tri != 0) {
+        unsigned tiles = 0;
+        for (unsigned j = 0; j < grid.y; ++j) tiles += (unsigned)tri_tiles<BM, BN>(tri, (int)grid.x, (int)j);
+        grid = dim3(tiles);
+    }
     return pdl_launch(kern, grid, CF::NT, CF::SMEM, h->stream, 1,
                       ta, tb, m, n, k, alpha, A, (long)lda, B, (long)ldb, beta, C, (long)ldc, tri);
 }
