@@ -215,7 +215,9 @@ __host__ __device__ constexpr int tri_tiles(int tri, int tm, int bn)
 // HALF: complex operands at 4 modulo 8.  CONJ: an operand may be conjugated
 // (choosing inside the k loop costs 12 selects per 32 complex products, and a
 // fifth of the time: 4096 x 4096 x 2048 NN 6656 us with, 5430 without).
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF, bool CONJ>
+// TRI: triangular output (finding the tile at run time cost every product:
+// 512^3 18.4 us without, 21.1 with).
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF, bool CONJ, bool TRI>
 __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     gemm_simt_kernel(int ta, int tb, int m, int n, int k, T alpha, const T* __restrict__ A, long lda,
                      const T* __restrict__ B, long ldb, T beta, T* __restrict__ C, long ldc, int tri)
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     constexpr int WX = TX / 8;  // warps along n
     const int ty = (warp / WX) * 4 + lane / 8, tx = (warp % WX) * 8 + lane % 8;
     int bm = blockIdx.x, bn = blockIdx.y;
-    if (tri != 0) {
+    if constexpr (TRI) {
         // tri 1 / 2: only C's lower (row >= col) / upper triangle is formed, by
         // a row of blocks for the tiles that meet it, column after column
         // (blocks of the others took places on the SMs too, and the rest lay
@@ -253,6 +255,10 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     // an SM before this one's end, so that an even grid of that launch came to
     // lie unevenly (1000 x 2000 x 2000, two 128 x 64 tiles an SM: 328 us in a
     // chain of such calls, 229 without; 512^3 the same either way)
+    // (a triangle's launch is TRI; with this test and the masks at the end left
+    // to run time the other instantiations come out faster: 512^3 18.8 us
+    // without, 18.4 so)
+    if (!TRI && tri != 0) return;
     const bool a_conj = ta == ICLBLAS_OP_C, b_conj = tb == ICLBLAS_OP_C;
     const TileCopy<T, BM, BK, NT, PA, HALF> ca(A, lda, ta != ICLBLAS_OP_N, m0, m);
     const TileCopy<T, BN, BK, NT, PB, HALF> cb(B, ldb, tb == ICLBLAS_OP_N, n0, n);
@@ -370,12 +376,12 @@ __global__ void __launch_bounds__(Cfg<T, BM, BN, BK, TM, TN, ST>::NT, MB)
     }
 }
 
-template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF = false, bool CONJ = false>
+template <class T, int BM, int BN, int BK, int TM, int TN, int ST, int MB, bool HALF = false, bool CONJ = false, bool TRI = false>
 cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alpha, const T* A, int lda, const T* B,
                    int ldb, T beta, T* C, int ldc, int tri)
 {
     using CF = Cfg<T, BM, BN, BK, TM, TN, ST>;
-    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB, HALF, CONJ>;
+    auto kern = gemm_simt_kernel<T, BM, BN, BK, TM, TN, ST, MB, HALF, CONJ, TRI>;
     if (CF::SMEM > 48 * 1024) {
         // the attribute belongs to the current device's copy of the kernel
         static std::atomic<unsigned long long> smem_set{0};
@@ -387,7 +393,7 @@ cudaError_t launch(iclblasHandle_t h, int ta, int tb, int m, int n, int k, T alp
         }
     }
     dim3 grid(ceil_div(m, BM), ceil_div(n, BN));
-    if (tri != 0) {
+    if (TRI) {
         unsigned tiles = 0;
         for (unsigned j = 0; j < grid.y; ++j) tiles += (unsigned)tri_tiles<BM, BN>(tri, (int)grid.x, (int)j);
         grid = dim3(tiles);
@@ -448,7 +454,9 @@ int pick_tile(const TileCost (&c)[N], int sms, int m, int n, int k, bool tri)
 cudaError_t sgemm_simt(iclblasHandle_t h, int ta, int tb, int m, int n, int k, float alpha, const float* A, int lda,
                        const float* B, int ldb, float beta, float* C, int ldc, int tri)
 {
-#define LAUNCH(...) launch<float, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri)
+#define LAUNCH(...)                                                                                               \
+    (tri != 0 ? launch<float, __VA_ARGS__, false, false, true>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, tri) \
+              : launch<float, __VA_ARGS__>(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, 0))
     switch (pick_tile(kRealTiles, h->sm_count, m, n, k, tri != 0)) {
     case 0:
         // 16 x 8 outputs a thread read less shared memory per product, 8 x 8
