@@ -420,7 +420,8 @@ def run_precision_legs(torch, dev, B, n_gemm=8192, trsm_m=8192, trsm_n=4096):
     pp = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pp):
         peaks = json.load(open(pp))
-    bf16_sus = peaks.get("bf16_tflops_sustained")
+    # a handful of calls of milliseconds each runs at full clock: the burst rate bounds them
+    bf16_peak = peaks.get("bf16_tflops")
     fp32_peak = fp32_fma_peak_tflops(torch, dev)
     nprod = {B.MATH_TF32: 1, B.MATH_BF16X3: 3, B.MATH_BF16X6: 6}
     out = {}
@@ -444,14 +445,14 @@ def run_precision_legs(torch, dev, B, n_gemm=8192, trsm_m=8192, trsm_n=4096):
         if mode == B.MATH_PLAIN_FP32:
             return {"bound": "fp32_fma", "peak": round(fp32_peak, 1), "peak_source": "nominal (SMs x 128 x 2 x max clock)",
                     "frac": round(tf / fp32_peak, 3)}
-        if not bf16_sus:
+        if not bf16_peak:
             return None
         ex = nprod[mode] * tf
         # TF32 runs at half the BF16 rate per product
         eff = ex * (2.0 if mode == B.MATH_TF32 else 1.0)
-        return {"bound": "tensor", "executed_tflops": round(ex, 1), "peak": bf16_sus,
-                "peak_source": "measured sustained bf16 (TF32 products counted at twice their cost)",
-                "frac": round(eff / bf16_sus, 3)}
+        return {"bound": "tensor", "executed_tflops": round(ex, 1), "peak": bf16_peak,
+                "peak_source": "measured burst bf16 (TF32 products counted at twice their cost)",
+                "frac": round(eff / bf16_peak, 3)}
 
     names = {B.MATH_PLAIN_FP32: "fp32", B.MATH_TF32: "tf32", B.MATH_BF16X3: "3xbf16", B.MATH_BF16X6: "6xbf16"}
     with B.Handle() as h, torch.cuda.stream(stream), Clocks(dev.index) as clk:

@@ -16,10 +16,11 @@
 // alignment of an operand changes the main loop, no register holds data in
 // flight, and K tiles are under way while earlier ones are multiplied.
 //
-// What bounds it: large products the FMA pipe (ncu at 4096^3: 72-76 % busy,
-// warps waiting for it) together with shared-memory reads (69 %: a 16-byte
-// read costs four passes however many lanes share the address, so 8 x 8
-// outputs a thread spend as many cycles reading as multiplying); small ones
+// What bounds it: large products the FMA pipe (ncu at 4096^3: 75 % busy, warps
+// waiting for it) together with shared-memory reads (47 % with 16 x 8 outputs
+// a thread, 69 % with 8 x 8: a 16-byte read costs four passes however many
+// lanes share the address, so 8 x 8 spend as many cycles reading as
+// multiplying); small ones
 // the latency of one k step times k, since each output sums k in order.
 // Against register-staged tiles of the same shapes (us before, after):
 // 8192 x 8192 x 4096 NN 11981, 11112, TN 11978, 10524; 2000 x 1500 x 3001 TN
