@@ -85,12 +85,14 @@ __device__ __forceinline__ void recip(cfloat d, cfloat& hi, cfloat& lo)
     lo = cfloat{(float)(re * q - (double)hi.re), (float)(-im * q - (double)hi.im)};
 }
 // v / d for 1 / d = hi + lo, right to less than a rounding where nothing
-// leaves the normal range
-__device__ __forceinline__ float times(float v, float hi, float lo) { return fmaf(v, hi, v * lo); }
+// leaves the normal range; an infinite v as hi alone has it (lo may be zero or
+// of the other sign)
+__device__ __forceinline__ float finite_or_0(float v) { return isfinite(v) ? v : 0.f; }
+__device__ __forceinline__ float times(float v, float hi, float lo) { return fmaf(v, hi, finite_or_0(v * lo)); }
 __device__ __forceinline__ cfloat times(cfloat v, cfloat hi, cfloat lo)
 {
-    return cfloat{fmaf(v.re, hi.re, fmaf(-v.im, hi.im, fmaf(v.re, lo.re, -v.im * lo.im))),
-                  fmaf(v.re, hi.im, fmaf(v.im, hi.re, fmaf(v.re, lo.im, v.im * lo.re)))};
+    const float re = finite_or_0(fmaf(v.re, lo.re, -v.im * lo.im)), im = finite_or_0(fmaf(v.re, lo.im, v.im * lo.re));
+    return cfloat{fmaf(v.re, hi.re, fmaf(-v.im, hi.im, re)), fmaf(v.re, hi.im, fmaf(v.im, hi.re, im))};
 }
 
 // One warp solves the nr x nr lower triangle with element (r, k) at
@@ -146,9 +148,9 @@ __device__ __forceinline__ void substitute(const T* D, int sr, int sc, int nr, b
 
 // Solves of up to kSmall rows, a CTA: the triangle goes to shared memory, the
 // first warp substitutes.  R: rows of a lane.
-// Measured (us, 64-row block kernel and this one): real n = 1 8.5, 2.0, n = 64
-// 12.4, 5.7, n = 128 16.4, 13.3; complex n = 1 12.5, 2.3, n = 64 16.9, 6.7,
-// n = 128 18.2, 15.3; n = 129 14.9 and 19.7 in the block kernel.
+// Measured (us, 64-row block kernel and this one): real n = 1 8.3, 2.1, n = 64
+// 12.3, 6.1, n = 128 16.4, 14.0; complex n = 1 12.5, 2.2, n = 64 17.1, 6.7,
+// n = 128 18.8, 15.9; n = 129 14.9 and 19.7 in the block kernel.
 constexpr int kSmall = 128;
 template <class T, int R>
 __global__ void __launch_bounds__(kThreads) trsv_small_kernel(int n, int lower_op, int op, int unit,
