@@ -148,9 +148,11 @@ __device__ __forceinline__ void substitute(const T* D, int sr, int sc, int nr, b
 
 // Solves of up to kSmall rows, a CTA: the triangle goes to shared memory, the
 // first warp substitutes.  R: rows of a lane.
-// Measured (us, 64-row block kernel and this one): real n = 1 8.3, 2.1, n = 64
-// 12.3, 6.1, n = 128 16.4, 14.0; complex n = 1 12.5, 2.2, n = 64 17.1, 6.7,
-// n = 128 18.8, 15.9; n = 129 14.9 and 19.7 in the block kernel.
+// Measured in one run (us, 64-row block kernel and this one): real n = 1 8.2,
+// 2.2, n = 64 12.3, 6.1, n = 96 13.9, 11.6, n = 128 13.9, 14.0; complex n = 1
+// 12.5, 2.3, n = 64 17.0, 6.7, n = 128 18.8, 15.9.  The line: at 128 real rows
+// the two are level, and the substitution grows by the row, the blocks do not
+// (n = 129 14.4 and 19.2 there).
 constexpr int kSmall = 128;
 template <class T, int R>
 __global__ void __launch_bounds__(kThreads) trsv_small_kernel(int n, int lower_op, int op, int unit,
