@@ -568,13 +568,17 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
                                                                  rps, partial, h->ws.counters)
     if (conj) { if (vec) LAUNCH(true, true, 1); else LAUNCH(true, false, 1); return cudaGetLastError(); }
     if constexpr (sizeof(T) == sizeof(float)) {
-        // batches of loads, unless many columns keep the SMs busy and most of a
-        // column's last batch would be empty: 1025 x 30000 69 us with one load
-        // at a time, 31 in batches, 100 x 100 2.5, 1.9, 100 x 30000 9.3, 8.8; but
-        // 300 x 30000 9.9, 13.4, 33 x 30000 6.3, 8.5
+        // batches of loads, unless other columns' warps hide the latency and
+        // most of a column's loads would be predicated off: columns of one or
+        // two loads a lane, and, with still more columns, those whose second
+        // batch is at least 3/8 empty.  Time in batches over time with one load
+        // at a time, several sets of operands in turn (one set, in L2): 33 x 2600
+        // 1.08 (1.06), 33 x 30000 1.34 (1.35); 300 x 3500 0.91 (1.09), 300 x 30000
+        // 1.21 (1.36), 416 x 8000 1.14 (1.13), 440 x 12000 0.94 (1.13), 480 x
+        // 12000 0.83 (1.06), 508 x 5036 0.43 (0.62), 1000 x 30000 0.37 (0.37)
         const int rows = min(m, rps);
-        const bool empty = rows <= 64 || (rows > 256 && rows < 512);
-        if (!vec && (n <= 2048 || !empty)) { LAUNCH(false, false, 8); return cudaGetLastError(); }
+        const bool single = rows <= 64 ? n > 2048 : rows > 256 && rows <= 416 && n > 6000;
+        if (!vec && !single) { LAUNCH(false, false, 8); return cudaGetLastError(); }
     }
     if (vec) LAUNCH(false, true, 1); else LAUNCH(false, false, 1);
 #undef LAUNCH

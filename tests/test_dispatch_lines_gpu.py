@@ -80,6 +80,15 @@ def test_gemv_t_of_tall_and_of_short_columns(us, cuda, cplx):
         assert odd <= factor * aligned + 1, (m, n)
 
 
+@pytest.mark.parametrize("n", [2600, 5036, 12000])
+def test_gemv_t_of_a_nearly_full_batch(us, cuda, n):
+    """Unaligned columns of almost two batches of loads (256 rows each) take no
+    longer than those of two and a half."""
+    A, x, y = buf(641 * n, False, cuda), buf(640, False, cuda), buf(n, False, cuda)
+    t508, t640 = (us(lambda h: B.iclblasSgemv(h, 1, m, n, 1.0, A, m + 1, x, 1, 0.0, y, 1)) for m in (508, 640))
+    assert t508 <= 1.15 * t640
+
+
 @pytest.mark.parametrize("cplx", [False, True])
 def test_gemv_n_of_few_columns(us, cuda, cplx):
     """One column more than a batch of 32 is no other slice."""
