@@ -468,21 +468,27 @@ __global__ void __launch_bounds__(kTThreads) gemv_t_block_kernel(int m, T alpha,
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// Whether op T / C of an unaligned m x n matrix takes a block a column: for
-// columns that are long enough for eight warps, yet no longer than one block
-// reads in the time the slices' sums cost, and not many more than the SMs
-// hold blocks.  Measured against the slices (us, operands in L2): real 1025 x
-// 1025 3.0, 3.6; 3000 x 1777 6.8, 8.8; 6000 x 6000 35, 39; but 1500 x 6000
-// 11.2, 9.4; 100000 x 33 23, 9.3; 1000000 x 4 215, 25.  Complex 1025 x 1025
-// 3.9, 5.2; 3000 x 1777 8.8, 10.3; 10000 x 600 9.2, 11.2; 30000 x 600 32, 41;
-// but 1500 x 3000 8.3, 7.5; 3000 x 6000 42, 38; 30000 x 33 12.3, 8.0; 100000 x
-// 200 80, 48.
+// Whether op T / C of an unaligned m x n matrix takes a block a column.  The
+// slices have a warp per 1024 rows of a column, so few columns leave the SMs
+// idle, all the more below 2048 rows, where a column is one slice; many columns
+// fill them, and then the blocks' reductions and partly empty last wave cost
+// more than the slices' sums.  Very long columns keep a block's eight warps
+// reading for longer than the slices' sums take, unless there are columns for
+// all SMs.  Complex columns of two slices lose to the blocks only up to twice
+// as many columns as the SMs hold blocks.
+// Time in blocks over time in slices, several sets of operands in turn (one
+// set, in L2): real 1297 x 800 0.58 (0.65), 1297 x 3500 1.24 (1.15), 2047 x
+// 2600 0.84 (0.86), 4001 x 4500 0.80 (0.82), 12001 x 500 1.13 (0.96), 30001 x
+// 100 2.05 (1.09), 1000001 x 33 13 (13); complex 2047 x 1700 0.50 (0.68), 1297
+// x 3500 1.03 (1.34), 3001 x 1700 0.88 (0.92), 3001 x 4500 1.41 (1.48), 4001 x
+// 3500 0.79 (0.80), 30001 x 300 1.42 (1.02), 30001 x 1200 0.81 (0.81).
 bool block_columns(bool cplx, int m, int n)
 {
     if (m < 1024 || n > 6000) return false;
-    if (!cplx) return m < 2048 ? n <= 2048 : m <= 32768;
-    if (m < 4096) return n <= (m < 2048 ? 1600 : 4096);
-    return m <= 12288 || (m <= 49152 && n >= 300);
+    if (m < 2048) return n <= 2 * m;
+    if (!cplx) return m <= 16384;
+    if (m < 3072) return n <= 2400;
+    return m <= 12288 || (m <= 65536 && n >= 500);
 }
 
 template <class T>

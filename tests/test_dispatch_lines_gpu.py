@@ -89,6 +89,20 @@ def test_gemv_t_of_a_nearly_full_batch(us, cuda, n):
     assert t508 <= 1.15 * t640
 
 
+def test_gemv_t_at_two_slices_a_column(us, cuda):
+    """Unaligned complex columns just below two slices take no longer than
+    those just above; ten matrices in turn, together larger than L2."""
+    from itertools import cycle
+    n, size = 1700, 2051 * 1700
+    A, x, y = buf(10 * size, True, cuda), buf(2049, True, cuda), buf(n, True, cuda)
+
+    def time(m):
+        at = cycle(range(0, 10 * size, size))
+        return us(lambda h: B.iclblasCgemv(h, 1, m, n, 1.0, A[next(at):], m + 2, x, 1, 0.0, y, 1))
+
+    assert time(2047) <= 1.15 * time(2049)
+
+
 @pytest.mark.parametrize("cplx", [False, True])
 def test_gemv_n_of_few_columns(us, cuda, cplx):
     """One column more than a batch of 32 is no other slice."""

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m,n", [(1, 1), (31, 8), (255, 7), (256, 9), (257, 65), (511, 1023), (513, 130), (3001, 177),
-                                 (77, 3001), (64, 2049), (416, 6001), (417, 6001)])
+                                 (77, 3001), (64, 2049), (416, 6001), (417, 6001), (1025, 2050),
+                                 (1025, 2051), (2049, 2400), (2049, 2401), (16385, 65)])
 @pytest.mark.parametrize("dtype", [np.float32, np.complex64])
 def test_unaligned(handle, cuda, m, n, dtype):
     import torch
