@@ -509,7 +509,12 @@ cudaError_t gemv_impl(iclblasHandle_t h, int trans, int m, int n, T alpha, const
         // batches (3000 x 33 4.1 us with two, 2.4), and so they are where the
         // row tiles nearly fill the GPU (100000 x 200 12.5, 8.9); with a batch
         // or two of columns three groups would be idle (complex 1000000 x 4
-        // 17 us with four groups, 5.8 with one; 100000 x 4 3.3, 2.4)
+        // 17 us with four groups, 5.8 with one; 100000 x 4 3.3, 2.4).  The other
+        // side: at 100 to 128 columns and a dozen to 40 row tiles two slices are
+        // faster on operands in HBM (complex 6001 x 128, lda 6001, 9.3 us in one,
+        // 6.1), but then a handle's first call would need scratch; over 200 to
+        // 1000000 rows and 1 to 2000 columns, in L2 and in HBM, this rule is 2.5 %
+        // above the best of the three on average, slices throughout 12 %
         const bool wide = rt >= 96, few = n <= 16 && (!vec || rt > 2 * h->sm_count);
         const bool small = (long)rt * max(1, n / 64) < target && !few && !(wide && n > 320);
         int splits = 1, unit = 8;
